@@ -304,6 +304,7 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
     R.f_beta = (float)d.beta;
     R.f_force = f32_force(R.f_beta, R.f_cforce);
     R.f_pairs = f32_pairs(R.f_omega, R.f_om1, R.f_c13, R.f_c2, R.f_force);
+    R.f_force2 = f32_force2(R.f_force, R.f_force);
     R.perturb_mode = d.perturb_mode;
     R.resample_mode = d.resample_mode;
     R.drag_mode = d.drag_mode;
@@ -631,9 +632,26 @@ struct LbPlan {
 
 static bool plan_active(const LbPlan &p, int r) { return p.active.empty() || p.active[r]; }
 
+// largest band of run r's split at its cluster size
+static int run_rows_max(const clbm_ctx *c, int r) {
+  const int cs = c->run_cs[r];
+  const std::vector<int> &row0 = c->run_rows[r];
+  if ((int)row0.size() != cs + 1) return (c->runs_h[r].H + cs - 1) / cs;
+  int m = 0;
+  for (int b = 0; b < cs; b++) m = std::max(m, row0[b + 1] - row0[b]);
+  return m;
+}
+
+// whether run r runs cluster-resident: its plan says so and its bands are
+// held on chip (temporal_resident); every other run streams
+static bool run_resident(const clbm_ctx *c, int r) {
+  return c->run_cs[r] > 0 && temporal_resident(c->runs_h[r].W, run_rows_max(c, r));
+}
+
 static LbPlan current_plan(const clbm_ctx *c, bool f64) {
   LbPlan p;
-  p.cs = f64 ? std::vector<int>(c->nruns, 0) : c->run_cs;
+  p.cs.assign(c->nruns, 0);
+  for (int r = 0; r < c->nruns && !f64; r++) p.cs[r] = run_resident(c, r) ? c->run_cs[r] : 0;
   p.tv = c->run_tv;
   p.rows = c->run_rows;
   const bool sub = !f64 && c->stream_subset;
@@ -731,19 +749,12 @@ static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int
   return cudaSuccess;
 }
 
-// Install a plan: per run cluster size (0 = streaming), thread variant and
-// band split (empty: even), the streaming runs' launch variant.  Captured
-// intervals are dropped.
-static cudaError_t set_plan(clbm_ctx *c, const std::vector<int> &cs, const std::vector<int> &tv, int variant,
-                            const std::vector<std::vector<int>> &rows = {}) {
-  c->run_cs = cs;
-  c->run_tv = tv;
-  c->run_rows = rows;
-  c->run_rows.resize(c->nruns);
-  c->step_variant = variant;
+// The streaming runs' table after a change of the plan or of a band split;
+// captured intervals are dropped.
+static cudaError_t refresh_stream_table(clbm_ctx *c) {
   std::vector<int> streaming;
   for (int r = 0; r < c->nruns; r++)
-    if (!cs[r]) streaming.push_back(r);
+    if (!run_resident(c, r)) streaming.push_back(r);
   c->stream_subset = (int)streaming.size() != c->nruns;
   cudaError_t e = cudaSuccess;
   if (c->stream_subset)
@@ -752,6 +763,18 @@ static cudaError_t set_plan(clbm_ctx *c, const std::vector<int> &cs, const std::
     c->stream_nruns = c->nruns;
   destroy_graphs(c);
   return e;
+}
+
+// Install a plan: per run cluster size (0 = streaming), thread variant and
+// band split (empty: even), the streaming runs' launch variant.
+static cudaError_t set_plan(clbm_ctx *c, const std::vector<int> &cs, const std::vector<int> &tv, int variant,
+                            const std::vector<std::vector<int>> &rows = {}) {
+  c->run_cs = cs;
+  c->run_tv = tv;
+  c->run_rows = rows;
+  c->run_rows.resize(c->nruns);
+  c->step_variant = variant;
+  return refresh_stream_table(c);
 }
 
 // Enqueue one interval on the context's stream (no synchronisation).
@@ -1155,6 +1178,11 @@ static bool shape_fits(const RunDev &R, int cs, int tv) {
          temporal_max_clusters(cs, tv, R.W, (R.H + cs - 1) / cs, R.field_mode != 0) >= 1;
 }
 
+// ... and is held on chip at it (the autotuner's candidates)
+static bool shape_resident(const RunDev &R, int cs, int tv) {
+  return temporal_resident(R.W, (R.H + cs - 1) / cs) && shape_fits(R, cs, tv);
+}
+
 // largest band of a split row0[0..cs]
 static int split_rows_max(const std::vector<int> &row0) {
   int m = 0;
@@ -1173,7 +1201,8 @@ static std::vector<int> balanced_split(const RunDev &R, int cs, int tv, double g
   even_band_rows(R.H, cs, even.data());
   if (!balanced_band_rows(R.W, R.H, R.xmin, R.xmax, R.ymin, R.ymax, cs, gamma, temporal_rows_limit(R.W),
                           row0.data()) ||
-      row0 == even || temporal_max_clusters(cs, tv, R.W, split_rows_max(row0), R.field_mode != 0) < 1)
+      row0 == even || !temporal_resident(R.W, split_rows_max(row0)) ||
+      temporal_max_clusters(cs, tv, R.W, split_rows_max(row0), R.field_mode != 0) < 1)
     return {};
   return row0;
 }
@@ -1307,7 +1336,7 @@ extern "C" int clbm_autotune(clbm_ctx *c, int launches, int *best, double *ms_pe
       const int vidx = variant_index(cs, tv);
       if (ms_per_variant) ms_per_variant[vidx] = -1.0;
       bool ok = true;
-      for (const RunDev &Rr : c->runs_h) ok = ok && shape_fits(Rr, cs, tv);
+      for (const RunDev &Rr : c->runs_h) ok = ok && shape_resident(Rr, cs, tv);
       if (!ok) continue;
       LbPlan p;
       cudaError_t e = full_plan(c, std::vector<int>(R, cs), std::vector<int>(R, tv), best_sv, p);
@@ -1382,7 +1411,7 @@ extern "C" int clbm_autotune(clbm_ctx *c, int launches, int *best, double *ms_pe
       double cbest = 1e30;
       for (const int cs : kClusterSizes)
         for (int tv = 0; tv < ntv; tv++) {
-          if (!shape_fits(c->runs_h[r], cs, tv)) continue;
+          if (!shape_resident(c->runs_h[r], cs, tv)) continue;
           p.cs[r] = cs;
           p.tv[r] = tv;
           double per = 0.0;
@@ -1504,7 +1533,7 @@ extern "C" int clbm_set_band_rows(clbm_ctx *c, int run, const int *rows, int nba
   const RunDev &R = c->runs_h[run];
   if (nbands == 0) {  // back to the even split
     c->run_rows[run].clear();
-    destroy_graphs(c);
+    CK(refresh_stream_table(c));
     return CLBM_OK;
   }
   if (c->run_cs[run] == 0 || nbands != c->run_cs[run])
@@ -1518,7 +1547,7 @@ extern "C" int clbm_set_band_rows(clbm_ctx *c, int run, const int *rows, int nba
   if (temporal_max_clusters(nbands, c->run_tv[run], R.W, split_rows_max(row0), R.field_mode != 0) < 1)
     return fail(CLBM_ERR_INVALID, "the largest band does not fit in shared memory at this variant");
   c->run_rows[run] = row0;
-  destroy_graphs(c);
+  CK(refresh_stream_table(c));
   return CLBM_OK;
 }
 

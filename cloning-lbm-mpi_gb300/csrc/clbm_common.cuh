@@ -75,6 +75,9 @@ __host__ __device__ inline f2_t f2_bits(float lo, float hi) {
 struct F32Pairs {
   f2_t om1, omega, w9, w36, c13, c2;  // (v, v)
   f2_t fb9_0, fb9_m, f13_0, f2_m;     // (fb9, 0), (fb9, -fb9), (f13, -0), (f2, -f2)
+  // literals of the two-node collision, (v, v): packed arithmetic takes no
+  // immediate, and from the constant bank they cost no move into registers
+  f2_t one, mone, c15, mc45, w49;     // 1, -1, 1.5, -4.5, 4/9
 };
 __host__ __device__ inline void f32_pairs_force(F32Pairs &p, const F32Force &f) {
   p.fb9_0 = f2_bits(f.fb9, 0.0f);
@@ -90,8 +93,30 @@ __host__ __device__ inline F32Pairs f32_pairs(float omega, float om1, float c13,
   p.w36 = f2_bits(1.0f / 36.0f, 1.0f / 36.0f);
   p.c13 = f2_bits(c13, c13);
   p.c2 = f2_bits(c2, c2);
+  p.one = f2_bits(1.0f, 1.0f);
+  p.mone = f2_bits(-1.0f, -1.0f);
+  p.c15 = f2_bits(1.5f, 1.5f);
+  p.mc45 = f2_bits(-4.5f, -4.5f);
+  p.w49 = f2_bits(4.0f / 9.0f, 4.0f / 9.0f);
   f32_pairs_force(p, f);
   return p;
+}
+
+// Force operands of the two-node collision (collide_f32_nodes): lane h holds
+// node h's value, with the signs that collision takes them in.
+struct F32Force2 {
+  f2_t hb, nfbm3, fb9, nfb9, f2, nf2, nf13;
+};
+__host__ __device__ inline F32Force2 f32_force2(const F32Force &a, const F32Force &b) {
+  F32Force2 f;
+  f.hb = f2_bits(a.hb, b.hb);
+  f.nfbm3 = f2_bits(-a.fbm3, -b.fbm3);
+  f.fb9 = f2_bits(a.fb9, b.fb9);
+  f.nfb9 = f2_bits(-a.fb9, -b.fb9);
+  f.f2 = f2_bits(a.f2, b.f2);
+  f.nf2 = f2_bits(-a.f2, -b.f2);
+  f.nf13 = f2_bits(-a.f13, -b.f13);
+  return f;
 }
 
 // One independent run (lattice, square, physics, clone block) of a batch.
@@ -125,6 +150,7 @@ struct RunDev {
   float f_omega, f_om1, f_c13, f_c2, f_cforce, f_beta;
   F32Force f_force;
   F32Pairs f_pairs;            // the same constants packed for the f32x2 collision
+  F32Force2 f_force2;          // f_force in both lanes, for the two-node collision
   int perturb_mode, resample_mode, ranks, nsnap;
   unsigned long long seed;
   unsigned run_id;

@@ -116,6 +116,7 @@ struct TemporalArgs {
   // node, clbm_step.cu), instead of reading it from src
   int fused;
   ReseedArgs rs;
+  unsigned div_wh;    // ceil(2^32 / pairs per row), set by launch_temporal
 };
 
 
@@ -162,6 +163,10 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
                             cudaStream_t s);
 int temporal_max_clusters(int cs, int variant, int W, int rows_max, bool field);
 int temporal_rows_limit(int W);
+// whether a band of `rows` rows is held on chip: a row of an odd width takes
+// the room of one node more, so a band at the very limit may not be (its run
+// then steps through the streaming kernel, the same results)
+bool temporal_resident(int W, int rows);
 int temporal_variant_count();
 // band splits (clbm_bands.cu): row0[0..cs] of H rows in cs bands, the first
 // H % cs one row more; or balanced for an estimated per-step cost in which a

@@ -256,6 +256,66 @@ __device__ __forceinline__ float collide_f32_pairs(const float g[9], float out[9
   return drho;
 }
 
+// collide_f32_pairs of two nodes at once, node h in lane h of every operand:
+// 77 packed operations and two reciprocals for two nodes, where one node at a
+// time spends 34 scalar and 21 packed ones.  Every lane takes the operations
+// of collide_f32_pairs in the same order with the same roundings.  Packed
+// arithmetic has no operand negation, so the chain from the reciprocal on
+// runs on negated values (nr = -1/rho, nux = -ux, ...): a rounded product or
+// fused multiply-add of negated operands is the negated result, exactly, and
+// the signs are taken back by an add for a sub and by negated constants
+// (F32Force2).  Left out are the two identities of collide_f32_pairs' lane 1,
+// fma(0, uy, fx) = fx and c13 ty - 0 = c13 ty (the sign of a zero aside).
+// Returns drho of both nodes.
+__device__ __forceinline__ f2_t collide_f32_nodes(const f2_t g[9], f2_t out[9], const F32Pairs &k,
+                                                  const F32Force2 &f) {
+  namespace X = f32x2op;
+  const f2_t a13 = X::add(g[1], g[3]), a24 = X::add(g[2], g[4]);
+  const f2_t d13 = X::sub(g[1], g[3]), d24 = X::sub(g[2], g[4]);
+  const f2_t s57 = X::sub(g[5], g[7]), t86 = X::sub(g[8], g[6]);
+  const f2_t drho = X::add(X::add(X::add(g[0], a13), a24), X::add(X::add(g[5], g[7]), X::add(g[6], g[8])));
+  const f2_t jx = X::add(d13, X::add(s57, t86));
+  const f2_t jy = X::add(d24, X::sub(s57, t86));
+  const f2_t nrho = X::sub(k.mone, drho);
+  const f2_t nr0 = f2_bits(rcp_approx(X::lo(nrho)), rcp_approx(X::hi(nrho)));
+  const f2_t ninv = X::fma(nr0, X::fma(drho, nr0, X::add(k.one, nr0)), nr0);
+  const f2_t nux = X::fma(jx, ninv, X::mul(f.hb, ninv));
+  const f2_t nuy = X::mul(jy, ninv);
+  const f2_t ntx = X::fma(drho, nux, nux), nty = X::fma(drho, nuy, nuy);
+  const f2_t u2 = X::mul(k.c15, X::fma(nux, nux, X::mul(nuy, nuy)));
+  const f2_t base = X::fma(nrho, u2, drho);
+  const f2_t fx = X::mul(f.nfbm3, nux);
+  const f2_t r45 = X::mul(k.mc45, nrho);
+  out[0] = X::fma(k.om1, g[0], X::mul(k.w49, X::fma(k.omega, base, fx)));
+  {  // (1, 3): e = ux, cx = 1
+    const f2_t ev = X::mul(k.w9, X::fma(k.omega, X::fma(X::mul(r45, nux), nux, base), X::fma(f.nfb9, nux, fx)));
+    const f2_t nod = X::fma(k.c13, ntx, f.nf13);
+    out[1] = X::fma(k.om1, g[1], X::sub(ev, nod));
+    out[3] = X::fma(k.om1, g[3], X::add(ev, nod));
+  }
+  {  // (2, 4): e = uy, cx = 0
+    const f2_t ev = X::mul(k.w9, X::fma(k.omega, X::fma(X::mul(r45, nuy), nuy, base), fx));
+    const f2_t nod = X::mul(k.c13, nty);
+    out[2] = X::fma(k.om1, g[2], X::sub(ev, nod));
+    out[4] = X::fma(k.om1, g[4], X::add(ev, nod));
+  }
+  {  // (5, 7): e = ux + uy, cx = 1
+    const f2_t ne = X::add(nux, nuy);
+    const f2_t ev = X::mul(k.w36, X::fma(k.omega, X::fma(X::mul(r45, ne), ne, base), X::fma(f.nfb9, ne, fx)));
+    const f2_t nod = X::fma(k.c2, X::add(ntx, nty), f.nf2);
+    out[5] = X::fma(k.om1, g[5], X::sub(ev, nod));
+    out[7] = X::fma(k.om1, g[7], X::add(ev, nod));
+  }
+  {  // (6, 8): e = uy - ux, cx = -1
+    const f2_t ne = X::sub(nuy, nux);
+    const f2_t ev = X::mul(k.w36, X::fma(k.omega, X::fma(X::mul(r45, ne), ne, base), X::fma(f.fb9, ne, fx)));
+    const f2_t nod = X::fma(k.c2, X::sub(nty, ntx), f.f2);
+    out[6] = X::fma(k.om1, g[6], X::sub(ev, nod));
+    out[8] = X::fma(k.om1, g[8], X::add(ev, nod));
+  }
+  return drho;
+}
+
 // The FP32 collision of one node of run R; field: the node's random-field
 // value, or nullptr under the uniform body force.
 __device__ __forceinline__ float collide_f32_run(const RunDev &R, const float S[9], float P[9],

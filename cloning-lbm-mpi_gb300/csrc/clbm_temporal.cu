@@ -3,9 +3,8 @@
 // One thread-block cluster per clone: the clone's H rows are split into CS
 // bands of consecutive rows, given by the launch (an even split, or one
 // balanced for the extra cost of the square's rows and the walls), each band
-// in one CTA's shared memory (nine floats per node, node after node).  The T steps
-// of the interval run without touching HBM except for the drag terms: P_0 is
-// loaded once, S_T stored once.
+// in one CTA's shared memory.  The T steps of the interval run without
+// touching HBM except for the drag terms: P_0 is loaded once, S_T stored once.
 //
 // In-place update ("AA" pattern): one buffer A holds, alternately,
 //   after a local step:  A[n][opp k] = P(n,k)        (post-collision, own node)
@@ -15,12 +14,32 @@
 // A[n + c_k][k], or to A[n][opp k] when slot (n, opp k) bounces back.  Step
 // t odd is a local step: S(n,k) = A[n][k], P(n,k) -> A[n][opp k].  In both,
 // the nine slots a node reads are exactly the nine it writes and no other
-// node touches them, so a step needs no barrier inside; one cluster barrier
-// separates steps.  These are the pull rules of clbm_step.cu (the reference's
-// collide / push-stream / bounce-back / reset / swap sequence,
-// src/mpi_LBM_GK_pops_perturb.cpp:426-443), so results are bit-identical to
-// the streaming kernel.  Neighbours across a band edge are read and written
-// in the adjacent CTA's shared memory (distributed shared memory).
+// node touches them, so a step needs no barrier inside.  These are the pull
+// rules of clbm_step.cu (the reference's collide / push-stream / bounce-back /
+// reset / swap sequence, src/mpi_LBM_GK_pops_perturb.cpp:426-443), so results
+// are bit-identical to the streaming kernel.  Neighbours across a band edge
+// are read and written in the adjacent CTA's shared memory.
+//
+// A thread takes a pair of nodes, x and x + ceil(W/2) of one row, one in each
+// lane of the packed FP32 arithmetic: every neighbour offset is the same for
+// both, so a pair's nine slots are nine 64-bit words and the whole collision
+// is packed.  Only the pairs at the two ends of a row (the seam: the periodic
+// wrap, and between the halves) have their lanes' neighbours in different
+// pairs; they are few and take per-lane addresses.  An odd width leaves the
+// last pair's lane 1 empty (a column of its own that no node reads).
+//
+// What bounds it: per 32 pairs 77 packed operations, 2 cycles each on the
+// FMA pipe of a scheduler (154), and 36 cycles of the SM's shared memory for
+// four schedulers' 18 accesses each (144).  On the 256x64 channel (bands
+// 23/18/23, 512 threads) a segment takes 215 (local step) to 270 cycles; 4096
+// clones run at 0.306 ms per step, where one node per thread with the four
+// direction pairs packed took 0.367; 1024 clones of 400x100 (9 bands) at 0.221
+// against 0.353.  What made the difference besides the packing (ms per step of
+// the 256x64 case): each warp's share of the deal kept in registers instead of
+// worked out in every step (0.344 -> 0.317), one population's row planes
+// instead of node records, so that what crosses a band edge goes as whole
+// sectors (0.317 -> 0.306; 400x100: 0.265 -> 0.225), and the split cluster
+// barrier with the edge rows first (400x100: 0.33 -> 0.28).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -35,7 +54,7 @@ namespace clbm {
 
 // Distributed shared memory through 32-bit shared::cluster addresses: the
 // address of this CTA's shared-memory offset `a` in the CTA of cluster rank
-// `rank`, and FP32 loads / stores at such addresses.
+// `rank`, and loads / stores of one float or one pair at such addresses.
 __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
   unsigned r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
@@ -49,11 +68,22 @@ __device__ __forceinline__ float ld_cluster(unsigned a) {
 __device__ __forceinline__ void st_cluster(unsigned a, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ f2_t ld_cluster2(unsigned a) {
+  f2_t v;
+  asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster2(unsigned a, f2_t v) {
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
 
 // Geometry of one CTA's band.
 struct Band {
-  int cs, rank, clone, W, H, rows, row0, nb, rowstep;
-  int rows_prev;  // rows of the previous band (its last row lies above this band's row 0)
+  int cs, rank, clone, W, H, rows, row0;
+  int Wh, np;      // pairs per row, pairs of the band
+  int ps, rowf;    // floats per plane of a row (2 Wh), per row (9 planes)
+  unsigned div_wh; // ceil(2^32 / Wh)
+  int rows_prev;   // rows of the previous band (its last row lies above this band's row 0)
   float *prev, *next;
   unsigned own_c, prev_c, next_c;  // shared::cluster byte addresses of A in this / previous / next CTA
   long long plane;
@@ -61,169 +91,295 @@ struct Band {
   float *dst;
 };
 
-// One node of one step, any position: bounce-back, band edges (distributed
-// shared memory), the square, walls.  i = band-local node index.
-__device__ __forceinline__ void update_general(const TemporalArgs &a, const Band &b, float *A, int i,
-                                               int t, bool gather, bool last, float *terms) {
+// Float offset, within a row of A, of column x's population 0 (population k
+// at + k ps): pair x or x - Wh, its lane 0 or 1.
+__device__ __forceinline__ int col_off(const Band &b, int x) { return x < b.Wh ? 2 * x : 2 * (x - b.Wh) + 1; }
+
+// A row of A: in this CTA, or anywhere in the cluster.
+struct RowL {
+  float *p;
+  __device__ __forceinline__ float ld(int o) const { return p[o]; }
+  __device__ __forceinline__ void st(int o, float v) const { p[o] = v; }
+  __device__ __forceinline__ f2_t ld2(int o) const { return *(const f2_t *)(p + o); }
+  __device__ __forceinline__ void st2(int o, f2_t v) const { *(f2_t *)(p + o) = v; }
+};
+struct RowC {
+  unsigned a;
+  __device__ __forceinline__ float ld(int o) const { return ld_cluster(a + 4u * o); }
+  __device__ __forceinline__ void st(int o, float v) const { st_cluster(a + 4u * o, v); }
+  __device__ __forceinline__ f2_t ld2(int o) const { return ld_cluster2(a + 4u * o); }
+  __device__ __forceinline__ void st2(int o, f2_t v) const { st_cluster2(a + 4u * o, v); }
+};
+
+// Columns of a pair: float offsets of the pair itself (lane 0; lane 1 is one
+// further) and of its left (m) and right (p) neighbours, per lane.
+struct Cols {
+  int o, m0, m1, p0, p1;
+};
+__device__ __forceinline__ Cols cols_inner(int xh) {
+  return Cols{2 * xh, 2 * xh - 2, 2 * xh - 1, 2 * xh + 2, 2 * xh + 3};
+}
+// any pair: the periodic wrap, and with an odd width lane 1 of the last pair,
+// which holds no node: it gets itself for both neighbours (a column of its
+// own, periodic over one node, that no node ever reads)
+__device__ __forceinline__ Cols cols_any(const Band &b, int xh) {
+  const int x1 = xh + b.Wh;
+  Cols c;
+  c.o = 2 * xh;
+  c.m0 = col_off(b, xh == 0 ? b.W - 1 : xh - 1);
+  c.p0 = col_off(b, xh + 1 == b.W ? 0 : xh + 1);
+  c.m1 = x1 < b.W ? col_off(b, x1 - 1) : c.o + 1;
+  c.p1 = x1 < b.W ? col_off(b, x1 + 1 == b.W ? 0 : x1 + 1) : c.o + 1;
+  return c;
+}
+
+// The seam: the pairs of a row whose lanes' neighbour columns do not both lie
+// at a constant offset -- the first and the last, and with an odd width the
+// one before the last (its lane 1 is the last node).  seam_count pairs per
+// row; the j-th of them.
+__device__ __forceinline__ bool on_seam(const Band &b, int xh) {
+  return xh == 0 || xh >= b.Wh - 1 - (b.W & 1);
+}
+__device__ __forceinline__ int seam_count(const Band &b) { return (b.W & 1) && b.Wh > 2 ? 3 : 2; }
+__device__ __forceinline__ int seam_pair(const Band &b, int j) { return j == 0 ? 0 : b.Wh - j; }
+
+// Index p within a row as the segments take its pairs: the pair Wh - 1 first,
+// then 0, 1, ..., so that the seam at the two ends falls into one segment.
+__device__ __forceinline__ int pair_of(const Band &b, int p) { return p == 0 ? b.Wh - 1 : p - 1; }
+
+// The two nodes' force: the run's, or under a random field from its values at
+// the nodes (where lane 1 holds no node, lane 0's).
+template <bool FIELD>
+__device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, const float *map, int y, int xh,
+                                                float feps) {
+  if (!FIELD) return R.f_force2;
+  const float *m = map + (long long)y * b.W + xh;
+  const float m0 = m[0], m1 = xh + b.Wh < b.W ? m[b.Wh] : m0;
+  return f32_force2(f32_force(field_beta_f32(R.f_beta, feps, m0), R.f_cforce),
+                    f32_force(field_beta_f32(R.f_beta, feps, m1), R.f_cforce));
+}
+
+// One pair of nodes in a gather step.  C, U, D: the pair's row and the rows
+// y - 1 and y + 1.  S(n,k) is read from A[n - c_k][opp k] and P(n, opp k)
+// goes back to that slot (the pull rules make the two the same).  WALL: 1 =
+// the bottom wall y = 0, whose slots 2, 5, 6 are the node's own; 2 = the top
+// wall, slots 4, 7, 8 (the row beyond the wall is not touched); 3 = by the
+// thread's wb / wt.  UNI: both lanes' neighbour columns lie in one pair, every
+// slot pair is one 64-bit access.  PRED: lane h is written only if !skip_h.
+template <bool FIELD, bool UNI, int WALL, bool PRED, class RC, class RU, class RD>
+__device__ __forceinline__ void gather_pair(const RunDev &R, int ps, const RC C, const RU U, const RD D, const Cols &c,
+                                            const F32Force2 &f, bool &bad, bool skip0 = false, bool skip1 = false,
+                                            bool wb = false, bool wt = false) {
+  auto ld = [](const auto &row, int a, int b2, int q) {
+    return UNI ? row.ld2(a + q) : f2_bits(row.ld(a + q), row.ld(b2 + q));
+  };
+  f2_t S[9];
+  S[0] = C.ld2(c.o);
+  S[1] = ld(C, c.m0, c.m1, 3 * ps);
+  S[3] = ld(C, c.p0, c.p1, ps);
+  // WALL 3: the slot is the thread's own (row C) or the neighbour's, chosen by address
+  const bool ob = WALL == 3 && wb, ot = WALL == 3 && wt;
+  const int u2 = c.o + (ob ? 2 : 4) * ps, d4 = c.o + (ot ? 4 : 2) * ps;
+  const int u5a = ob ? c.o + 5 * ps : c.m0 + 7 * ps, u5b = ob ? c.o + 1 + 5 * ps : c.m1 + 7 * ps;
+  const int u6a = ob ? c.o + 6 * ps : c.p0 + 8 * ps, u6b = ob ? c.o + 1 + 6 * ps : c.p1 + 8 * ps;
+  const int d7a = ot ? c.o + 7 * ps : c.p0 + 5 * ps, d7b = ot ? c.o + 1 + 7 * ps : c.p1 + 5 * ps;
+  const int d8a = ot ? c.o + 8 * ps : c.m0 + 6 * ps, d8b = ot ? c.o + 1 + 8 * ps : c.m1 + 6 * ps;
+  if (WALL == 1) {
+    S[2] = C.ld2(c.o + 2 * ps);
+    S[5] = C.ld2(c.o + 5 * ps);
+    S[6] = C.ld2(c.o + 6 * ps);
+  } else {
+    S[2] = U.ld2(u2);
+    S[5] = ld(U, u5a, u5b, 0);
+    S[6] = ld(U, u6a, u6b, 0);
+  }
+  if (WALL == 2) {
+    S[4] = C.ld2(c.o + 4 * ps);
+    S[7] = C.ld2(c.o + 7 * ps);
+    S[8] = C.ld2(c.o + 8 * ps);
+  } else {
+    S[4] = D.ld2(d4);
+    S[7] = ld(D, d7a, d7b, 0);
+    S[8] = ld(D, d8a, d8b, 0);
+  }
+  f2_t P[9];
+  const f2_t drho = collide_f32_nodes(S, P, R.f_pairs, f);
+  bad |= (!(f32x2op::lo(drho) > -1.0f) && !(PRED && skip0)) || (!(f32x2op::hi(drho) > -1.0f) && !(PRED && skip1));
+  auto st = [&](const auto &row, int a, int b2, int q, f2_t v) {
+    if (UNI && !PRED) {
+      row.st2(a + q, v);
+    } else {
+      if (!PRED || !skip0) row.st(a + q, f32x2op::lo(v));
+      if (!PRED || !skip1) row.st(b2 + q, f32x2op::hi(v));
+    }
+  };
+  auto st2 = [&](const auto &row, int a, f2_t v) {  // a slot pair of one column pair
+    if (!PRED) {
+      row.st2(a, v);
+    } else {
+      if (!skip0) row.st(a, f32x2op::lo(v));
+      if (!skip1) row.st(a + 1, f32x2op::hi(v));
+    }
+  };
+  st2(C, c.o, P[0]);
+  st(C, c.m0, c.m1, 3 * ps, P[3]);
+  st(C, c.p0, c.p1, ps, P[1]);
+  if (WALL == 1) {
+    st2(C, c.o + 2 * ps, P[4]);
+    st2(C, c.o + 5 * ps, P[7]);
+    st2(C, c.o + 6 * ps, P[8]);
+  } else {
+    st2(U, u2, P[4]);
+    st(U, u5a, u5b, 0, P[7]);
+    st(U, u6a, u6b, 0, P[8]);
+  }
+  if (WALL == 2) {
+    st2(C, c.o + 4 * ps, P[2]);
+    st2(C, c.o + 7 * ps, P[5]);
+    st2(C, c.o + 8 * ps, P[6]);
+  } else {
+    st2(D, d4, P[2]);
+    st(D, d7a, d7b, 0, P[5]);
+    st(D, d8a, d8b, 0, P[6]);
+  }
+}
+
+// One pair of nodes in a local step: S(n,k) = A[n][k], P(n,k) -> A[n][opp k].
+template <bool PRED>
+__device__ __forceinline__ void local_pair(const RunDev &R, int ps, float *o, const F32Force2 &f, bool &bad,
+                                           bool skip0 = false, bool skip1 = false) {
+  f2_t S[9], P[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) S[k] = *(const f2_t *)(o + k * ps);
+  const f2_t drho = collide_f32_nodes(S, P, R.f_pairs, f);
+  bad |= (!(f32x2op::lo(drho) > -1.0f) && !(PRED && skip0)) || (!(f32x2op::hi(drho) > -1.0f) && !(PRED && skip1));
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    if (!PRED) {
+      *(f2_t *)(o + opp_of(k) * ps) = P[k];
+    } else {
+      if (!skip0) o[opp_of(k) * ps] = f32x2op::lo(P[k]);
+      if (!skip1) o[opp_of(k) * ps + 1] = f32x2op::hi(P[k]);
+    }
+  }
+}
+
+__device__ __forceinline__ bool in_box(const RunDev &R, int x, int y) {
+  return x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
+}
+
+// Node j of the square's perimeter within rows [ylo, yhi]: the left and right
+// columns row by row, then the rest of the bottom and top rows.  The count of
+// such nodes is perimeter_count.
+__device__ __forceinline__ int perimeter_count(const RunDev &R, int ylo, int yhi) {
+  if (yhi < ylo) return 0;
+  const int ncol = R.xmax > R.xmin ? 2 : 1, nin = R.xmax > R.xmin ? R.xmax - R.xmin - 1 : 0;
+  return ncol * (yhi - ylo + 1) + (ylo == R.ymin ? nin : 0) + (yhi == R.ymax && R.ymax > R.ymin ? nin : 0);
+}
+__device__ __forceinline__ void perimeter_node(const RunDev &R, int ylo, int yhi, int j, int &x, int &y) {
+  const int ncol = R.xmax > R.xmin ? 2 : 1, side = ncol * (yhi - ylo + 1), nin = R.xmax - R.xmin - 1;
+  if (j < side) {
+    y = ylo + (ncol == 2 ? j >> 1 : j);
+    x = ncol == 2 && (j & 1) ? R.xmax : R.xmin;
+  } else {
+    const int q = j - side;
+    const bool bottom = ylo == R.ymin && q < nin;
+    y = bottom ? R.ymin : R.ymax;
+    x = R.xmin + 1 + (ylo == R.ymin && !bottom ? q - nin : q);
+  }
+}
+
+// One node of the square's perimeter, not the last step of the interval:
+// bounce-back masks, drag terms.  Gather step: P(n, opp k) goes back to the
+// slot S(n,k) came from, unless that lies inside the square (the push is
+// dropped); with the square at a band edge the rows may lie in adjacent bands
+// (shared::cluster addresses), else the three are in this CTA (plain indexing, which the compiler
+// schedules freely).
+template <bool GATHER>
+__device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Band &b, int x, int y, bool edge,
+                                                 const float *map, float feps, bool &bad, float *terms, float *A) {
   const RunDev &R = a.rd;
-  const int W = b.W, H = b.H, rows = b.rows, rowstep = b.rowstep;
-  const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * W, y = b.row0 + ly;
-  const int cm = (x == 0 ? i + W - 1 : i - 1) * 9;
-  const int c0 = i * 9;
-  const int cp = (x == W - 1 ? i - (W - 1) : i + 1) * 9;
-  const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
-  const int mask = (in_box || y == 0 || y == H - 1) ? bounce_mask(R, x, y) : 0;
-  const long long n = (long long)y * W + x;
+  const bool remote = GATHER && edge;  // a local step stays in A
+  const int ly = y - b.row0, rf = b.rowf;
+  const int mask = GATHER ? bounce_mask(R, x, y) : 0;
+  const int co = col_off(b, x);
+  int at[9];  // float offset of slot k's home: in A, or (remote) in the cluster window
+  const int rowC = (remote ? (int)(b.own_c >> 2) : 0) + ly * rf;
+  if (GATHER) {
+    const int cm = col_off(b, x == 0 ? b.W - 1 : x - 1), cp = col_off(b, x == b.W - 1 ? 0 : x + 1);
+    const int rowU = remote && ly == 0 ? (int)(b.prev_c >> 2) + (b.rows_prev - 1) * rf : rowC - rf;
+    const int rowD = remote && ly == b.rows - 1 ? (int)(b.next_c >> 2) : rowC + rf;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {  // S(n,k) = A[n - c_k][opp k], or its own slot
+      const int cx = cx_of(k), cy = cy_of(k);
+      const int row = cy == 1 ? rowU : (cy == -1 ? rowD : rowC), sx = cx == 1 ? cm : (cx == -1 ? cp : co);
+      at[k] = (mask >> k) & 1 ? rowC + co + k * b.ps : row + sx + opp_of(k) * b.ps;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 9; k++) at[k] = rowC + co + k * b.ps;
+  }
+  float S[9], P[9];
+  if (remote) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) S[k] = ld_cluster(4u * (unsigned)at[k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 9; k++) S[k] = A[at[k]];
+  }
+  const float drho = collide_f32_run(R, S, P, map ? map + (long long)y * b.W + x : nullptr, feps);
+  bad |= !(drho > -1.0f);
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const int ok = opp_of(k);
+    bool keep = true;
+    if (GATHER && !((mask >> ok) & 1)) {  // into the square?
+      const int cx = cx_of(k);
+      const int tx = cx == 1 ? (x == b.W - 1 ? 0 : x + 1) : (cx == -1 ? (x == 0 ? b.W - 1 : x - 1) : x);
+      const int ty = y + cy_of(k);
+      keep = !(tx > R.xmin && tx < R.xmax && ty > R.ymin && ty < R.ymax);
+    }
+    if (remote) {
+      if (keep) st_cluster(4u * (unsigned)at[ok], P[k]);
+    } else {
+      if (keep) A[at[ok]] = P[k];
+    }
+  }
+  store_drag_terms<false>(R, S, x, y, b.clone, terms);
+}
+
+// One node of the last step: S_T (and its drag terms), any position.
+__device__ __forceinline__ void store_last(const TemporalArgs &a, const Band &b, const float *A, int x, int ly,
+                                           bool gather, float *terms) {
+  const RunDev &R = a.rd;
+  const int y = b.row0 + ly, rf = b.rowf;
+  const bool box = in_box(R, x, y);
+  const int mask = (box || y == 0 || y == b.H - 1) ? bounce_mask(R, x, y) : 0;
+  const long long n = (long long)y * b.W + x;
   if (mask & 512) {  // inside the square
-    if (last) {
 #pragma unroll
-      for (int k = 0; k < 9; k++) b.dst[k * b.plane + n] = 0.0f;
-    }
+    for (int k = 0; k < 9; k++) b.dst[k * b.plane + n] = 0.0f;
     return;
   }
-  float S[9];
+  const int co = col_off(b, x), cm = col_off(b, x == 0 ? b.W - 1 : x - 1), cp = col_off(b, x == b.W - 1 ? 0 : x + 1);
+  const float *rowC = A + ly * rf;
+  const float *rowU = ly == 0 ? b.prev + (b.rows_prev - 1) * rf : rowC - rf;
+  const float *rowD = ly == b.rows - 1 ? b.next : rowC + rf;
+  float S[9], d = 0.f;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    if (!gather || ((mask >> k) & 1)) {
-      S[k] = A[c0 + k];
-    } else {
-      const int cx = cx_of(k), cy = cy_of(k);
-      const int sxc = cx == 1 ? cm : (cx == -1 ? cp : c0);  // column, row ly
-      const int sl = ly - cy;                                 // source row, band-local
-      const float *base = sl < 0 ? b.prev : (sl >= rows ? b.next : A);
-      const int roff = sl < 0 ? (b.rows_prev - 1 - ly) * rowstep : (sl >= rows ? -ly * rowstep : -cy * rowstep);
-      S[k] = base[sxc + roff + opp_of(k)];
-    }
+    const int cx = cx_of(k), cy = cy_of(k);
+    const float *row = cy == 1 ? rowU : (cy == -1 ? rowD : rowC);
+    const int sx = cx == 1 ? cm : (cx == -1 ? cp : co);
+    S[k] = (!gather || ((mask >> k) & 1)) ? rowC[co + k * b.ps] : row[sx + opp_of(k) * b.ps];
   }
-  if (in_box) store_drag_terms<false>(R, S, x, y, b.clone, terms);
-  if (last) {
-    float d = 0.f;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      b.dst[k * b.plane + n] = S[k];
-      d += S[k];
-    }
-    if (!(d > -1.0f)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
-    return;
-  }
-  const float *fm = (R.field_mode && t + 1 < R.field_steps && a.maps)
-                        ? a.maps + R.map_base + (long long)b.clone * R.nodes + n
-                        : nullptr;
-  float P[9];
-  const float drho = collide_f32_run(R, S, P, fm, R.f_field_eps);
-  if (!(drho > -1.0f)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
+  if (box) store_drag_terms<false>(R, S, x, y, b.clone, terms);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const int ok = opp_of(k);
-    if (!gather || ((mask >> ok) & 1)) {
-      A[c0 + ok] = P[k];
-    } else {
-      const int cx = cx_of(k), cy = cy_of(k);
-      const int tx = cx == 1 ? (x == W - 1 ? 0 : x + 1) : (cx == -1 ? (x == 0 ? W - 1 : x - 1) : x);
-      const int ty = y + cy;
-      if (ty < 0 || ty >= H) continue;
-      if (tx > R.xmin && tx < R.xmax && ty > R.ymin && ty < R.ymax) continue;  // into the square
-      const int txc = cx == 1 ? cp : (cx == -1 ? cm : c0);
-      const int tl = ly + cy;
-      float *base = tl < 0 ? b.prev : (tl >= rows ? b.next : A);
-      const int roff = tl < 0 ? (b.rows_prev - 1 - ly) * rowstep : (tl >= rows ? -ly * rowstep : cy * rowstep);
-      base[txc + roff + k] = P[k];
-    }
+    b.dst[k * b.plane + n] = S[k];
+    d += S[k];
   }
-}
-
-// update_general for a gather step that is not the last: every slot the node
-// reads is addressed once (32-bit shared::cluster address: this CTA, or the
-// neighbour CTA across a band edge), and P(n,k) goes back to the slot S(n,
-// opp k) came from -- the pull rules make the two the same slot (own slot opp
-// k when that slot bounces, else (n + c_k, k)) -- unless the target row lies
-// outside the channel or the target inside the square (the push is dropped,
-// as in update_general).  PLAIN: a node off the walls and the square's box
-// (a band-edge row): nothing bounces back and no push is dropped, only the
-// neighbour rows may lie in the adjacent CTAs.  LOCAL: the node's row and
-// both neighbour rows are in this CTA (1 <= ly <= rows - 2): the same slots
-// through plain shared-memory indexing of A, which the compiler schedules
-// freely (the shared::cluster accesses are ordered asm).
-template <bool PLAIN = false, bool LOCAL = false>
-__device__ __forceinline__ void update_general_gather(const TemporalArgs &a, const Band &b, int i, int t,
-                                                      bool &bad, float *terms, float *A = nullptr) {
-  const RunDev &R = a.rd;
-  const int W = b.W, H = b.H, rows = b.rows, rs = b.rowstep;
-  const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * W, y = b.row0 + ly;
-  const int xm = x == 0 ? W - 1 : x - 1, xp = x == W - 1 ? 0 : x + 1;
-  const bool in_box = !PLAIN && x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
-  const int mask = (!PLAIN && (in_box || y == 0 || y == H - 1)) ? bounce_mask(R, x, y) : 0;
-  if (mask & 512) return;  // inside the square
-  // byte addresses of column 0 of the rows y-1, y, y+1
-  const unsigned rowC = b.own_c + 4u * (unsigned)(ly * rs);
-  const unsigned rowU = ly == 0 ? b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rs) : rowC - 4u * (unsigned)rs;
-  const unsigned rowD = ly == rows - 1 ? b.next_c : rowC + 4u * (unsigned)rs;
-  const unsigned own = rowC + 36u * (unsigned)x;
-  unsigned ad[9];
-  float S[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    if ((mask >> k) & 1) {
-      ad[k] = own + 4u * k;
-    } else {  // S(n,k) = A[n - c_k][opp k]
-      const int cx = cx_of(k), cy = cy_of(k);
-      const int sx = cx == 1 ? xm : (cx == -1 ? xp : x);
-      const unsigned row = cy == 1 ? rowU : (cy == -1 ? rowD : rowC);
-      ad[k] = row + 36u * (unsigned)sx + 4u * opp_of(k);
-    }
-    if (LOCAL)
-      S[k] = A[(ad[k] - b.own_c) >> 2];
-    else
-      S[k] = ld_cluster(ad[k]);
-  }
-  if (in_box) store_drag_terms<false>(R, S, x, y, b.clone, terms);
-  const long long n = (long long)y * W + x;
-  const float *fm = (R.field_mode && t + 1 < R.field_steps && a.maps)
-                        ? a.maps + R.map_base + (long long)b.clone * R.nodes + n
-                        : nullptr;
-  float P[9];
-  const float drho = collide_f32_run(R, S, P, fm, R.f_field_eps);
-  bad |= !(drho > -1.0f);
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    const int ok = opp_of(k);
-    if (!PLAIN && !((mask >> ok) & 1)) {
-      const int cx = cx_of(k), cy = cy_of(k);
-      const int tx = cx == 1 ? xp : (cx == -1 ? xm : x);
-      const int ty = y + cy;
-      if (ty < 0 || ty >= H) continue;
-      if (tx > R.xmin && tx < R.xmax && ty > R.ymin && ty < R.ymax) continue;  // into the square
-    }
-    if (LOCAL)
-      A[(ad[ok] - b.own_c) >> 2] = P[k];
-    else
-      st_cluster(ad[ok], P[k]);
-  }
-}
-
-// update_general for a local step that is not the last: the node swaps its
-// own slots; only the square's box needs more (drag terms, the interior).
-__device__ __forceinline__ void update_general_local(const TemporalArgs &a, const Band &b, float *A, int i,
-                                                     int t, bool &bad, float *terms) {
-  const RunDev &R = a.rd;
-  const int W = b.W;
-  const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * W, y = b.row0 + ly;
-  const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
-  if (in_box && (bounce_mask(R, x, y) & 512)) return;  // inside the square
-  const int c0 = i * 9;
-  float S[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) S[k] = A[c0 + k];
-  if (in_box) store_drag_terms<false>(R, S, x, y, b.clone, terms);
-  const long long n = (long long)y * W + x;
-  const float *fm = (R.field_mode && t + 1 < R.field_steps && a.maps)
-                        ? a.maps + R.map_base + (long long)b.clone * R.nodes + n
-                        : nullptr;
-  float P[9];
-  const float drho = collide_f32_run(R, S, P, fm, R.f_field_eps);
-  bad |= !(drho > -1.0f);
-#pragma unroll
-  for (int k = 0; k < 9; k++) A[c0 + opp_of(k)] = P[k];
+  if (!(d > -1.0f)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
 }
 
 __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::cluster_group &cluster) {
@@ -233,11 +389,14 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
   b.clone = blockIdx.x / b.cs;
   b.W = a.rd.W;
   b.H = a.rd.H;
+  b.Wh = (b.W + 1) / 2;
+  b.div_wh = a.div_wh;
   b.row0 = a.band_row0[b.rank];
   b.rows = a.band_row0[b.rank + 1] - b.row0;
   b.rows_prev = b.rank > 0 ? b.row0 - a.band_row0[b.rank - 1] : b.rows;
-  b.nb = b.rows * b.W;
-  b.rowstep = b.W * 9;
+  b.np = b.rows * b.Wh;
+  b.ps = 2 * b.Wh;
+  b.rowf = 9 * b.ps;
   b.prev = b.rank > 0 ? cluster.map_shared_rank(A, b.rank - 1) : A;
   b.next = b.rank + 1 < b.cs ? cluster.map_shared_rank(A, b.rank + 1) : A;
   const unsigned a_cta = (unsigned)__cvta_generic_to_shared(A);
@@ -248,147 +407,37 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
   const long long cb = a.rd.pop_base + (long long)b.clone * 9 * b.plane;
   b.src = a.src + cb;
   b.dst = a.dst + cb;
+  // opaque: held in registers, not worked out again from the lattice width
+  asm volatile("" : "+r"(b.ps), "+r"(b.rowf), "+r"(b.Wh), "+r"(b.div_wh), "+r"(b.np));
   return b;
 }
 
-// P_0 into the "after a local step" layout A[node*9 + opp k]
-template <int THREADS>
-__device__ __forceinline__ void load_band(const Band &b, float *A) {
-  for (int i = threadIdx.x; i < b.nb; i += THREADS) {
-    const long long n = (long long)b.row0 * b.W + i;
-#pragma unroll
-    for (int k = 0; k < 9; k++) A[i * 9 + opp_of(k)] = b.src[k * b.plane + n];
-  }
-}
-
-// P_0 formed here from the previous interval's S (fused reseed: parent copy,
-// perturbation, first collision; the same per-node function as the reseed
-// kernel, so bit-identical), in the same layout.  Square-interior nodes get
-// zeros: their slots are never read before the last step writes them.
-template <int THREADS>
-__device__ __forceinline__ void load_band_reseed(const TemporalArgs &a, const Band &b, float *A) {
+// P_0 into the "after a local step" layout A[n][opp k].  FUSED: formed here
+// from the previous interval's S (parent copy, perturbation, first collision;
+// the same per-node function as the reseed kernel, so bit-identical).
+// Square-interior nodes and the empty lane of an odd width's last pair get
+// zeros (the fluid at rest).
+template <int THREADS, bool FUSED>
+__device__ __forceinline__ void load_band(const TemporalArgs &a, const Band &b, float *A) {
   const RunDev &R = a.rd;
-  for (int i = threadIdx.x; i < b.nb; i += THREADS) {
-    const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * b.W, y = b.row0 + ly;
+#pragma unroll 1
+  for (int j = threadIdx.x; j < 2 * b.np; j += THREADS) {
+    const int h = j >= b.np, i = h ? j - b.np : j;
+    const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = i - ly * b.Wh, x = xh + h * b.Wh, y = b.row0 + ly;
     float P[9];
-    if (x > R.xmin && x < R.xmax && y > R.ymin && y < R.ymax) {
+    if (x >= b.W || (FUSED && x > R.xmin && x < R.xmax && y > R.ymin && y < R.ymax)) {
 #pragma unroll
       for (int k = 0; k < 9; k++) P[k] = 0.0f;
-    } else {
+    } else if (FUSED) {
       reseed_node<false>(a.rs, R, a.run, b.clone, x, y, y * b.W + x, P);
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k++) A[i * 9 + opp_of(k)] = P[k];
-  }
-}
-
-// One node away from the square, not the last step of the interval.  C, U,
-// D = the node's row and the rows above (y-1) and below (y+1); om, o0, op =
-// the column offsets of x-1, x, x+1 (times 9).  GATHER: S(n,k) = A[n -
-// c_k][opp k], P(n,k) -> A[n + c_k][k]; local step: S(n,k) = A[n][k], P(n,k)
-// -> A[n][opp k].  WALL (gather step): 1 = the bottom wall y = 0, whose
-// slots 2, 5, 6 bounce back (S(n,k) = A[n][k], and P(n, opp k) returns
-// there); 2 = the top wall y = H - 1, slots 4, 7, 8; the row beyond the wall
-// is not touched.  FIELD: beta scaled by (1 + feps * map[0]), feps = 0 once
-// the field's steps are over (field_beta_f32 then returns beta exactly).  A
-// density at or below zero sets `bad`.
-template <bool GATHER, bool FIELD, int WALL = 0>
-__device__ __forceinline__ void update_fast(const RunDev &R, float *C, float *U, float *D, int om, int o0,
-                                            int op, const float *map, float feps, bool &bad) {
-  float S[9];
-  if (GATHER) {
-    S[0] = C[o0 + 0];
-    S[1] = C[om + 3];
-    S[3] = C[op + 1];
-    S[2] = WALL == 1 ? C[o0 + 2] : U[o0 + 4];
-    S[5] = WALL == 1 ? C[o0 + 5] : U[om + 7];
-    S[6] = WALL == 1 ? C[o0 + 6] : U[op + 8];
-    S[4] = WALL == 2 ? C[o0 + 4] : D[o0 + 2];
-    S[7] = WALL == 2 ? C[o0 + 7] : D[op + 5];
-    S[8] = WALL == 2 ? C[o0 + 8] : D[om + 6];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 9; k++) S[k] = C[o0 + k];
-  }
-  float P[9];
-  const float drho = collide_f32_run(R, S, P, FIELD ? map : nullptr, feps);
-  bad |= !(drho > -1.0f);
-  if (GATHER) {
-    C[o0 + 0] = P[0];
-    C[op + 1] = P[1];
-    C[om + 3] = P[3];
-    if (WALL == 2) {
-      C[o0 + 4] = P[2];
-      C[o0 + 7] = P[5];
-      C[o0 + 8] = P[6];
     } else {
-      D[o0 + 2] = P[2];
-      D[op + 5] = P[5];
-      D[om + 6] = P[6];
-    }
-    if (WALL == 1) {
-      C[o0 + 2] = P[4];
-      C[o0 + 5] = P[7];
-      C[o0 + 6] = P[8];
-    } else {
-      U[o0 + 4] = P[4];
-      U[om + 7] = P[7];
-      U[op + 8] = P[8];
-    }
-  } else {
+      const long long n = (long long)y * b.W + x;
 #pragma unroll
-    for (int k = 0; k < 9; k++) C[o0 + opp_of(k)] = P[k];
-  }
-}
-
-// A gather step of one node of a band-edge row (the band holds at least two
-// rows): UP, the row above (y - 1) is the previous CTA's last row; else the
-// row below (y + 1) is the next CTA's first row.  The remote row's slots are
-// read and written at 32-bit shared::cluster addresses (Rc = that row's
-// column 0), the node's own row C and the other neighbour row L in this CTA's
-// shared memory; same slots and arithmetic as update_fast.
-template <bool FIELD, bool UP>
-__device__ __forceinline__ void update_edge(const RunDev &R, float *C, float *L, unsigned Rc, int om, int o0,
-                                            int op, const float *map, float feps, bool &bad) {
-  float S[9];
-  S[0] = C[o0 + 0];
-  S[1] = C[om + 3];
-  S[3] = C[op + 1];
-  if (UP) {
-    S[4] = L[o0 + 2];
-    S[7] = L[op + 5];
-    S[8] = L[om + 6];
-    S[2] = ld_cluster(Rc + 4u * (o0 + 4));
-    S[5] = ld_cluster(Rc + 4u * (om + 7));
-    S[6] = ld_cluster(Rc + 4u * (op + 8));
-  } else {
-    S[2] = L[o0 + 4];
-    S[5] = L[om + 7];
-    S[6] = L[op + 8];
-    S[4] = ld_cluster(Rc + 4u * (o0 + 2));
-    S[7] = ld_cluster(Rc + 4u * (op + 5));
-    S[8] = ld_cluster(Rc + 4u * (om + 6));
-  }
-  float P[9];
-  const float drho = collide_f32_run(R, S, P, FIELD ? map : nullptr, feps);
-  bad |= !(drho > -1.0f);
-  C[o0 + 0] = P[0];
-  C[op + 1] = P[1];
-  C[om + 3] = P[3];
-  if (UP) {
-    L[o0 + 2] = P[2];
-    L[op + 5] = P[5];
-    L[om + 6] = P[6];
-    st_cluster(Rc + 4u * (o0 + 4), P[4]);
-    st_cluster(Rc + 4u * (om + 7), P[7]);
-    st_cluster(Rc + 4u * (op + 8), P[8]);
-  } else {
-    L[o0 + 4] = P[4];
-    L[om + 7] = P[7];
-    L[op + 8] = P[8];
-    st_cluster(Rc + 4u * (o0 + 2), P[2]);
-    st_cluster(Rc + 4u * (op + 5), P[5]);
-    st_cluster(Rc + 4u * (om + 6), P[6]);
+      for (int k = 0; k < 9; k++) P[k] = b.src[k * b.plane + n];
+    }
+    float *o = A + ly * b.rowf + 2 * xh + h;
+#pragma unroll
+    for (int k = 0; k < 9; k++) o[opp_of(k) * b.ps] = P[k];
   }
 }
 
@@ -397,118 +446,304 @@ __device__ __forceinline__ float field_eps(const TemporalArgs &a, int t) {
 }
 
 // Shared memory of one CTA: the band's populations, then the segment list,
-// one class byte per 32-node segment and the five range ends of the list.
+// one class byte per segment and the ends of the list's ranges.  temporal_smem
+// (a function of the nodes alone) is what a shape is accepted by; pair_smem
+// what a band takes: the same populations for an even width, one node more per
+// row for an odd one.
 __host__ __device__ inline size_t temporal_smem(int nb) {
   const int nseg = (nb + 31) / 32;
   return sizeof(float) * 9 * (size_t)nb + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
 }
-
-// One step of every segment of the band (all but the interval's last step).
-// The list holds the segments by class, in this order: the square's box (and
-// a partial last segment, and wall or band-edge segments that span two rows
-// at a wall), the wall rows, the band-edge rows, other segments spanning two
-// rows at a band edge, the bulk segments with the periodic wrap and the
-// interior bulk segments; range[c] = the end of the c-th range, and entry k
-// of every range belongs to warp k % NW.  Gather step: the box range through
-// the general path; wall rows through update_fast with the wall's bounce-back
-// built in; band-edge rows with the neighbour row across the band edge at
-// shared::cluster addresses and the rest in this CTA; rows spanning a band
-// edge through the plain form of the general path (no bounce-back, every
-// slot at a shared::cluster address); wrap segments with per-node column
-// offsets; interior segments with their nine slots at constant offsets from
-// the node's own (-9 / +9 floats for x -+ 1, -+ rowstep for y -+ 1).  Local
-// step: a node touches only its own nine slots, so only the box range (drag
-// terms, the interior) needs the general path.
-// LOCAL_BOX: box segments whose rows all lie inside the band take the
-// general gather through plain shared-memory indexing (compiled into the
-// uniform-force kernels only: in the random-field ones it raised register
-// spills).
-template <int NW, bool GATHER, bool FIELD, bool LOCAL_BOX>
-__device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, float *A,
-                                          const unsigned short *list, int nseg, const int *range,
-                                          int warp, int lane, int t, const float *map, bool &bad) {
-  const RunDev &R = a.rd;
-  const float feps = FIELD ? field_eps(a, t) : 0.0f;
-  float *terms = a.terms + (long long)t * a.term_slab + R.term_base;
-  const int ngen = range[0];
-  for (int k = warp; k < ngen; k += NW) {
-    const int i = list[k] * 32 + lane;
-    const int ly = (int)__umulhi((unsigned)i, R.div_w);
-    const bool inner = LOCAL_BOX && __all_sync(0xffffffffu, i < b.nb && ly >= 1 && ly <= b.rows - 2);
-    if (i >= b.nb) continue;
-    if (GATHER) {
-      if (inner)
-        update_general_gather<false, true>(a, b, i, t, bad, terms, A);
-      else
-        update_general_gather(a, b, i, t, bad, terms);
-    } else {
-      update_general_local(a, b, A, i, t, bad, terms);
-    }
-  }
-  if (!GATHER) {
-    for (int k = ngen + ((warp - ngen) & (NW - 1)); k < nseg; k += NW) {
-      const int i = list[k] * 32 + lane;
-      float *C = A + i * 9;
-      update_fast<false, FIELD>(R, C, C, C, 0, 0, 0, map + i, feps, bad);
-    }
-    return;
-  }
-  const int rs = b.rowstep;
-  const int nwall = range[1], nedge = range[2], nspan = range[3], nwrap = range[4];
-  for (int k = ngen + ((warp - ngen) & (NW - 1)); k < nwall; k += NW) {
-    const int i = list[k] * 32 + lane;
-    const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * b.W;
-    const int o0 = x * 9, om = (x == 0 ? b.W - 1 : x - 1) * 9, op = (x == b.W - 1 ? 0 : x + 1) * 9;
-    float *C = A + ly * rs;
-    if (b.row0 + ly == 0)  // warp-uniform: a wall segment lies in one row
-      update_fast<true, FIELD, 1>(R, C, C - rs, C + rs, om, o0, op, map + i, feps, bad);
-    else
-      update_fast<true, FIELD, 2>(R, C, C - rs, C + rs, om, o0, op, map + i, feps, bad);
-  }
-  for (int k = nwall + ((warp - nwall) & (NW - 1)); k < nedge; k += NW) {
-    const int i = list[k] * 32 + lane;
-    const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * b.W;
-    const int o0 = x * 9, om = (x == 0 ? b.W - 1 : x - 1) * 9, op = (x == b.W - 1 ? 0 : x + 1) * 9;
-    float *C = A + ly * rs;
-    if (ly == 0)  // warp-uniform: an edge segment lies in one row
-      update_edge<FIELD, true>(R, C, C + rs, b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rs), om, o0, op,
-                               map + i, feps, bad);
-    else
-      update_edge<FIELD, false>(R, C, C - rs, b.next_c, om, o0, op, map + i, feps, bad);
-  }
-  for (int k = nedge + ((warp - nedge) & (NW - 1)); k < nspan; k += NW)
-    update_general_gather<true>(a, b, list[k] * 32 + lane, t, bad, terms);
-  for (int k = nspan + ((warp - nspan) & (NW - 1)); k < nwrap; k += NW) {
-    const int i = list[k] * 32 + lane;
-    const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * b.W;
-    const int o0 = x * 9, om = (x == 0 ? b.W - 1 : x - 1) * 9, op = (x == b.W - 1 ? 0 : x + 1) * 9;
-    float *C = A + ly * rs;
-    update_fast<true, FIELD>(R, C, C - rs, C + rs, om, o0, op, map + i, feps, bad);
-  }
-  for (int k = nwrap + ((warp - nwrap) & (NW - 1)); k < nseg; k += NW) {
-    const int i = list[k] * 32 + lane;
-    float *C = A + i * 9;
-    update_fast<true, FIELD>(R, C, C - rs, C + rs, -9, 0, 9, map + i, feps, bad);
-  }
+// segments of 32 pairs: the first and the last row by themselves, then the
+// rows between them
+__host__ __device__ inline int segment_count(int rows, int Wh) {
+  const int spr = (Wh + 31) / 32;
+  return rows == 1 ? spr : 2 * spr + ((rows - 2) * Wh + 31) / 32;
+}
+__host__ __device__ inline size_t pair_smem(int rows, int W) {
+  const int Wh = (W + 1) / 2, nseg = segment_count(rows, Wh);
+  return 8 * 9 * (size_t)rows * Wh + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
 }
 
-// Generic kernel: any W.  The band's nodes form 32-node segments; segments
-// that cost more than a bulk segment (the square's box on the general path,
-// then walls and band edges) are dealt out first, one per warp, and the bulk
-// segments fill in after them: entry k of the list goes to warp k % NW.  The
-// step time is that of the slowest warp (every step ends at a cluster
-// barrier), which this keeps near the mean.  (Measured on a 256x64 channel,
-// all slower than this: band-edge and wall rows through generic
-// distributed-shared-memory pointers, a cost-weighted water-filling of the
-// bulk segments over the warps, a fixed column per thread with compile-time
-// shared-memory offsets, segments taken from a shared counter in one
-// dispatch loop, the band geometry in shared memory.)
+// Segment classes, in the order of the list.
+enum : int { SEG_GENERAL = 0, SEG_EDGE, SEG_WALL, SEG_BOX, SEG_PART, SEG_INNER, SEG_CLASSES };
+
+// Split cluster barrier: a thread arrives once it has done its share of what
+// the neighbouring bands wait for, and waits before it next touches theirs.
+// (A warp that wrote nothing the neighbours read has nothing to release.)
+__device__ __forceinline__ void cluster_arrive(bool release) {
+  __syncwarp();  // the aligned form takes whole warps
+  if (release)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  else
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// One step of the band (all but the interval's last step).  Work comes in
+// warp-sized entries, dealt out in this order:
+//   seam    (gather) the seam pairs of the first and the last row, every slot
+//           at a per-lane shared::cluster address
+//   GENERAL segments of a one-row band, or where the square touches a
+//           band-edge row: the same path
+//   EDGE    a band-edge row, the row across the edge at shared::cluster
+//           addresses
+//   perimeter  32 nodes of the square's perimeter, one per lane
+//           (bounce-back, drag terms)
+//   seam    (gather) 32 seam pairs of the rows between, per-lane addresses
+//   WALL    a wall row, bounce-back built in
+//   BOX     segments with nodes of the square: as INNER, lanes in the square
+//           not written
+//   PART    as INNER, but partial or with seam pairs (left out) in it
+//   INNER   every slot pair one 64-bit access at a constant offset
+// In a local step a node touches only its own slots, the seam included.  The
+// deal is round robin, except that the warps holding the first kinds, up to
+// the perimeter, sit out one round: those wait on the neighbour's memory, or
+// take one node per lane through the drag's divisions.
+// Neighbouring bands wait only for nodes of the rows at their common edge:
+// once a warp's entries up to there are done it arrives at the cluster
+// barrier, and it waits for it at the start of the next step, by which time
+// the others have long arrived.  Within the CTA a block barrier ends the step.
+// The drag terms' global stores come after the arrival, whose release would
+// wait for them (unless the square touches an edge row).
+// What a warp keeps of the deal between steps, [0] local, [1] gather: its
+// first entry after the head (an index into the list; a gather step's inner
+// seam entries come before the list, at nedge - einner and up) and the
+// distance to its second one, and what the head holds for it.
+struct WarpPlan {
+  int k[2], dk[2];
+  int nbox, npart, nseg;
+  unsigned flags;
+};
+enum : unsigned {
+  PLAN_HEAD = 1u,       // entries ahead of the arrival (<< 1: in a gather step)
+  PLAN_PERIMETER = 4u,  // perimeter entries (<< 1: in a gather step)
+  PLAN_BOX_EDGE = 16u,  // the square touches a row at a band edge
+};
+
+// The head of the deal in a step of one kind.
+struct Head {
+  int ns, nouter, ninner;        // seam pairs per row; of the first and last row, of those between
+  int eouter, einner, eper;      // their entries, the perimeter's
+  int ylo, yhi, nper;
+  bool box_edge;
+  __device__ __forceinline__ Head(const RunDev &R, const Band &b, bool gather) {
+    ns = seam_count(b);
+    nouter = gather ? ns * min(b.rows, 2) : 0;
+    ninner = gather ? ns * max(b.rows - 2, 0) : 0;
+    eouter = (nouter + 31) / 32;
+    einner = (ninner + 31) / 32;
+    ylo = max(R.ymin, b.row0);
+    yhi = min(R.ymax, b.row0 + b.rows - 1);
+    nper = perimeter_count(R, ylo, yhi);
+    eper = (nper + 31) / 32;
+    box_edge = yhi >= ylo &&
+               ((ylo == b.row0 && b.rank > 0) || (yhi == b.row0 + b.rows - 1 && b.rank + 1 < b.cs));
+  }
+};
+
+// The warp's plan, from the class ends of the list.
+template <int NW>
+__device__ __forceinline__ WarpPlan warp_plan(const RunDev &R, const Band &b, const int *range, int warp) {
+  WarpPlan p;
+  p.nbox = range[SEG_BOX];
+  p.npart = range[SEG_PART];
+  p.nseg = range[SEG_INNER];
+  p.flags = 0;
+  const int nedge = range[SEG_EDGE];
+#pragma unroll
+  for (int g = 0; g < 2; g++) {
+    const Head h(R, b, g);
+    const int lead = h.eouter + nedge, nhead = lead + h.eper;
+    // positions NW .. NW + nhead - 1 of the round robin are left out
+    const int q = nhead >= NW ? (warp - nhead % NW + NW) % NW : (warp >= nhead ? warp - nhead : 2 * (NW - nhead) + warp);
+    p.k[g] = q - h.einner + nedge;
+    p.dk[g] = nhead < NW && warp >= nhead ? NW - nhead : NW;
+    if (warp < lead) p.flags |= PLAN_HEAD << g;
+    if (h.nper > 0 && (warp - lead % NW + NW) % NW < h.eper) p.flags |= PLAN_PERIMETER << g;
+    if (h.box_edge) p.flags |= PLAN_BOX_EDGE;
+  }
+  // opaque: held in registers over the steps, not worked out again in each
+#pragma unroll
+  for (int g = 0; g < 2; g++) asm volatile("" : "+r"(p.k[g]), "+r"(p.dk[g]));
+  asm volatile("" : "+r"(p.nbox), "+r"(p.npart), "+r"(p.nseg), "+r"(p.flags));
+  return p;
+}
+
+template <int NW, bool GATHER, bool FIELD>
+__device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, const WarpPlan &w, float *A,
+                                          const unsigned short *list, const int *range, int warp, int lane, int t,
+                                          const float *map, bool &bad) {
+  const RunDev &R = a.rd;
+  const float feps = FIELD ? field_eps(a, t) : 0.0f;
+  const int ps = b.ps, rf = b.rowf;
+  // the pair of segment position i: its row and column, inactive past `lim`
+#define CLBM_PAIR(lim)                                                                         \
+  const int i = list[k] + lane;                                                                \
+  if (i >= (lim)) continue;                                                                    \
+  const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = pair_of(b, i - ly * b.Wh), y = b.row0 + ly
+  auto general = [&](int ly, int xh) {
+    const int y = b.row0 + ly;
+    const RowC C{b.own_c + 4u * (unsigned)(ly * rf)};
+    const bool wb = y == 0, wt = y == b.H - 1;
+    const RowC U{wb ? C.a : (ly == 0 ? b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf) : C.a - 4u * (unsigned)rf)};
+    const RowC D{wt ? C.a : (ly == b.rows - 1 ? b.next_c : C.a + 4u * (unsigned)rf)};
+    gather_pair<FIELD, false, 3, true>(R, ps, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh, feps), bad,
+                                       in_box(R, xh, y), in_box(R, xh + b.Wh, y), wb, wt);
+  };
+  auto local = [&](int ly, int xh, auto pred) {
+    const int y = b.row0 + ly;
+    constexpr bool P = decltype(pred)::value;
+    local_pair<P>(R, ps, A + ly * rf + 2 * xh, pair_force<FIELD>(R, b, map, y, xh, feps), bad, P && in_box(R, xh, y),
+                  P && in_box(R, xh + b.Wh, y));
+  };
+  const bool lead = w.flags & (PLAN_HEAD << GATHER);
+  if (b.cs > 1) cluster_wait();
+  // ---- what the neighbouring bands wait for
+  if (lead) {
+    const int nedge = range[SEG_EDGE];
+    int e = warp;  // this warp's next entry, counted within the kind at hand
+    if (GATHER) {
+      const Head h(R, b, true);
+#pragma unroll 1
+      for (; e < h.eouter; e += NW) {
+        const int j = e * 32 + lane;
+        if (j >= h.nouter) continue;
+        const int last = j >= h.ns;
+        general(last ? b.rows - 1 : 0, seam_pair(b, last ? j - h.ns : j));
+      }
+      e -= h.eouter;
+      const int ngen = range[SEG_GENERAL];
+#pragma unroll 1
+      for (; e < ngen; e += NW) {
+        const int k = e;
+        CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
+        if (!on_seam(b, xh)) general(y - b.row0, xh);
+      }
+#pragma unroll 1
+      for (; e < nedge; e += NW) {
+        const int k = e;
+        CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
+        if (on_seam(b, xh)) continue;
+        float *C = A + ly * rf;
+        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh, feps);
+        if (ly == 0)  // warp-uniform
+          gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowC{b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf)},
+                                             RowL{C + rf}, cols_inner(xh), f, bad);
+        else
+          gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowC{b.next_c}, cols_inner(xh), f, bad);
+      }
+    } else {
+#pragma unroll 1
+      for (; e < nedge; e += NW) {
+        const int k = e;
+        CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
+        local(y - b.row0, xh, std::integral_constant<bool, true>());
+      }
+    }
+  }
+  // ---- the perimeter before the arrival if it is part of that, else after it
+  const bool box_edge = w.flags & PLAN_BOX_EDGE;
+  if (b.cs > 1 && !box_edge) cluster_arrive(lead);
+  if (w.flags & (PLAN_PERIMETER << GATHER)) {
+    const Head h(R, b, GATHER);
+    float *terms = a.terms + (long long)t * a.term_slab + R.term_base;
+#pragma unroll 1
+    for (int e = (warp - (h.eouter + range[SEG_EDGE]) % NW + NW) % NW; e < h.eper; e += NW) {
+      const int j = e * 32 + lane;
+      if (j >= h.nper) continue;
+      int x, y;
+      perimeter_node(R, h.ylo, h.yhi, j, x, y);
+      perimeter_update<GATHER>(a, b, x, y, box_edge, FIELD ? map : nullptr, feps, bad, terms, A);
+    }
+  }
+  if (b.cs > 1 && box_edge) cluster_arrive(true);
+  // ---- the rest
+  int k = w.k[GATHER], dk = w.dk[GATHER];
+  auto step = [&]() {
+    k += dk;
+    dk = NW;
+  };
+  if (k < w.nbox) {
+    const int nwall = range[SEG_WALL], top = b.np - b.Wh;  // first pair of the last row
+    if (GATHER) {
+      const int ns = seam_count(b), ninner = ns * max(b.rows - 2, 0), nedge = range[SEG_EDGE];
+#pragma unroll 1
+      for (; k < nedge; step()) {
+        const int j = (k - nedge + (ninner + 31) / 32) * 32 + lane;
+        if (j >= ninner) continue;
+        const int r = ns == 2 ? j >> 1 : j / 3, ly = r + 1, xh = seam_pair(b, j - ns * r), y = b.row0 + ly;
+        float *C = A + ly * rf;
+        gather_pair<FIELD, false, 0, true>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_any(b, xh),
+                                           pair_force<FIELD>(R, b, map, y, xh, feps), bad, in_box(R, xh, y),
+                                           in_box(R, xh + b.Wh, y));
+      }
+#pragma unroll 1
+      for (; k < nwall; step()) {
+        CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
+        if (on_seam(b, xh)) continue;
+        float *C = A + ly * rf;
+        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh, feps);
+        if (y == 0)  // warp-uniform
+          gather_pair<FIELD, true, 1, false>(R, ps, RowL{C}, RowL{C}, RowL{C + rf}, cols_inner(xh), f, bad);
+        else
+          gather_pair<FIELD, true, 2, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C}, cols_inner(xh), f, bad);
+      }
+#pragma unroll 1
+      for (; k < w.nbox; step()) {
+        CLBM_PAIR(top);
+        if (on_seam(b, xh)) continue;
+        float *C = A + ly * rf;
+        gather_pair<FIELD, true, 0, true>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                          pair_force<FIELD>(R, b, map, y, xh, feps), bad, in_box(R, xh, y),
+                                          in_box(R, xh + b.Wh, y));
+      }
+    } else {
+#pragma unroll 1
+      for (; k < w.nbox; step()) {
+        CLBM_PAIR(k < nwall ? (list[k] < b.Wh ? b.Wh : b.np) : top);
+        local(y - b.row0, xh, std::integral_constant<bool, true>());
+      }
+    }
+  }
+#pragma unroll 1
+  for (; k < w.npart; step()) {
+    CLBM_PAIR(b.np - b.Wh);
+    if (GATHER) {
+      if (on_seam(b, xh)) continue;
+      float *C = A + ly * rf;
+      gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                         pair_force<FIELD>(R, b, map, y, xh, feps), bad);
+    } else {
+      local(ly, xh, std::integral_constant<bool, false>());
+    }
+  }
+#pragma unroll 1
+  for (; k < w.nseg; step()) {
+    const int i = list[k] + lane;
+    const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = i - ly * b.Wh - 1;
+    // the pair itself: the slots lie at offsets from here that are the same
+    // for every pair of the band
+    float *C = A + ly * rf + 2 * xh;
+    const F32Force2 f = pair_force<FIELD>(R, b, map, b.row0 + ly, xh, feps);
+    if (GATHER)
+      gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(0), f, bad);
+    else
+      local_pair<false>(R, ps, C, f, bad);
+  }
+#undef CLBM_PAIR
+  __syncthreads();
+}
+
 template <int THREADS, int MINB, bool FIELD>
 __global__ void __launch_bounds__(THREADS, MINB) k_temporal_f32(TemporalArgs a) {
-  // A[node * 9 + k]: a node's nine values together (stride 9 words: no bank
-  // conflicts across a warp), so every access is a base register plus an
-  // immediate offset
-  extern __shared__ float A[];
+  // A[row][k][pair]: a warp's accesses to one population are consecutive 64-bit
+  // words, in this CTA (no bank conflicts) and across a band edge (whole
+  // sectors on the way to the other SM)
+  extern __shared__ __align__(16) float A[];
   constexpr int NW = THREADS / 32;
   cg::cluster_group cluster = cg::this_cluster();
   const Band b = make_band(a, A, cluster);
@@ -516,84 +751,83 @@ __global__ void __launch_bounds__(THREADS, MINB) k_temporal_f32(TemporalArgs a) 
   // (the fused load is compiled into the uniform-force kernels only: in the
   // random-field ones it raised register spills in the step loop)
   if (!FIELD && a.fused)
-    load_band_reseed<THREADS>(a, b, A);
+    load_band<THREADS, true>(a, b, A);
   else
-    load_band<THREADS>(b, A);
-  const int nseg = (b.nb + 31) / 32;
-  unsigned short *list = (unsigned short *)(A + (size_t)9 * b.nb);
+    load_band<THREADS, false>(a, b, A);
+  const int nseg = segment_count(b.rows, b.Wh), spr = (b.Wh + 31) / 32;
+  unsigned short *list = (unsigned short *)(A + (size_t)18 * b.np);
   unsigned char *cls = (unsigned char *)(list + ((nseg + 7) & ~7));
-  int *count_s = (int *)(cls + ((nseg + 15) & ~15));
+  int *range = (int *)(cls + ((nseg + 15) & ~15));
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  // segment classes: 5 touches the square's box, or past the band's end
-  // (partial last segment), or a wall row that is not alone in its segment or
-  // in its band; 4 a wall row (its neighbour row in this CTA); 3 a band-edge
-  // row (neighbour row in another CTA, the other in this one); 2 other
-  // segments touching a band-edge row (spanning two rows, or a one-row band);
-  // 1 bulk with the periodic wrap; 0 interior bulk
+  // first pair of segment sg: the first row's, the last row's, those between
+  auto seg_start = [&](int sg) {
+    return sg < spr ? 32 * sg : (sg < 2 * spr ? (b.rows - 1) * b.Wh + 32 * (sg - spr) : b.Wh + 32 * (sg - 2 * spr));
+  };
   for (int sg = warp; sg < nseg; sg += NW) {
-    const int i = sg * 32 + lane;
-    const int ly = (int)__umulhi((unsigned)i, R.div_w), x = i - ly * b.W, y = b.row0 + ly;
-    const bool pad = i >= b.nb;
-    const bool box = !pad && x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
-    const bool wall = !pad && (y == 0 || y == b.H - 1);
-    const bool edge = !pad && b.cs > 1 && (ly == 0 || ly == b.rows - 1);
-    // (every lane takes part in the shuffle: it is not under the && below)
-    const int ly0 = __shfl_sync(0xffffffffu, ly, 0);
-    const bool one_row = __all_sync(0xffffffffu, !pad && ly == ly0) && b.rows > 1;
-    const bool inner = __all_sync(0xffffffffu, !pad && x > 0 && x < b.W - 1);
+    const int i = seg_start(sg) + lane;
+    const int lim = sg < spr ? b.Wh : (sg < 2 * spr ? b.np : b.np - b.Wh);
+    const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = pair_of(b, i - ly * b.Wh), y = b.row0 + ly;
+    const bool in = i < lim;
+    const bool any_box = __any_sync(0xffffffffu, in && (in_box(R, xh, y) || in_box(R, xh + b.Wh, y)));
+    const bool full = __all_sync(0xffffffffu, in && !on_seam(b, xh));
     int c;
-    if (__any_sync(0xffffffffu, box || pad))
-      c = 5;
-    else if (__any_sync(0xffffffffu, wall))
-      c = one_row ? 4 : 5;
-    else if (__any_sync(0xffffffffu, edge))
-      c = one_row ? 3 : 2;
-    else
-      c = inner ? 0 : 1;
+    if (sg < 2 * spr) {
+      const bool wall = sg < spr ? b.row0 == 0 : b.row0 + b.rows == b.H;
+      c = b.rows == 1 || any_box ? SEG_GENERAL : (wall ? SEG_WALL : SEG_EDGE);
+    } else {
+      c = any_box ? SEG_BOX : (full ? SEG_INNER : SEG_PART);
+    }
     if (lane == 0) cls[sg] = (unsigned char)c;
   }
   __syncthreads();
-  if (warp == 0) {  // the list, class 5 first; range ends after classes 5, 4, 3, 2, 1
+  if (warp == 0) {  // the list and its ranges' ends
     const unsigned lower = (1u << lane) - 1u;
     int n = 0;
-    for (int pass = 5; pass >= 0; pass--) {
+    for (int pass = 0; pass < SEG_CLASSES; pass++) {
       for (int c = 0; c < nseg; c += 32) {
         const bool take = c + lane < nseg && cls[c + lane] == pass;
         const unsigned m = __ballot_sync(0xffffffffu, take);
-        if (take) list[n + __popc(m & lower)] = (unsigned short)(c + lane);
+        if (take) list[n + __popc(m & lower)] = (unsigned short)seg_start(c + lane);
         n += __popc(m);
       }
-      if (lane == 0 && pass >= 1) count_s[5 - pass] = n;
+      if (lane == 0) range[pass] = n;
     }
   }
   __syncthreads();
-  const int *range = count_s;  // read at each loop start: five registers fewer held across the steps
-  const float *map = FIELD ? a.maps + R.map_base + (long long)b.clone * R.nodes + (long long)b.row0 * b.W : nullptr;
+  const float *map = FIELD ? a.maps + R.map_base + (long long)b.clone * R.nodes : nullptr;
+  const WarpPlan plan = warp_plan<NW>(R, b, range, warp);
   bool bad = false;
   cluster.sync();
+  if (b.cs > 1) cluster_arrive(true);  // the first step's wait
   // every step but the last
   // (steps past the field's run through the uniform-force path: with eps = 0
   // the field path computes the same beta and constants bit for bit)
+#pragma unroll 1
   for (int t = 0; t + 1 < a.steps; t++) {
     const bool field = FIELD && t + 1 < R.field_steps;
     if ((t & 1) == 0) {
       if (field)
-        band_step<NW, true, FIELD, !FIELD>(a, b, A, list, nseg, range, warp, lane, t, map, bad);
+        band_step<NW, true, FIELD>(a, b, plan, A, list, range, warp, lane, t, map, bad);
       else
-        band_step<NW, true, false, !FIELD>(a, b, A, list, nseg, range, warp, lane, t, map, bad);
+        band_step<NW, true, false>(a, b, plan, A, list, range, warp, lane, t, map, bad);
     } else {
       if (field)
-        band_step<NW, false, FIELD, !FIELD>(a, b, A, list, nseg, range, warp, lane, t, map, bad);
+        band_step<NW, false, FIELD>(a, b, plan, A, list, range, warp, lane, t, map, bad);
       else
-        band_step<NW, false, false, !FIELD>(a, b, A, list, nseg, range, warp, lane, t, map, bad);
+        band_step<NW, false, false>(a, b, plan, A, list, range, warp, lane, t, map, bad);
     }
-    cluster.sync();
   }
-  // the last step stores S_T (one step in T: every node through update_general)
+  // the last step stores S_T
+  if (b.cs > 1) cluster_wait();
   {
     const int t = a.steps - 1;
     float *terms = a.terms + (long long)t * a.term_slab + R.term_base;
-    for (int i = threadIdx.x; i < b.nb; i += THREADS) update_general(a, b, A, i, t, (t & 1) == 0, true, terms);
+#pragma unroll 1
+    for (int j = threadIdx.x; j < 2 * b.np; j += THREADS) {
+      const int h = j >= b.np, i = h ? j - b.np : j;
+      const int ly = (int)__umulhi((unsigned)i, b.div_wh), x = i - ly * b.Wh + h * b.Wh;
+      if (x < b.W) store_last(a, b, A, x, ly, (t & 1) == 0, terms);
+    }
   }
   if (bad) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
   cluster.sync();  // no CTA leaves while a neighbour may still read its shared memory
@@ -610,13 +844,15 @@ int temporal_rows_limit(int W) {
   return r;
 }
 
+bool temporal_resident(int W, int rows) { return pair_smem(rows, W) <= kSmemLimit; }
+
 struct TemporalVariant {
   int threads;
   TemporalFn fn[2];  // [field]
 };
 
 #define GENERIC(T, M) {k_temporal_f32<T, M, false>, k_temporal_f32<T, M, true>}
-static const TemporalVariant kTemporal[] = {{1024, GENERIC(1024, 1)}, {512, GENERIC(512, 2)}, {256, GENERIC(256, 4)}};
+static const TemporalVariant kTemporal[] = {{1024, GENERIC(1024, 1)}, {512, GENERIC(512, 1)}, {256, GENERIC(256, 2)}};
 #undef GENERIC
 
 int temporal_variant_count() { return (int)(sizeof(kTemporal) / sizeof(kTemporal[0])); }
@@ -665,20 +901,23 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
     rows_max = std::max(rows_max, rows);
   }
   TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field);
-  if (!fn || a.steps < 1) return cudaErrorInvalidConfiguration;
-  const size_t smem = temporal_smem(rows_max * W);
+  if (!fn || !temporal_resident(W, rows_max) || a.steps < 1) return cudaErrorInvalidConfiguration;
+  const size_t smem = pair_smem(rows_max, W);
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
+  TemporalArgs args = a;
+  const unsigned long long wh = (W + 1) / 2;
+  args.div_wh = (unsigned)(((1ULL << 32) + wh - 1) / wh);
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = temporal_config(cs, variant, nclones, smem, s, attr);
-  return cudaLaunchKernelEx(&cfg, fn, a);
+  return cudaLaunchKernelEx(&cfg, fn, args);
 }
 
 // Whether the cluster shape can be resident at all (occupancy query, no launch).
 int temporal_max_clusters(int cs, int variant, int W, int rows_max, bool field) {
   TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field);
   if (!fn) return 0;
-  const size_t smem = temporal_smem(rows_max * W);
+  const size_t smem = std::min(pair_smem(rows_max, W), kSmemLimit);
   if (prepare(fn, cs, smem) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = temporal_config(cs, variant, 64, smem, nullptr, attr);
