@@ -630,6 +630,9 @@ struct LbPlan {
   int nstream = 0, tiles[3] = {0, 0, 0}, variant = 0;
 };
 
+// the FP64 kernels' grid: 64-node tiles of every clone's padded planes
+static int tiles64(const clbm_ctx *c) { return (int)(c->pop_elems / 576); }
+
 static bool plan_active(const LbPlan &p, int r) { return p.active.empty() || p.active[r]; }
 
 // largest band of run r's split at its cluster size
@@ -738,8 +741,8 @@ static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int
     int cur = src;
     for (int t = 0; t < steps; t++) {
       StepArgs a{p.table, p.nstream, t, c->pop[cur], c->pop[1 - cur], c->d.terms, c->d.term_slab,
-                 c->d.err, c->total_clones, c->max_nodes, {p.tiles[0], p.tiles[1], p.tiles[2]}, c->d_maps};
-      if ((e = launch_step(f64, !timing && t == steps - 1, a, c->total_blocks, s, p.variant)) != cudaSuccess)
+                 c->d.err, c->total_clones, c->max_nodes, {p.tiles[0], p.tiles[1], p.tiles[2]}, c->d_maps, tiles64(c)};
+      if ((e = launch_step(f64, !timing && t == steps - 1, a, s, p.variant)) != cudaSuccess)
         return e;
       if (!timing) cur = 1 - cur;
     }
@@ -817,7 +820,7 @@ static cudaError_t enqueue_interval(clbm_ctx *c, int steps, int sbuf, bool prof 
   // clusters still copy parents.)
   bool fuse = !f64 && !c->any_field && steps % 2 == 0;
   for (int r = 0; r < c->nruns; r++) fuse = fuse && plan.cs[r] > 0;
-  if (!fuse && (e = launch_reseed(f64, ra, c->total_blocks, s)) != cudaSuccess) return e;
+  if (!fuse && (e = launch_reseed(f64, ra, c->total_blocks, tiles64(c), s)) != cudaSuccess) return e;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (prof) {
     if ((size_t)c->ev_used + 2 > c->ev.size()) {
@@ -1644,13 +1647,13 @@ extern "C" int clbm_drag_fwd(clbm_ctx *c, int steps, int every, double *J) {
   // interval (the ones clbm_get_field_map returns)
   ReseedArgs ra{c->d.runs, c->nruns, c->adj.s0, loc(0), c->d_identity, c->d_zeros, c->d.pert,
                 c->d.prefactors, c->d.snaps, c->d.state, c->d.err, c->d_maps};
-  CK(launch_reseed(f64, ra, c->total_blocks, s));
+  CK(launch_reseed(f64, ra, c->total_blocks, tiles64(c), s));
   for (int t = 0; t < steps; t++) {
     char *dst = (t + 1 < steps) ? loc(t + 1) : c->adj.sig[(t + 1) % 2];
     StepArgs a{c->d.runs, c->nruns, t, loc(t), dst, c->d.terms, c->d.term_slab, c->d.err,
                c->total_clones, c->max_nodes, {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]},
-               c->d_maps};
-    CK(launch_step(f64, false, a, c->total_blocks, s, c->step_variant));
+               c->d_maps, tiles64(c)};
+    CK(launch_step(f64, false, a, s, c->step_variant));
   }
   CK(launch_drag_reduce(f64, c->d, c->nruns, c->total_clones, steps, c->any_stress, c->any_momentum, s));
   if (J) CK(cudaMemcpyAsync(J, c->d.sacc, sizeof(double) * c->total_clones, cudaMemcpyDeviceToHost, s));
@@ -1679,8 +1682,8 @@ extern "C" int clbm_drag_bwd(clbm_ctx *c) {
     for (int p = lo; p < hi; p++) {  // recompute P_lo .. P_hi from the checkpoint (step p of the forward)
       StepArgs a{c->d.runs, c->nruns, p, segP(lo, p), segP(lo, p + 1), c->d.terms, c->d.term_slab,
                  c->d.err, c->total_clones, c->max_nodes,
-                 {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]}, c->d_maps};
-      CK(launch_step(f64, false, a, c->total_blocks, s, c->step_variant));
+                 {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]}, c->d_maps, tiles64(c)};
+      CK(launch_step(f64, false, a, s, c->step_variant));
     }
     for (int p = hi; p >= lo; p--) {
       if (p == T - 1) {

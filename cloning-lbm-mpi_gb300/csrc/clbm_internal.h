@@ -78,6 +78,7 @@ struct StepArgs {
   int max_nodes;
   int total_tiles[3]; // FP32 step grid for tiles of 128 / 256 / 512 nodes
   const float *maps;  // random body-force fields (nullable)
+  int tiles64;        // FP64 step grid: 64-node tiles of every clone (pop elements / 576)
 };
 
 struct ReseedArgs {
@@ -121,11 +122,10 @@ struct TemporalArgs {
 
 
 // kernel launchers (clbm_step.cu, clbm_cloning.cu)
-cudaError_t launch_step(bool f64, bool last, const StepArgs &a, int blocks, cudaStream_t s,
-                        int variant);
+cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, int variant);
 int step_variant_count();
 int step_variant_block(int variant);
-cudaError_t launch_reseed(bool f64, const ReseedArgs &a, int blocks, cudaStream_t s);
+cudaError_t launch_reseed(bool f64, const ReseedArgs &a, int blocks, int tiles64, cudaStream_t s);
 cudaError_t launch_perturb_norms(bool f64, const RunDev *runs, int nruns, const void *src,
                                  const int *labels, const int *mark, const double *prefactors,
                                  const double *snaps, double *partials, double *pert,

@@ -40,52 +40,111 @@ __device__ __forceinline__ Moments64 moments_ref64(const double f[9]) {
   return m;
 }
 
-// c_k . u for the nine directions, as the reference evaluates cx*ux + cy*uy
-__device__ __forceinline__ double eu_ref64(int k, double ux, double uy) {
-  switch (k) {
-    case 0: return 0.0;
-    case 1: return ux;
-    case 2: return uy;
-    case 3: return -ux;
-    case 4: return -uy;
-    case 5: return DADD(ux, uy);
-    case 6: return DADD(-ux, uy);
-    case 7: return DADD(-ux, -uy);
-    default: return DADD(ux, -uy);
+// Quotients by one divisor, each the correctly rounded a / b.  The FP64 pipe
+// (about two operations per clock and SM) bounds every FP64 kernel, and three
+// divisions by the same density are a sixth of a collision.  Markstein's
+// method (IBM J. Res. Dev. 34, 1990): with y the correctly rounded 1/b and q
+// next to a / b, r = a - b q is exact and q + r y rounds to a / b.  Here y
+// comes from the hardware approximation by a cubic step (3 operations, within
+// a unit) and a correcting step (2), yl = (1 - b y) y is what it still lacks
+// (2), and a quotient costs 4: q = a y + a yl is within half a unit (1 + 2^-50)
+// of Q = a / b.  The rounded value then differs from Q by at most
+// |Q - q| |b y - 1|, 2^-54 b units for 0.5 <= b < 1 and 2^-55 b for 1 <= b < 2,
+// while no midpoint of two doubles lies within 2^-54 / b (2^-53 / b) of a
+// quotient: it rounds as Q does.  A significand of b that is all ones (where
+// the correcting step may fail), a density outside [0.5, 2) or numerators at
+// the ends of the exponent range take the division.
+struct Divisor64 {
+  double b, y, yl;
+  bool ok;
+};
+__device__ __forceinline__ Divisor64 divisor64(double b) {
+  Divisor64 d;
+  d.b = b;
+  const int hi = __double2hiint(b);
+  d.ok = (unsigned)(hi - 0x3fe00000) < 0x00200000u && !((hi & 0xfffff) == 0xfffff && __double2loint(b) == -1);
+  double y0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+  const double e = __fma_rn(-b, y0, 1.0);
+  const double y1 = __fma_rn(__fma_rn(e, e, e), y0, y0);
+  d.y = __fma_rn(__fma_rn(-b, y1, 1.0), y1, y1);
+  d.yl = DMUL(__fma_rn(-b, d.y, 1.0), d.y);
+  return d;
+}
+// whether a is far from the ends of the exponent range (or zero)
+__device__ __forceinline__ bool mid_range64(double a) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  return h - 0x10000000u < 0x60000000u || (h | (unsigned)__double2loint(a)) == 0u;
+}
+__device__ __forceinline__ double div64(double a, const Divisor64 &d) {
+  const double q = __fma_rn(a, d.y, DMUL(a, d.yl));
+  const double v = __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+  // a zero keeps its sign
+  return __hiloint2double(__double2hiint(v) | (__double2hiint(a) & 0x80000000), __double2loint(v));
+}
+
+// The velocity of the collision, shifted by the force (streamCollCompute.cpp:28-29)
+__device__ __forceinline__ void velocity_ref64(const Moments64 &m, double half_beta, double &ux, double &uy) {
+  const Divisor64 d = divisor64(m.rho);
+  if (d.ok && mid_range64(m.jx) && mid_range64(m.jy) && mid_range64(half_beta)) {
+    ux = DADD(div64(m.jx, d), div64(half_beta, d));
+    uy = div64(m.jy, d);
+  } else {
+    ux = DADD(DDIV(m.jx, m.rho), DDIV(half_beta, m.rho));
+    uy = DDIV(m.jy, m.rho);
   }
 }
 
-// w[k]*rho*(1 + 3 eu + 4.5 eu^2 + u2), u2 = -1.5 |u|^2 (streamCollCompute.cpp:32-34)
-__device__ __forceinline__ double feq_ref64(int k, double rho, double eu, double u2) {
-  const double eueu = DMUL(DMUL(4.5, eu), eu);
-  return DMUL(DMUL(w_of(k), rho), DADD(DADD(DADD(1.0, DMUL(3.0, eu)), eueu), u2));
+// 1 + 3 eu + 4.5 eu^2 + u2 for eu = e and eu = -e, u2 = -1.5 |u|^2
+// (streamCollCompute.cpp:32-34): the products of -e are those of e with the
+// sign changed, exactly, so an opposite pair of directions shares them.  t3 = 3 e.
+__device__ __forceinline__ void feq_pair_ref64(double e, double t3, double u2, double &plus, double &minus) {
+  const double ee = DMUL(DMUL(4.5, e), e);
+  plus = DADD(DADD(DADD(1.0, t3), ee), u2);
+  minus = DADD(DADD(DSUB(1.0, t3), ee), u2);
 }
 
 // BGK collision with the Guo forcing term, velocity shifted by beta/(2 rho)
-// (streamCollCompute.cpp:28-37).  wcb[k] = (w[k]*(1 - omega/2))*beta.
+// (streamCollCompute.cpp:28-37), every value the reference's, bit for bit.
+// wcb[k] = (w[k]*(1 - omega/2))*beta.  The reference evaluates c_k.u, the
+// equilibrium and the drive 3 (cx - ux) + 9 cx eu direction by direction;
+// here what differs between directions in sign only is formed once: c_k.u of
+// opposite directions, 3 ux (the drive's of cx = 0), 3 (1 + ux) (minus the
+// drive's of cx = -1), 9 eu, the products w rho.  150 FP64 operations a node
+// (about 205 direction by direction, with three divisions): 2.72 -> 3.32 G
+// updates per second on 256 clones of 256x64.
 __device__ __forceinline__ void collide_ref64(const double f[9], double out[9], double beta,
                                               const double wcb[9], double omega,
                                               double om1, double *rho_o = nullptr,
                                               double *ux_o = nullptr, double *uy_o = nullptr) {
   const Moments64 m = moments_ref64(f);
-  const double ux = DADD(DDIV(m.jx, m.rho), DDIV(DMUL(0.5, beta), m.rho));
-  const double uy = DDIV(m.jy, m.rho);
+  double ux, uy;
+  velocity_ref64(m, DMUL(0.5, beta), ux, uy);
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
+  const double es = DADD(ux, uy), ed = DSUB(ux, uy);  // c_5.u = -c_7.u, c_8.u = -c_6.u
+  const double t3x = DMUL(3.0, ux);
+  double q[9];
+  q[0] = DADD(1.0, u2);
+  feq_pair_ref64(ux, t3x, u2, q[1], q[3]);
+  feq_pair_ref64(uy, DMUL(3.0, uy), u2, q[2], q[4]);
+  feq_pair_ref64(es, DMUL(3.0, es), u2, q[5], q[7]);
+  feq_pair_ref64(ed, DMUL(3.0, ed), u2, q[8], q[6]);
+  const double right = DMUL(3.0, DSUB(1.0, ux)), left = DMUL(3.0, DADD(1.0, ux));
+  const double nx = DMUL(9.0, ux), ns = DMUL(9.0, es), nd = DMUL(9.0, ed);
+  double drive[9];
+  drive[0] = DMUL(wcb[0], -t3x);
+  drive[2] = drive[4] = DMUL(wcb[1], -t3x);
+  drive[1] = DMUL(wcb[1], DADD(right, nx));
+  drive[5] = DMUL(wcb[5], DADD(right, ns));
+  drive[8] = DMUL(wcb[5], DADD(right, nd));
+  drive[3] = DMUL(wcb[1], DSUB(nx, left));
+  drive[7] = DMUL(wcb[5], DSUB(ns, left));
+  drive[6] = DMUL(wcb[5], DSUB(nd, left));
+  const double r0 = DMUL(w_of(0), m.rho), r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const double eu = eu_ref64(k, ux, uy);
-    const double feq = feq_ref64(k, m.rho, eu, u2);
-    const int c = cx_of(k);
-    // 3*(cx - ux) + 9*cx*eu
-    double drive;
-    if (c == 0)
-      drive = DMUL(3.0, -ux);
-    else if (c == 1)
-      drive = DADD(DMUL(3.0, DSUB(1.0, ux)), DMUL(9.0, eu));
-    else
-      drive = DADD(DMUL(3.0, DSUB(-1.0, ux)), DMUL(-9.0, eu));
-    drive = DMUL(wcb[k], drive);
-    out[k] = DADD(DADD(DMUL(f[k], om1), DMUL(feq, omega)), drive);
+    const double feq = DMUL(k == 0 ? r0 : (k <= 4 ? r1 : r5), q[k]);
+    out[k] = DADD(DADD(DMUL(f[k], om1), DMUL(feq, omega)), drive[k]);
   }
   if (rho_o) {
     *rho_o = m.rho;
@@ -99,12 +158,21 @@ __device__ __forceinline__ void collide_ref64(const double f[9], double out[9], 
 __device__ __forceinline__ void pi_ref64(const double f[9], double &rho, double &pxx,
                                          double &pxy) {
   const Moments64 m = moments_ref64(f);
-  const double uy = DDIV(m.jy, m.rho);
-  const double ux = DDIV(m.jx, m.rho);
+  const Divisor64 d = divisor64(m.rho);
+  const bool fast = d.ok && mid_range64(m.jx) && mid_range64(m.jy);
+  const double uy = fast ? div64(m.jy, d) : DDIV(m.jy, m.rho);
+  const double ux = fast ? div64(m.jx, d) : DDIV(m.jx, m.rho);
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
+  const double es = DADD(ux, uy), ed = DSUB(ux, uy);
+  double q[9];
+  feq_pair_ref64(ux, DMUL(3.0, ux), u2, q[1], q[3]);
+  feq_pair_ref64(es, DMUL(3.0, es), u2, q[5], q[7]);
+  feq_pair_ref64(ed, DMUL(3.0, ed), u2, q[8], q[6]);
+  const double r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
   double fneq[9];
 #pragma unroll
-  for (int k = 1; k < 9; k++) fneq[k] = DSUB(f[k], feq_ref64(k, m.rho, eu_ref64(k, ux, uy), u2));
+  for (int k = 1; k < 9; k++)
+    if (cx_of(k) != 0) fneq[k] = DSUB(f[k], DMUL(k <= 4 ? r1 : r5, q[k]));
   rho = m.rho;
   pxx = DADD(DADD(DADD(DADD(DADD(fneq[1], fneq[3]), fneq[5]), fneq[6]), fneq[7]), fneq[8]);
   pxy = DSUB(DADD(DSUB(fneq[5], fneq[6]), fneq[7]), fneq[8]);

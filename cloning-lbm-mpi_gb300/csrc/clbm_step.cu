@@ -47,25 +47,35 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
   return L;
 }
 
-template <bool F64>
-__device__ __forceinline__ bool density_ok(const pop_t<F64> S[9]) {
-  if constexpr (F64) {
-    double r = S[0];
-#pragma unroll
-    for (int k = 1; k < 9; k++) r += S[k];
-    return r > 0.0;
-  } else {
-    float d = 0.f;
-#pragma unroll
-    for (int k = 0; k < 9; k++) d += S[k];
-    return d > -1.0f;
-  }
+// The FP64 step and reseed take tiles of 64 nodes: the planes are multiples of
+// 64 elements, so a run's tiles start at pop_base / 576 and a clone has
+// plane / 64 of them.  The FP64 pipe bounds these kernels, and the SM with the
+// most nodes sets the time: tiles of 256 gave 16 clones of 200x50 4.1 of them
+// per SM (5 on some), and one state of 129x129 only 65 busy SMs.
+constexpr int TILE64 = 64;
+__device__ __forceinline__ NodeLoc locate64(const RunDev *runs, int nruns) {
+  NodeLoc L;
+  const long long first = 9LL * TILE64 * blockIdx.x;  // pop_base the tile would have
+  int r = 0;
+  while (r + 1 < nruns && first >= runs[r + 1].pop_base) r++;
+  const RunDev &R = runs[r];
+  const unsigned per = (unsigned)(R.plane / TILE64);
+  const unsigned local = blockIdx.x - (unsigned)(R.pop_base / (9 * TILE64));
+  L.run = r;
+  L.clone = (int)(local / per);
+  L.n = (int)(local - (unsigned)L.clone * per) * TILE64 + threadIdx.x;
+  L.valid = L.n < R.nodes;
+  L.y = (int)__umulhi((unsigned)L.n, R.div_w);
+  L.x = L.n - L.y * R.W;
+  return L;
 }
 
-template <bool F64, bool LAST>
-__global__ void __launch_bounds__(STEP_BLOCK) k_step(StepArgs a) {
-  using T = pop_t<F64>;
-  const NodeLoc L = locate(a.runs, a.nruns);
+// FP64 step, the reference's arithmetic.
+template <bool LAST>
+__global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
+  using T = double;
+  constexpr bool F64 = true;
+  const NodeLoc L = locate64(a.runs, a.nruns);
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const long long plane = R.plane;
@@ -101,7 +111,8 @@ __global__ void __launch_bounds__(STEP_BLOCK) k_step(StepArgs a) {
     T *terms = (T *)a.terms + (long long)a.step * a.term_slab + R.term_base;
     store_drag_terms<F64>(R, S, x, y, L.clone, terms);
   }
-  if (!density_ok<F64>(S)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
+  // (the density as moments_ref64 sums it: one sum for both uses)
+  if (!(moments_ref64(S).rho > 0.0)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
   if (LAST) {
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = S[k];
@@ -220,13 +231,12 @@ int step_variant_count() { return (int)(sizeof(kF32Variants) / sizeof(kF32Varian
 
 int step_variant_block(int v) { return kF32Variants[v].block; }
 
-cudaError_t launch_step(bool f64, bool last, const StepArgs &a, int blocks, cudaStream_t s,
-                        int variant) {
+cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, int variant) {
   if (f64) {
     if (last)
-      k_step<true, true><<<blocks, STEP_BLOCK, 0, s>>>(a);
+      k_step<true><<<a.tiles64, TILE64, 0, s>>>(a);
     else
-      k_step<true, false><<<blocks, STEP_BLOCK, 0, s>>>(a);
+      k_step<false><<<a.tiles64, TILE64, 0, s>>>(a);
   } else {
     if (variant < 0 || variant >= step_variant_count()) variant = 0;
     const F32Variant &v = kF32Variants[variant];
@@ -246,9 +256,9 @@ cudaError_t launch_step(bool f64, bool last, const StepArgs &a, int blocks, cuda
 // perturbed (:412-416: snapshot mix, generatePerturbedState.cpp:4-38, or the
 // counter-based uniform noise), and the result is collided into P.
 template <bool F64>
-__global__ void __launch_bounds__(STEP_BLOCK) k_reseed(ReseedArgs a) {
+__global__ void __launch_bounds__(F64 ? TILE64 : STEP_BLOCK) k_reseed(ReseedArgs a) {
   using T = pop_t<F64>;
-  const NodeLoc L = locate(a.runs, a.nruns);
+  const NodeLoc L = F64 ? locate64(a.runs, a.nruns) : locate(a.runs, a.nruns);
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const int x = L.x, y = L.y, n = L.n;
@@ -261,9 +271,9 @@ __global__ void __launch_bounds__(STEP_BLOCK) k_reseed(ReseedArgs a) {
   for (int k = 0; k < 9; k++) dst[k * R.plane + n] = P[k];
 }
 
-cudaError_t launch_reseed(bool f64, const ReseedArgs &a, int blocks, cudaStream_t s) {
+cudaError_t launch_reseed(bool f64, const ReseedArgs &a, int blocks, int tiles64, cudaStream_t s) {
   if (f64)
-    k_reseed<true><<<blocks, STEP_BLOCK, 0, s>>>(a);
+    k_reseed<true><<<tiles64, TILE64, 0, s>>>(a);
   else
     k_reseed<false><<<blocks, STEP_BLOCK, 0, s>>>(a);
   return cudaGetLastError();
