@@ -70,12 +70,22 @@ __device__ __forceinline__ NodeLoc locate64(const RunDev *runs, int nruns) {
   return L;
 }
 
+// Consecutive steps are launched with programmatic stream serialisation: a
+// step's blocks may take their places while the previous step drains, find
+// their nodes, and wait here until it has completed and its writes are
+// visible.  (step_begin is the first thing that touches the populations.)
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // FP64 step, the reference's arithmetic.
 template <bool LAST>
 __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
   using T = double;
   constexpr bool F64 = true;
   const NodeLoc L = locate64(a.runs, a.nruns);
+  step_begin();
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const long long plane = R.plane;
@@ -153,6 +163,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_f32(StepArgs a) {
   const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
   const bool near = valid && (in_box || y == 0 || y == H - 1);
   const bool warp_near = __any_sync(0xffffffffu, near);
+  step_begin();
   if (!valid) return;
   const int plane = (int)R.plane;
   const long long cb = R.pop_base + (long long)clone * 9 * R.plane;
@@ -232,22 +243,20 @@ int step_variant_count() { return (int)(sizeof(kF32Variants) / sizeof(kF32Varian
 int step_variant_block(int v) { return kF32Variants[v].block; }
 
 cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, int variant) {
-  if (f64) {
-    if (last)
-      k_step<true><<<a.tiles64, TILE64, 0, s>>>(a);
-    else
-      k_step<false><<<a.tiles64, TILE64, 0, s>>>(a);
-  } else {
-    if (variant < 0 || variant >= step_variant_count()) variant = 0;
-    const F32Variant &v = kF32Variants[variant];
-    const int ts = v.block == 128 ? 0 : (v.block == 256 ? 1 : 2);
-    const int grid = a.total_tiles[ts];
-    if (last)
-      v.last<<<grid, v.block, 0, s>>>(a);
-    else
-      v.body<<<grid, v.block, 0, s>>>(a);
-  }
-  return cudaGetLastError();
+  if (variant < 0 || variant >= step_variant_count()) variant = 0;
+  const F32Variant &v = kF32Variants[variant];
+  const int ts = v.block == 128 ? 0 : (v.block == 256 ? 1 : 2);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(f64 ? a.tiles64 : a.total_tiles[ts]);
+  cfg.blockDim = dim3(f64 ? TILE64 : v.block);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void (*fn)(StepArgs) = f64 ? (last ? k_step<true> : k_step<false>) : (last ? v.last : v.body);
+  return cudaLaunchKernelEx(&cfg, fn, a);
 }
 
 // ---------------------------------------------------------------------------
