@@ -12,7 +12,12 @@
 #include <cstring>
 #include <string>
 #include <algorithm>
+#include <atomic>
+#include <map>
+#include <mutex>
 #include <vector>
+
+#include <cuda.h>
 
 #include "../../include/clbm.h"
 #include "clbm_internal.h"
@@ -40,12 +45,73 @@ static int fail(int status, const char *msg) {
   return status;
 }
 
+// The pool of call_alloc.  The device's default pool gives its memory back to
+// the system at every synchronisation, which made each small temporary cost
+// about 200 us of mapping; this one keeps up to 64 MB (a dump's or a snapshot's
+// stage) and gives it back with the last context.  Stream-ordered, so any
+// stream and thread may use it.  One per CUDA context, told apart by the
+// context's id: a pool does not outlive a cudaDeviceReset.
+namespace {
+constexpr unsigned long long kPoolKeep = 64ull << 20;
+std::mutex g_pool_mutex;
+std::map<unsigned long long, cudaMemPool_t> g_pools;
+std::atomic<int> g_contexts{0};
+
+// the current context's pool, or nullptr (create: make it if there is none)
+cudaMemPool_t current_pool(bool create) {
+  typedef CUresult (*GetId)(CUcontext, unsigned long long *);
+  static const GetId get_id = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return (GetId)fn;
+  }();
+  int dev = 0;
+  unsigned long long id = 0;
+  // (no context yet, a first call: the default pool)
+  if (!get_id || cudaGetDevice(&dev) != cudaSuccess || get_id(nullptr, &id) != CUDA_SUCCESS) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  auto it = g_pools.find(id);
+  if (it != g_pools.end() || !create) return it != g_pools.end() ? it->second : nullptr;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  unsigned long long keep = kPoolKeep;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    pool = nullptr;  // (kept: this context goes on with the default pool)
+  }
+  g_pools[id] = pool;
+  return pool;
+}
+}  // namespace
+
+cudaError_t clbm::call_alloc(void **p, size_t bytes, cudaStream_t s) {
+  cudaMemPool_t pool = current_pool(true);
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+
 struct GraphEntry {
   cudaGraphExec_t exec = nullptr;
   int sbuf = -1, steps = -1;
 };
 
 struct clbm_ctx {
+  clbm_ctx() { g_contexts++; }
+  ~clbm_ctx() {
+    if (--g_contexts == 0)
+      if (cudaMemPool_t pool = current_pool(false)) cudaMemPoolTrimTo(pool, 0);
+  }
   int nruns = 0, precision = 0, max_steps = 0, flags = 0;
   std::vector<clbm_run_desc> desc;
   std::vector<RunDev> runs_h;
@@ -517,7 +583,7 @@ extern "C" int clbm_load_run_aos_f64(clbm_ctx *c, int run, const double *aos) {
   const int chunk = (int)std::min<size_t>(R.nclones, half / clone_bytes);
   if (chunk < 1) {  // one clone larger than half the buffer: a temporary stage
     double *stage = nullptr;
-    CK(cudaMallocAsync((void **)&stage, clone_bytes, c->stream));
+    CK(call_alloc((void **)&stage, clone_bytes, c->stream));
     cudaError_t e = cudaSuccess;
     for (int j = 0; j < R.nclones && e == cudaSuccess; j++) {
       e = cudaMemcpyAsync(stage, aos + (size_t)j * n, clone_bytes, cudaMemcpyHostToDevice, c->stream);
@@ -566,7 +632,7 @@ extern "C" int clbm_load_pops_aos_f64(clbm_ctx *c, int run, int clone, const dou
   if (clone < 0 || clone >= R.nclones || !aos) return fail(CLBM_ERR_INVALID, "bad clone or NULL array");
   const size_t n = 9 * (size_t)R.nodes;
   double *stage = nullptr;
-  CK(cudaMallocAsync((void **)&stage, n * 8, c->stream));
+  CK(call_alloc((void **)&stage, n * 8, c->stream));
   cudaError_t e = cudaMemcpyAsync(stage, aos, n * 8, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess)
     e = launch_aos_to_soa(c->precision == CLBM_FP64, c->d.runs, run, R.nodes, clone, 1, stage, c->pop[c->s_buf], c->stream);
@@ -579,17 +645,20 @@ extern "C" int clbm_dump_pops_aos_f64(clbm_ctx *c, int run, int clone, double *a
   if (int s = check_run(c, run)) return s;
   const RunDev &R = c->runs_h[run];
   if (clone < 0 || clone >= R.nclones || !aos) return fail(CLBM_ERR_INVALID, "bad clone or NULL array");
-  int parent = clone;
-  CK(cudaMemcpyAsync(&parent, c->d.labels + R.clone_base + clone, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  if (parent < 0 || parent >= R.nclones) return fail(CLBM_ERR_DEVICE, "corrupt pending label");
   const size_t n = 9 * (size_t)R.nodes;
+  const int *labels = c->d.labels + R.clone_base;
   double *stage = nullptr;
-  CK(cudaMallocAsync((void **)&stage, n * 8, c->stream));
-  cudaError_t e = launch_soa_to_aos(c->precision == CLBM_FP64, c->d.runs, run, R.nodes, parent, c->pop[c->s_buf], stage, c->stream);
+  CK(call_alloc((void **)&stage, n * 8, c->stream));
+  cudaError_t e = launch_soa_to_aos(c->precision == CLBM_FP64, c->d.runs, run, R.nodes, clone, labels, true,
+                                    c->pop[c->s_buf], stage, c->stream);
+  // (no clone step pending: every slot is its own parent)
+  int parent = clone;
+  if (e == cudaSuccess && c->pending)
+    e = cudaMemcpyAsync(&parent, labels + clone, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(aos, stage, n * 8, cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(stage, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess && (parent < 0 || parent >= R.nclones)) return fail(CLBM_ERR_DEVICE, "corrupt pending label");
   return clbm_status_from_cuda(e);
 }
 
@@ -600,7 +669,7 @@ extern "C" int clbm_set_snapshots_aos_f64(clbm_ctx *c, int run, int nsnap, const
   if (nsnap != R.nsnap || !aos) return fail(CLBM_ERR_INVALID, "nsnap differs from the run descriptor");
   const size_t n = 9 * (size_t)R.nodes * nsnap;
   double *stage = nullptr;
-  CK(cudaMallocAsync((void **)&stage, n * 8, c->stream));
+  CK(call_alloc((void **)&stage, n * 8, c->stream));
   cudaError_t e = cudaMemcpyAsync(stage, aos, n * 8, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = launch_snaps_to_soa(c->d.runs, run, R.nodes, nsnap, stage, c->d.snaps, c->stream);
   cudaFreeAsync(stage, c->stream);
@@ -1266,8 +1335,6 @@ static cudaError_t full_plan(clbm_ctx *c, const std::vector<int> &cs, const std:
 // streaming ones -- is timed as a whole and kept if it beats the uniform
 // winner.  Results are cached per (lattice sizes, clone counts) for the
 // process.
-#include <map>
-#include <mutex>
 struct TuneResult {
   int best;
   std::vector<int> cs, tv;
@@ -1585,7 +1652,7 @@ extern "C" int clbm_scgf(clbm_ctx *c, int run, int first, int count, double dT, 
   if (first < 0 || first + count > done || first + count > c->d.max_intervals)
     return fail(CLBM_ERR_INVALID, "requested intervals outside the recorded history");
   double *d_out = nullptr;
-  CK(cudaMallocAsync((void **)&d_out, sizeof(double), c->stream));
+  CK(call_alloc((void **)&d_out, sizeof(double), c->stream));
   cudaError_t e = launch_scgf(c->d.logr + (size_t)run * c->d.max_intervals, first, count, dT, d_out, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(psi, d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(d_out, c->stream);
@@ -1709,16 +1776,13 @@ extern "C" int clbm_get_drag_grad_aos_f64(clbm_ctx *c, int run, int clone, doubl
   if (c->adj.result < 0) return fail(CLBM_ERR_INVALID, "no gradient: call clbm_drag_bwd first");
   const size_t n = 9 * (size_t)R.nodes;
   double *stage = nullptr;
-  CK(cudaMallocAsync((void **)&stage, n * 8, c->stream));
-  cudaError_t e = launch_soa_to_aos(c->precision == CLBM_FP64, c->d.runs, run, R.nodes, clone,
-                                    c->adj.sig[c->adj.result], stage, c->stream);
+  CK(call_alloc((void **)&stage, n * 8, c->stream));
+  cudaError_t e = launch_soa_to_aos(c->precision == CLBM_FP64, c->d.runs, run, R.nodes, clone, nullptr,
+                                    false, c->adj.sig[c->adj.result], stage, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(aos, stage, n * 8, cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(stage, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return clbm_status_from_cuda(e);
-  if (c->precision != CLBM_FP64)  // soa_to_aos adds back w[k] for states; a gradient has no shift
-    for (size_t i = 0; i < n; i++) aos[i] -= w_of((int)(i % 9));
-  return CLBM_OK;
+  return clbm_status_from_cuda(e);
 }
 
 // ---------------------------------------------------------------------------
@@ -1761,8 +1825,8 @@ extern "C" int clbm_reconstruct_lineages(clbm_ctx *c, int run, int *nintervals, 
   const int steps = c->hist_steps;
   int *d_anc = nullptr;
   double *d_out = nullptr;
-  CK(cudaMallocAsync((void **)&d_anc, sizeof(int) * (size_t)R.nclones * n, c->stream));
-  cudaError_t e = cudaMallocAsync((void **)&d_out, sizeof(double) * (size_t)R.nclones * n * steps, c->stream);
+  CK(call_alloc((void **)&d_anc, sizeof(int) * (size_t)R.nclones * n, c->stream));
+  cudaError_t e = call_alloc((void **)&d_out, sizeof(double) * (size_t)R.nclones * n * steps, c->stream);
   if (e == cudaSuccess)
     e = launch_reconstruct(c->hist_drag, c->hist_labels, c->total_clones, R.clone_base, R.nclones, n, steps,
                            c->max_steps, d_anc, d_out, c->stream);
@@ -1783,7 +1847,7 @@ extern "C" int clbm_macro_fields(clbm_ctx *c, int run, int clone, double *rho, d
   if (c->pending) return fail(CLBM_ERR_INVALID, "a clone step is pending; run an interval first");
   const size_t n = R.nodes;
   double *d = nullptr;
-  CK(cudaMallocAsync((void **)&d, 3 * n * sizeof(double), c->stream));
+  CK(call_alloc((void **)&d, 3 * n * sizeof(double), c->stream));
   cudaError_t e = launch_macro(c->precision == CLBM_FP64, c->d.runs, run, clone, R.nodes, c->pop[c->s_buf], d,
                                d + n, d + 2 * n, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(rho, d, n * 8, cudaMemcpyDeviceToHost, c->stream);

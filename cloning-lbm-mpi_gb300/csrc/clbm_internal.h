@@ -121,6 +121,10 @@ struct TemporalArgs {
 };
 
 
+// Device memory for the length of one call (freed with cudaFreeAsync), from
+// the library's own pool: clbm_api.cu.
+cudaError_t call_alloc(void **p, size_t bytes, cudaStream_t s);
+
 // kernel launchers (clbm_step.cu, clbm_cloning.cu)
 cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, int variant);
 int step_variant_count();
@@ -182,8 +186,10 @@ cudaError_t launch_init_equilibrium(bool f64, const RunDev *runs, int nruns, int
                                     cudaStream_t s);
 cudaError_t launch_aos_to_soa(bool f64, const RunDev *runs, int run, int nodes, int clone0, int nclone,
                               const double *aos, void *pop, cudaStream_t s);
-cudaError_t launch_soa_to_aos(bool f64, const RunDev *runs, int run, int nodes, int clone, const void *pop,
-                              double *aos, cudaStream_t s);
+// labels (nullable): the run's pending labels, slot `clone` then gives its
+// parent's state.  shift: FP32 values are f - w[k] (a state; not a gradient)
+cudaError_t launch_soa_to_aos(bool f64, const RunDev *runs, int run, int nodes, int clone, const int *labels,
+                              bool shift, const void *pop, double *aos, cudaStream_t s);
 cudaError_t launch_macro(bool f64, const RunDev *runs, int run, int clone, int nodes, const void *pop,
                          double *rho, double *ux, double *uy, cudaStream_t s);
 cudaError_t launch_snaps_to_soa(const RunDev *runs, int run, int nodes, int nsnap, const double *aos,

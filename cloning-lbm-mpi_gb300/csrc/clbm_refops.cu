@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "../../include/clbm.h"
+#include "clbm_internal.h"
 #include "clbm_physics.cuh"
 
 namespace clbm {
@@ -101,8 +102,8 @@ __global__ void k_ref_interior(GeomDev g, double *fout) {
   for (int k = 0; k < 9; k++) fout[aos(g, x, y, k)] = w_of(k);
 }
 
-// force.cpp:8-144: per-node terms in parallel, then the four sides summed in
-// node order by one thread.
+// force.cpp:8-144: per-node terms in parallel, then each side summed in node
+// order by a thread of its own.
 __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *out) {
   extern __shared__ double terms[];
   const int sx = g.xmax - g.xmin + 1, sy = g.ymax - g.ymin + 1;
@@ -128,30 +129,28 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
     terms[i] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double side[4];
-    const int len[4] = {sy, sy, sx, sx};
-    int i = 0;
-    for (int s = 0; s < 4; s++) {
-      double v = terms[i];
-      for (int q = 1; q < len[s]; q++) v = DADD(v, terms[i + q]);
-      side[s] = v;
-      i += len[s];
-    }
-    *out = DADD(DADD(DADD(side[0], side[1]), side[2]), side[3]);
+  if (threadIdx.x < 4) {
+    const int s = threadIdx.x, len = s < 2 ? sy : sx, i = s < 2 ? s * sy : 2 * sy + (s - 2) * sx;
+    double v = terms[i];
+    for (int q = 1; q < len; q++) v = DADD(v, terms[i + q]);
+    const double a = __shfl_sync(0xfu, v, 1), b = __shfl_sync(0xfu, v, 2), c4 = __shfl_sync(0xfu, v, 3);
+    if (s == 0) *out = DADD(DADD(DADD(v, a), b), c4);
   }
 }
 
 // generatePerturbedState.cpp:4-38 in two passes: fixed-order norm reduction,
 // then the element-wise update.
+struct Prefactors {
+  double v[64];
+};
 __global__ void k_ref_perturb_norms(const double *fin, const double *snaps, int nsnap, int n,
-                                    const double *pref, double *partials) {
+                                    const Prefactors pref, double *partials) {
   __shared__ double red[2][256 / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double n0 = 0.0, n1 = 0.0;
   if (i < n) {
-    double mix = DMUL(pref[0], snaps[i]);
-    for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref[q], snaps[(long long)q * n + i]));
+    double mix = DMUL(pref.v[0], snaps[i]);
+    for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
     n0 = DMUL(fin[i], fin[i]);
     n1 = DMUL(mix, mix);
   }
@@ -175,32 +174,48 @@ __global__ void k_ref_perturb_norms(const double *fin, const double *snaps, int 
   }
 }
 
-// The two norms summed over the blocks' partials in block order, once:
-// out[0] = |f| / |mix| (the mix weight), out[1] = 1 / (1 + eps * sum(pref) * weight)
+// The two norms summed over the blocks' partials, once, by one block in a fixed
+// order (thread t the partials t, t + 256, ..., then a tree; a single thread
+// spent 100 us on the 2323 pairs of a 257x257 state): out[0] = |f| / |mix| (the
+// mix weight), out[1] = 1 / (1 + eps * sum(pref) * weight)
 // (generatePerturbedState.cpp:22-36).
-__global__ void k_ref_perturb_finalize(const double *pref, int nsnap, const double *partials,
-                                       int nblocks, double eps, double *out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double a0 = partials[0], a1 = partials[1];
-  for (int b = 1; b < nblocks; b++) {
+__global__ void __launch_bounds__(256) k_ref_perturb_finalize(const Prefactors pref, int nsnap, const double *partials,
+                                                              int nblocks, double eps, double *out) {
+  __shared__ double red[2][256 / 32];
+  double a0 = 0.0, a1 = 0.0;
+  for (int b = threadIdx.x; b < nblocks; b += 256) {
     a0 = DADD(a0, partials[2 * b]);
     a1 = DADD(a1, partials[2 * b + 1]);
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    a0 = DADD(a0, __shfl_down_sync(0xffffffffu, a0, o));
+    a1 = DADD(a1, __shfl_down_sync(0xffffffffu, a1, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = a0;
+    red[1][threadIdx.x >> 5] = a1;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 256 / 32; w++) {
+    a0 = DADD(a0, red[0][w]);
+    a1 = DADD(a1, red[1][w]);
+  }
   const double weight = DDIV(__dsqrt_rn(a0), __dsqrt_rn(a1));
-  double sum = pref[0];
-  for (int q = 1; q < nsnap; q++) sum = DADD(sum, pref[q]);
+  double sum = pref.v[0];
+  for (int q = 1; q < nsnap; q++) sum = DADD(sum, pref.v[q]);
   out[0] = weight;
   out[1] = DDIV(1., DADD(1.0, DMUL(DMUL(sum, eps), weight)));
 }
 
 // f <- (f + eps * mix * weight) / a with (weight, 1/a) from k_ref_perturb_finalize
 __global__ void k_ref_perturb_apply(double *fin, const double *snaps, int nsnap, int n,
-                                    const double *pref, const double *wa, double eps) {
+                                    const Prefactors pref, const double *wa, double eps) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double w = wa[0], inv = wa[1];
-  double mix = DMUL(pref[0], snaps[i]);
-  for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref[q], snaps[(long long)q * n + i]));
+  double mix = DMUL(pref.v[0], snaps[i]);
+  for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
   fin[i] = DMUL(DADD(fin[i], DMUL(DMUL(eps, mix), w)), inv);
 }
 
@@ -218,6 +233,19 @@ static int check_geom(const clbm_geom *g) {
     return CLBM_ERR_INVALID;
   }
   return CLBM_OK;
+}
+
+// The three passes of a perturbation; wa: the weight pair, part: two norm
+// partials per 256 values (device).
+static cudaError_t run_perturb(double *fin, const double *snaps, double eps, int nsnap, int n, const double *prefactors,
+                               double *wa, double *part, cudaStream_t st) {
+  Prefactors pref = {};
+  for (int q = 0; q < nsnap; q++) pref.v[q] = prefactors[q];
+  const int nb = (n + 255) / 256;
+  k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, part);
+  k_ref_perturb_finalize<<<1, 256, 0, st>>>(pref, nsnap, part, nb, eps, wa);
+  k_ref_perturb_apply<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, wa, eps);
+  return cudaGetLastError();
 }
 
 static GeomDev to_dev(const clbm_geom *g) {
@@ -276,7 +304,7 @@ extern "C" int clbm_ref_force_on_square(const clbm_geom *g, const double *f, dou
   if (!f || !result) return CLBM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
   double *d_out = nullptr;
-  cudaError_t e = cudaMallocAsync(&d_out, sizeof(double), st);
+  cudaError_t e = call_alloc((void **)&d_out, sizeof(double), st);
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
   const int nterm = 2 * (g->xmax - g->xmin + 1) + 2 * (g->ymax - g->ymin + 1);
   k_ref_force<<<1, 256, nterm * sizeof(double), st>>>(to_dev(g), f, omega, d_out);
@@ -293,16 +321,9 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
   cudaStream_t st = (cudaStream_t)stream;
   const int nb = (n + 255) / 256;
   double *d_buf = nullptr;
-  cudaError_t e = cudaMallocAsync(&d_buf, sizeof(double) * (nsnap + 2 + 2 * (size_t)nb), st);
+  cudaError_t e = call_alloc((void **)&d_buf, sizeof(double) * (2 + 2 * (size_t)nb), st);
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
-  double *d_pref = d_buf, *d_wa = d_buf + nsnap, *d_part = d_buf + nsnap + 2;
-  e = cudaMemcpyAsync(d_pref, prefactors, sizeof(double) * nsnap, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) {
-    k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, d_pref, d_part);
-    k_ref_perturb_finalize<<<1, 32, 0, st>>>(d_pref, nsnap, d_part, nb, eps, d_wa);
-    k_ref_perturb_apply<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, d_pref, d_wa, eps);
-    e = cudaGetLastError();
-  }
+  e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, d_buf, d_buf + 2, st);
   cudaFreeAsync(d_buf, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return clbm_status_from_cuda(e);
@@ -310,21 +331,21 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
 
 // ---------------------------------------------------------------------------
 // clbm_ref_perturbed_state_noalloc: the same kernels as
-// clbm_ref_perturbed_state, with their scratch (the snapshot prefactors and
-// two norm partial sums per 256 values, the mix weight) in a fixed device
-// array instead of a per-call allocation.  It serves callers that must not allocate device
-// memory at all: code running under an allocator that already owns the whole
-// device, or inside a time-critical loop where an allocation's implicit
-// synchronisation is not acceptable.
+// clbm_ref_perturbed_state, with their scratch (two norm partial sums per 256
+// values, the mix weight) in a fixed device array instead of a per-call
+// allocation.  It serves callers that must not allocate device memory at all:
+// code running under an allocator that already owns the whole device, or
+// inside a time-critical loop where an allocation's implicit synchronisation
+// is not acceptable.
 namespace {
 constexpr int NOALLOC_MAX_N = 1 << 20;                     // values per state, 9*Dx*Dy
 constexpr int NOALLOC_MAX_BLOCKS = NOALLOC_MAX_N / 256;    // norm partials (pairs)
-constexpr int NOALLOC_PREF = 64;                           // prefactor slots (nsnap <= 64)
+constexpr int NOALLOC_PREF = 64;                           // prefactors (nsnap <= 64)
 // Shared by every call on a device and kept until the process exits
-// (66 KB per device that loads the library): the prefactors, the mix weight
-// and 1/a, then the norm partials.  Nothing in it has to start at zero: each
-// call overwrites the prefactors, the weight pair and every partial it reads.
-static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_PREF + 2 + 2 * NOALLOC_MAX_BLOCKS];
+// (64 KB per device that loads the library): the mix weight and 1/a, then the
+// norm partials.  Nothing in it has to start at zero: each call overwrites the
+// weight pair and every partial it reads.
+static __device__ __align__(256) double g_noalloc_scratch[2 + 2 * NOALLOC_MAX_BLOCKS];
 
 constexpr int NOALLOC_MAX_DEVICES = 64;
 std::mutex g_noalloc_mutex;
@@ -367,16 +388,7 @@ extern "C" int clbm_ref_perturbed_state_noalloc(double *fin, const double *snaps
   double *scratch = nullptr;
   if (int s = noalloc_scratch(&scratch)) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  const int nb = (n + 255) / 256;
-  double *d_pref = scratch, *d_wa = scratch + NOALLOC_PREF, *d_part = scratch + NOALLOC_PREF + 2;
-  cudaError_t e = cudaMemcpyAsync(d_pref, prefactors, sizeof(double) * nsnap,
-                                  cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) {
-    k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, d_pref, d_part);
-    k_ref_perturb_finalize<<<1, 32, 0, st>>>(d_pref, nsnap, d_part, nb, eps, d_wa);
-    k_ref_perturb_apply<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, d_pref, d_wa, eps);
-    e = cudaGetLastError();
-  }
+  cudaError_t e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, scratch, scratch + 2, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return clbm_status_from_cuda(e);
 }

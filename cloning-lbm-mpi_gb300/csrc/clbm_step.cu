@@ -456,17 +456,21 @@ __global__ void k_aos_to_soa(const RunDev *runs, int run, int clone0, const doub
   for (int k = 0; k < 9; k++) dst[k * R.plane] = F64 ? (T)src[k] : (T)(src[k] - w_of(k));
 }
 
+// (a parent out of range writes nothing; the host checks the label it reads)
 template <bool F64>
-__global__ void k_soa_to_aos(const RunDev *runs, int run, int clone, const void *popv,
-                             double *aos) {
+__global__ void k_soa_to_aos(const RunDev *runs, int run, int clone, const int *labels, bool shift,
+                             const void *popv, double *aos) {
   using T = pop_t<F64>;
   const RunDev &R = runs[run];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= R.nodes) return;
+  if (labels) clone = labels[clone];
+  if (clone < 0 || clone >= R.nclones) return;
   const int x = t / R.H, y = t - x * R.H;
   const T *src = (const T *)popv + R.pop_base + (long long)clone * 9 * R.plane + (long long)y * R.W + x;
 #pragma unroll
-  for (int k = 0; k < 9; k++) aos[9LL * t + k] = F64 ? (double)src[k * R.plane] : w_of(k) + (double)src[k * R.plane];
+  for (int k = 0; k < 9; k++)
+    aos[9LL * t + k] = F64 || !shift ? (double)src[k * R.plane] : w_of(k) + (double)src[k * R.plane];
 }
 
 __global__ void k_snaps_to_soa(const RunDev *runs, int run, const double *aos, double *snaps) {
@@ -523,12 +527,12 @@ cudaError_t launch_aos_to_soa(bool f64, const RunDev *runs, int run, int nodes, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_soa_to_aos(bool f64, const RunDev *runs, int run, int nodes, int clone, const void *pop,
-                              double *aos, cudaStream_t s) {
+cudaError_t launch_soa_to_aos(bool f64, const RunDev *runs, int run, int nodes, int clone, const int *labels,
+                              bool shift, const void *pop, double *aos, cudaStream_t s) {
   if (f64)
-    k_soa_to_aos<true><<<(nodes + 255) / 256, 256, 0, s>>>(runs, run, clone, pop, aos);
+    k_soa_to_aos<true><<<(nodes + 255) / 256, 256, 0, s>>>(runs, run, clone, labels, shift, pop, aos);
   else
-    k_soa_to_aos<false><<<(nodes + 255) / 256, 256, 0, s>>>(runs, run, clone, pop, aos);
+    k_soa_to_aos<false><<<(nodes + 255) / 256, 256, 0, s>>>(runs, run, clone, labels, shift, pop, aos);
   return cudaGetLastError();
 }
 
