@@ -371,6 +371,7 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
     R.f_force = f32_force(R.f_beta, R.f_cforce);
     R.f_pairs = f32_pairs(R.f_omega, R.f_om1, R.f_c13, R.f_c2, R.f_force);
     R.f_force2 = f32_force2(R.f_force, R.f_force);
+    R.f_field_ops = f32_field_ops(R.f_beta, (float)d.field_eps, R.f_cforce);
     R.perturb_mode = d.perturb_mode;
     R.resample_mode = d.resample_mode;
     R.drag_mode = d.drag_mode;
@@ -882,12 +883,12 @@ static cudaError_t enqueue_interval(clbm_ctx *c, int steps, int sbuf, bool prof 
   ReseedArgs ra{c->d.runs, c->nruns, S, c->pop[1 - sbuf], c->d.labels, c->d.mark, c->d.pert,
                 c->d.prefactors, c->d.snaps, c->d.state, c->d.err, c->d_maps};
   const LbPlan plan = current_plan(c, f64);
-  // Every run cluster-resident under the uniform body force and an even step
-  // count (S_T then goes to the other buffer than S): the interval kernels do
-  // the reseed while loading their clones, which saves writing P_0 and
-  // reading it back.  (With an odd count S_T would overwrite S while other
-  // clusters still copy parents.)
-  bool fuse = !f64 && !c->any_field && steps % 2 == 0;
+  // Every run cluster-resident and an even step count (S_T then goes to the
+  // other buffer than S): the interval kernels do the reseed while loading
+  // their clones, which saves writing P_0 and reading it back (with the random
+  // field 1.1 ms of 4096 clones of 256x64).  (With an odd count S_T would
+  // overwrite S while other clusters still copy parents.)
+  bool fuse = !f64 && steps % 2 == 0;
   for (int r = 0; r < c->nruns; r++) fuse = fuse && plan.cs[r] > 0;
   if (!fuse && (e = launch_reseed(f64, ra, c->total_blocks, tiles64(c), s)) != cudaSuccess) return e;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -119,6 +119,26 @@ __host__ __device__ inline F32Force2 f32_force2(const F32Force &a, const F32Forc
   return f;
 }
 
+// Constants (v, v) of a node pair's force under a random field
+// (pair_force): beta, eps of the field, cforce, and f32_force's factors.
+struct F32FieldOps {
+  f2_t beta, eps, cforce, half, three, nine, mnine, mthird, twelfth, mtwelfth;
+};
+__host__ __device__ inline F32FieldOps f32_field_ops(float beta, float eps, float cforce) {
+  F32FieldOps o;
+  o.beta = f2_bits(beta, beta);
+  o.eps = f2_bits(eps, eps);
+  o.cforce = f2_bits(cforce, cforce);
+  o.half = f2_bits(0.5f, 0.5f);
+  o.three = f2_bits(3.0f, 3.0f);
+  o.nine = f2_bits(9.0f, 9.0f);
+  o.mnine = f2_bits(-9.0f, -9.0f);
+  o.mthird = f2_bits(-(1.0f / 3.0f), -(1.0f / 3.0f));
+  o.twelfth = f2_bits(1.0f / 12.0f, 1.0f / 12.0f);
+  o.mtwelfth = f2_bits(-(1.0f / 12.0f), -(1.0f / 12.0f));
+  return o;
+}
+
 // One independent run (lattice, square, physics, clone block) of a batch.
 struct RunDev {
   int W, H;                    // Dx, Dy
@@ -151,6 +171,7 @@ struct RunDev {
   F32Force f_force;
   F32Pairs f_pairs;            // the same constants packed for the f32x2 collision
   F32Force2 f_force2;          // f_force in both lanes, for the two-node collision
+  F32FieldOps f_field_ops;     // the same under a random field, per pair
   int perturb_mode, resample_mode, ranks, nsnap;
   unsigned long long seed;
   unsigned run_id;

@@ -31,15 +31,19 @@
 // What bounds it: per 32 pairs 77 packed operations, 2 cycles each on the
 // FMA pipe of a scheduler (154), and 36 cycles of the SM's shared memory for
 // four schedulers' 18 accesses each (144).  On the 256x64 channel (bands
-// 23/18/23, 512 threads) a segment takes 215 (local step) to 270 cycles; 4096
-// clones run at 0.306 ms per step, where one node per thread with the four
-// direction pairs packed took 0.367; 1024 clones of 400x100 (9 bands) at 0.221
-// against 0.353.  What made the difference besides the packing (ms per step of
-// the 256x64 case): each warp's share of the deal kept in registers instead of
-// worked out in every step (0.344 -> 0.317), one population's row planes
-// instead of node records, so that what crosses a band edge goes as whole
-// sectors (0.317 -> 0.306; 400x100: 0.265 -> 0.225), and the split cluster
-// barrier with the edge rows first (400x100: 0.33 -> 0.28).
+// 23/18/23, 512 threads) a segment takes about 210 (local step) to 260 cycles;
+// 4096 clones run at 0.297 ms per step, where one node per thread with the
+// four direction pairs packed took 0.367; 1024 clones of 400x100 (9 bands) at
+// 0.204 against 0.353.  What made the difference besides the packing (ms per
+// step of the 256x64 case): each warp's share of the deal kept in registers
+// instead of worked out in every step (0.344 -> 0.317), whole planes per
+// population instead of node records, so that what crosses a band edge goes as
+// whole sectors (0.317 -> 0.306; 400x100: 0.265 -> 0.225), planes a constant
+// distance apart, so that a pair's slots are constant offsets (0.306 -> 0.297),
+// and the split cluster barrier with the edge rows first (400x100: 0.33 ->
+// 0.28).  Random-field steps read two values per pair from L2: loaded one
+// segment ahead, 0.343 -> 0.329 ms per step over an interval with 20 of 100
+// such steps.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -77,11 +81,14 @@ __device__ __forceinline__ void st_cluster2(unsigned a, f2_t v) {
   asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
 
-// Geometry of one CTA's band.
-struct Band {
+// Geometry of one CTA's band.  NP: the pairs a plane of A has room for, a
+// constant, so that the nine slots of a pair lie at constant offsets.
+template <int NP>
+struct BandT {
+  static constexpr int ps = 2 * NP;  // floats per plane
   int cs, rank, clone, W, H, rows, row0;
   int Wh, np;      // pairs per row, pairs of the band
-  int ps, rowf;    // floats per plane of a row (2 Wh), per row (9 planes)
+  int rowf;        // floats per row of a plane (2 Wh)
   unsigned div_wh; // ceil(2^32 / Wh)
   int rows_prev;   // rows of the previous band (its last row lies above this band's row 0)
   float *prev, *next;
@@ -93,6 +100,7 @@ struct Band {
 
 // Float offset, within a row of A, of column x's population 0 (population k
 // at + k ps): pair x or x - Wh, its lane 0 or 1.
+template <class Band>
 __device__ __forceinline__ int col_off(const Band &b, int x) { return x < b.Wh ? 2 * x : 2 * (x - b.Wh) + 1; }
 
 // A row of A: in this CTA, or anywhere in the cluster.
@@ -122,6 +130,7 @@ __device__ __forceinline__ Cols cols_inner(int xh) {
 // any pair: the periodic wrap, and with an odd width lane 1 of the last pair,
 // which holds no node: it gets itself for both neighbours (a column of its
 // own, periodic over one node, that no node ever reads)
+template <class Band>
 __device__ __forceinline__ Cols cols_any(const Band &b, int xh) {
   const int x1 = xh + b.Wh;
   Cols c;
@@ -137,26 +146,51 @@ __device__ __forceinline__ Cols cols_any(const Band &b, int xh) {
 // at a constant offset -- the first and the last, and with an odd width the
 // one before the last (its lane 1 is the last node).  seam_count pairs per
 // row; the j-th of them.
+template <class Band>
 __device__ __forceinline__ bool on_seam(const Band &b, int xh) {
   return xh == 0 || xh >= b.Wh - 1 - (b.W & 1);
 }
+template <class Band>
 __device__ __forceinline__ int seam_count(const Band &b) { return (b.W & 1) && b.Wh > 2 ? 3 : 2; }
+template <class Band>
 __device__ __forceinline__ int seam_pair(const Band &b, int j) { return j == 0 ? 0 : b.Wh - j; }
 
 // Index p within a row as the segments take its pairs: the pair Wh - 1 first,
 // then 0, 1, ..., so that the seam at the two ends falls into one segment.
+template <class Band>
 __device__ __forceinline__ int pair_of(const Band &b, int p) { return p == 0 ? b.Wh - 1 : p - 1; }
 
-// The two nodes' force: the run's, or under a random field from its values at
-// the nodes (where lane 1 holds no node, lane 0's).
-template <bool FIELD>
-__device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, const float *map, int y, int xh,
-                                                float feps) {
-  if (!FIELD) return R.f_force2;
+// The random field's values at a pair's nodes (where lane 1 holds no node,
+// lane 0's).
+template <class Band>
+__device__ __forceinline__ f2_t pair_map(const Band &b, const float *map, int y, int xh) {
   const float *m = map + (long long)y * b.W + xh;
-  const float m0 = m[0], m1 = xh + b.Wh < b.W ? m[b.Wh] : m0;
-  return f32_force2(f32_force(field_beta_f32(R.f_beta, feps, m0), R.f_cforce),
-                    f32_force(field_beta_f32(R.f_beta, feps, m1), R.f_cforce));
+  return f2_bits(m[0], m[xh + b.Wh < b.W ? b.Wh : 0]);
+}
+
+// The two nodes' force: the run's, or under a random field (while its steps
+// last) from its values m at the nodes -- field_beta_f32 and f32_force of both
+// nodes in packed arithmetic.
+template <bool FIELD>
+__device__ __forceinline__ F32Force2 pair_force(const RunDev &R, f2_t m) {
+  if (!FIELD) return R.f_force2;
+  namespace X = f32x2op;
+  const F32FieldOps &o = R.f_field_ops;
+  const f2_t beta = X::mul(o.beta, X::fma(o.eps, m, R.f_pairs.one));
+  const f2_t fb = X::mul(o.cforce, beta);
+  F32Force2 f;
+  f.hb = X::mul(o.half, beta);
+  f.nfbm3 = X::mul(o.three, fb);
+  f.fb9 = X::mul(o.nine, fb);
+  f.nfb9 = X::mul(o.mnine, fb);
+  f.f2 = X::mul(o.twelfth, fb);
+  f.nf2 = X::mul(o.mtwelfth, fb);
+  f.nf13 = X::mul(o.mthird, fb);
+  return f;
+}
+template <bool FIELD, class Band>
+__device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, const float *map, int y, int xh) {
+  return pair_force<FIELD>(R, FIELD ? pair_map(b, map, y, xh) : 0ull);
 }
 
 // One pair of nodes in a gather step.  C, U, D: the pair's row and the rows
@@ -166,8 +200,8 @@ __device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, 
 // wall, slots 4, 7, 8 (the row beyond the wall is not touched); 3 = by the
 // thread's wb / wt.  UNI: both lanes' neighbour columns lie in one pair, every
 // slot pair is one 64-bit access.  PRED: lane h is written only if !skip_h.
-template <bool FIELD, bool UNI, int WALL, bool PRED, class RC, class RU, class RD>
-__device__ __forceinline__ void gather_pair(const RunDev &R, int ps, const RC C, const RU U, const RD D, const Cols &c,
+template <int ps, bool UNI, int WALL, bool PRED, class RC, class RU, class RD>
+__device__ __forceinline__ void gather_pair(const RunDev &R, const RC C, const RU U, const RD D, const Cols &c,
                                             const F32Force2 &f, bool &bad, bool skip0 = false, bool skip1 = false,
                                             bool wb = false, bool wt = false) {
   auto ld = [](const auto &row, int a, int b2, int q) {
@@ -245,8 +279,8 @@ __device__ __forceinline__ void gather_pair(const RunDev &R, int ps, const RC C,
 }
 
 // One pair of nodes in a local step: S(n,k) = A[n][k], P(n,k) -> A[n][opp k].
-template <bool PRED>
-__device__ __forceinline__ void local_pair(const RunDev &R, int ps, float *o, const F32Force2 &f, bool &bad,
+template <int ps, bool PRED>
+__device__ __forceinline__ void local_pair(const RunDev &R, float *o, const F32Force2 &f, bool &bad,
                                            bool skip0 = false, bool skip1 = false) {
   f2_t S[9], P[9];
 #pragma unroll
@@ -295,7 +329,7 @@ __device__ __forceinline__ void perimeter_node(const RunDev &R, int ylo, int yhi
 // dropped); with the square at a band edge the rows may lie in adjacent bands
 // (shared::cluster addresses), else the three are in this CTA (plain indexing, which the compiler
 // schedules freely).
-template <bool GATHER>
+template <bool GATHER, class Band>
 __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Band &b, int x, int y, bool edge,
                                                  const float *map, float feps, bool &bad, float *terms, float *A) {
   const RunDev &R = a.rd;
@@ -349,6 +383,7 @@ __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Ba
 }
 
 // One node of the last step: S_T (and its drag terms), any position.
+template <class Band>
 __device__ __forceinline__ void store_last(const TemporalArgs &a, const Band &b, const float *A, int x, int ly,
                                            bool gather, float *terms) {
   const RunDev &R = a.rd;
@@ -382,6 +417,7 @@ __device__ __forceinline__ void store_last(const TemporalArgs &a, const Band &b,
   if (!(d > -1.0f)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
 }
 
+template <class Band>
 __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::cluster_group &cluster) {
   Band b;
   b.cs = (int)cluster.num_blocks();
@@ -395,8 +431,7 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
   b.rows = a.band_row0[b.rank + 1] - b.row0;
   b.rows_prev = b.rank > 0 ? b.row0 - a.band_row0[b.rank - 1] : b.rows;
   b.np = b.rows * b.Wh;
-  b.ps = 2 * b.Wh;
-  b.rowf = 9 * b.ps;
+  b.rowf = 2 * b.Wh;
   b.prev = b.rank > 0 ? cluster.map_shared_rank(A, b.rank - 1) : A;
   b.next = b.rank + 1 < b.cs ? cluster.map_shared_rank(A, b.rank + 1) : A;
   const unsigned a_cta = (unsigned)__cvta_generic_to_shared(A);
@@ -408,7 +443,7 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
   b.src = a.src + cb;
   b.dst = a.dst + cb;
   // opaque: held in registers, not worked out again from the lattice width
-  asm volatile("" : "+r"(b.ps), "+r"(b.rowf), "+r"(b.Wh), "+r"(b.div_wh), "+r"(b.np));
+  asm volatile("" : "+r"(b.rowf), "+r"(b.Wh), "+r"(b.div_wh), "+r"(b.np));
   return b;
 }
 
@@ -417,7 +452,7 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
 // the same per-node function as the reseed kernel, so bit-identical).
 // Square-interior nodes and the empty lane of an odd width's last pair get
 // zeros (the fluid at rest).
-template <int THREADS, bool FUSED>
+template <int THREADS, bool FUSED, class Band>
 __device__ __forceinline__ void load_band(const TemporalArgs &a, const Band &b, float *A) {
   const RunDev &R = a.rd;
 #pragma unroll 1
@@ -445,24 +480,25 @@ __device__ __forceinline__ float field_eps(const TemporalArgs &a, int t) {
   return t + 1 < a.rd.field_steps ? a.rd.f_field_eps : 0.0f;
 }
 
-// Shared memory of one CTA: the band's populations, then the segment list,
-// one class byte per segment and the ends of the list's ranges.  temporal_smem
-// (a function of the nodes alone) is what a shape is accepted by; pair_smem
-// what a band takes: the same populations for an even width, one node more per
-// row for an odd one.
+// Shared memory of one CTA: the nine planes, then the segment list, one class
+// byte per segment and the ends of the list's ranges.  temporal_smem (a
+// function of the nodes alone) is what a shape is accepted by; a plane of
+// kPairs takes the largest band of an even width that it accepts (3219
+// pairs), one of kPairsHalf lets two CTAs share an SM.
 __host__ __device__ inline size_t temporal_smem(int nb) {
   const int nseg = (nb + 31) / 32;
   return sizeof(float) * 9 * (size_t)nb + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
 }
+constexpr int kPairs = 3220, kPairsHalf = 1600;
 // segments of 32 pairs: the first and the last row by themselves, then the
 // rows between them
 __host__ __device__ inline int segment_count(int rows, int Wh) {
   const int spr = (Wh + 31) / 32;
   return rows == 1 ? spr : 2 * spr + ((rows - 2) * Wh + 31) / 32;
 }
-__host__ __device__ inline size_t pair_smem(int rows, int W) {
-  const int Wh = (W + 1) / 2, nseg = segment_count(rows, Wh);
-  return 8 * 9 * (size_t)rows * Wh + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
+__host__ __device__ inline size_t pair_smem(int planes_np, int rows, int W) {
+  const int nseg = segment_count(rows, (W + 1) / 2);
+  return 8 * 9 * (size_t)planes_np + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
 }
 
 // Segment classes, in the order of the list.
@@ -530,6 +566,7 @@ struct Head {
   int eouter, einner, eper;      // their entries, the perimeter's
   int ylo, yhi, nper;
   bool box_edge;
+  template <class Band>
   __device__ __forceinline__ Head(const RunDev &R, const Band &b, bool gather) {
     ns = seam_count(b);
     nouter = gather ? ns * min(b.rows, 2) : 0;
@@ -546,7 +583,7 @@ struct Head {
 };
 
 // The warp's plan, from the class ends of the list.
-template <int NW>
+template <int NW, class Band>
 __device__ __forceinline__ WarpPlan warp_plan(const RunDev &R, const Band &b, const int *range, int warp) {
   WarpPlan p;
   p.nbox = range[SEG_BOX];
@@ -573,13 +610,14 @@ __device__ __forceinline__ WarpPlan warp_plan(const RunDev &R, const Band &b, co
   return p;
 }
 
-template <int NW, bool GATHER, bool FIELD>
+template <int NW, bool GATHER, bool FIELD, class Band>
 __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, const WarpPlan &w, float *A,
                                           const unsigned short *list, const int *range, int warp, int lane, int t,
                                           const float *map, bool &bad) {
   const RunDev &R = a.rd;
   const float feps = FIELD ? field_eps(a, t) : 0.0f;
-  const int ps = b.ps, rf = b.rowf;
+  constexpr int ps = Band::ps;
+  const int rf = b.rowf;
   // the pair of segment position i: its row and column, inactive past `lim`
 #define CLBM_PAIR(lim)                                                                         \
   const int i = list[k] + lane;                                                                \
@@ -591,13 +629,13 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
     const bool wb = y == 0, wt = y == b.H - 1;
     const RowC U{wb ? C.a : (ly == 0 ? b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf) : C.a - 4u * (unsigned)rf)};
     const RowC D{wt ? C.a : (ly == b.rows - 1 ? b.next_c : C.a + 4u * (unsigned)rf)};
-    gather_pair<FIELD, false, 3, true>(R, ps, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh, feps), bad,
+    gather_pair<ps, false, 3, true>(R, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh), bad,
                                        in_box(R, xh, y), in_box(R, xh + b.Wh, y), wb, wt);
   };
   auto local = [&](int ly, int xh, auto pred) {
     const int y = b.row0 + ly;
     constexpr bool P = decltype(pred)::value;
-    local_pair<P>(R, ps, A + ly * rf + 2 * xh, pair_force<FIELD>(R, b, map, y, xh, feps), bad, P && in_box(R, xh, y),
+    local_pair<ps, P>(R, A + ly * rf + 2 * xh, pair_force<FIELD>(R, b, map, y, xh), bad, P && in_box(R, xh, y),
                   P && in_box(R, xh + b.Wh, y));
   };
   const bool lead = w.flags & (PLAN_HEAD << GATHER);
@@ -629,12 +667,12 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
         if (on_seam(b, xh)) continue;
         float *C = A + ly * rf;
-        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh, feps);
+        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh);
         if (ly == 0)  // warp-uniform
-          gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowC{b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf)},
+          gather_pair<ps, true, 0, false>(R, RowL{C}, RowC{b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf)},
                                              RowL{C + rf}, cols_inner(xh), f, bad);
         else
-          gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowC{b.next_c}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowC{b.next_c}, cols_inner(xh), f, bad);
       }
     } else {
 #pragma unroll 1
@@ -677,8 +715,8 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         if (j >= ninner) continue;
         const int r = ns == 2 ? j >> 1 : j / 3, ly = r + 1, xh = seam_pair(b, j - ns * r), y = b.row0 + ly;
         float *C = A + ly * rf;
-        gather_pair<FIELD, false, 0, true>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_any(b, xh),
-                                           pair_force<FIELD>(R, b, map, y, xh, feps), bad, in_box(R, xh, y),
+        gather_pair<ps, false, 0, true>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_any(b, xh),
+                                           pair_force<FIELD>(R, b, map, y, xh), bad, in_box(R, xh, y),
                                            in_box(R, xh + b.Wh, y));
       }
 #pragma unroll 1
@@ -686,19 +724,19 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         CLBM_PAIR(list[k] < b.Wh ? b.Wh : b.np);
         if (on_seam(b, xh)) continue;
         float *C = A + ly * rf;
-        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh, feps);
+        const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh);
         if (y == 0)  // warp-uniform
-          gather_pair<FIELD, true, 1, false>(R, ps, RowL{C}, RowL{C}, RowL{C + rf}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 1, false>(R, RowL{C}, RowL{C}, RowL{C + rf}, cols_inner(xh), f, bad);
         else
-          gather_pair<FIELD, true, 2, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 2, false>(R, RowL{C}, RowL{C - rf}, RowL{C}, cols_inner(xh), f, bad);
       }
 #pragma unroll 1
       for (; k < w.nbox; step()) {
         CLBM_PAIR(top);
         if (on_seam(b, xh)) continue;
         float *C = A + ly * rf;
-        gather_pair<FIELD, true, 0, true>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
-                                          pair_force<FIELD>(R, b, map, y, xh, feps), bad, in_box(R, xh, y),
+        gather_pair<ps, true, 0, true>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                          pair_force<FIELD>(R, b, map, y, xh), bad, in_box(R, xh, y),
                                           in_box(R, xh + b.Wh, y));
       }
     } else {
@@ -715,47 +753,52 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
     if (GATHER) {
       if (on_seam(b, xh)) continue;
       float *C = A + ly * rf;
-      gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
-                                         pair_force<FIELD>(R, b, map, y, xh, feps), bad);
+      gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                         pair_force<FIELD>(R, b, map, y, xh), bad);
     } else {
       local(ly, xh, std::integral_constant<bool, false>());
     }
   }
+  // (the field's values come from L2, 700 cycles away, a step's worth of them
+  // fits no nearer: those of the next segment are loaded ahead of this one)
+  auto field_at = [&](int k) -> f2_t {
+    if (!FIELD || k >= w.nseg) return 0;
+    const int i = list[k] + lane, ly = (int)__umulhi((unsigned)i, b.div_wh);
+    return pair_map(b, map, b.row0 + ly, i - ly * b.Wh - 1);
+  };
+  f2_t ahead = field_at(k);
 #pragma unroll 1
   for (; k < w.nseg; step()) {
-    const int i = list[k] + lane;
-    const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = i - ly * b.Wh - 1;
-    // the pair itself: the slots lie at offsets from here that are the same
-    // for every pair of the band
-    float *C = A + ly * rf + 2 * xh;
-    const F32Force2 f = pair_force<FIELD>(R, b, map, b.row0 + ly, xh, feps);
+    float *C = A + 2 * (list[k] + lane - 1);  // the pair itself
+    const f2_t m = ahead;
+    ahead = field_at(k + dk);
+    const F32Force2 f = pair_force<FIELD>(R, m);
     if (GATHER)
-      gather_pair<FIELD, true, 0, false>(R, ps, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(0), f, bad);
+      gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(0), f, bad);
     else
-      local_pair<false>(R, ps, C, f, bad);
+      local_pair<ps, false>(R, C, f, bad);
   }
 #undef CLBM_PAIR
   __syncthreads();
 }
 
-template <int THREADS, int MINB, bool FIELD>
+template <int THREADS, int MINB, int NP, bool FIELD>
 __global__ void __launch_bounds__(THREADS, MINB) k_temporal_f32(TemporalArgs a) {
-  // A[row][k][pair]: a warp's accesses to one population are consecutive 64-bit
+  // A[k][pair]: a warp's accesses to one population are consecutive 64-bit
   // words, in this CTA (no bank conflicts) and across a band edge (whole
   // sectors on the way to the other SM)
+  using Band = BandT<NP>;
   extern __shared__ __align__(16) float A[];
   constexpr int NW = THREADS / 32;
   cg::cluster_group cluster = cg::this_cluster();
-  const Band b = make_band(a, A, cluster);
+  const Band b = make_band<Band>(a, A, cluster);
   const RunDev &R = a.rd;
-  // (the fused load is compiled into the uniform-force kernels only: in the
-  // random-field ones it raised register spills in the step loop)
-  if (!FIELD && a.fused)
+  if (a.fused)
     load_band<THREADS, true>(a, b, A);
   else
     load_band<THREADS, false>(a, b, A);
   const int nseg = segment_count(b.rows, b.Wh), spr = (b.Wh + 31) / 32;
-  unsigned short *list = (unsigned short *)(A + (size_t)18 * b.np);
+  unsigned short *list = (unsigned short *)(A + 9 * Band::ps);
   unsigned char *cls = (unsigned char *)(list + ((nseg + 7) & ~7));
   int *range = (int *)(cls + ((nseg + 15) & ~15));
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -844,25 +887,34 @@ int temporal_rows_limit(int W) {
   return r;
 }
 
-bool temporal_resident(int W, int rows) { return pair_smem(rows, W) <= kSmemLimit; }
+bool temporal_resident(int W, int rows) {
+  return (long long)rows * ((W + 1) / 2) <= kPairs && pair_smem(kPairs, rows, W) <= kSmemLimit;
+}
 
 struct TemporalVariant {
   int threads;
-  TemporalFn fn[2];  // [field]
+  TemporalFn fn[2][2];  // [plane size: kPairs, kPairsHalf][field]
 };
 
-#define GENERIC(T, M) {k_temporal_f32<T, M, false>, k_temporal_f32<T, M, true>}
-static const TemporalVariant kTemporal[] = {{1024, GENERIC(1024, 1)}, {512, GENERIC(512, 1)}, {256, GENERIC(256, 2)}};
+#define GENERIC(T, M, N) {k_temporal_f32<T, M, N, false>, k_temporal_f32<T, M, N, true>}
+// (1024 and 512 threads take an SM's registers alone: no use for the half planes)
+static const TemporalVariant kTemporal[] = {{1024, {GENERIC(1024, 1, kPairs), {nullptr, nullptr}}},
+                                            {512, {GENERIC(512, 1, kPairs), {nullptr, nullptr}}},
+                                            {256, {GENERIC(256, 2, kPairs), GENERIC(256, 2, kPairsHalf)}}};
 #undef GENERIC
 
 int temporal_variant_count() { return (int)(sizeof(kTemporal) / sizeof(kTemporal[0])); }
 
-// the kernel of a variant for this band shape, or nullptr when it cannot run it
-static TemporalFn temporal_fn(int variant, int cs, int W, int rows_max, bool field) {
+// the kernel of a variant for this band shape and its shared memory, or
+// nullptr when it cannot run it
+static TemporalFn temporal_fn(int variant, int cs, int W, int rows_max, bool field, size_t *smem) {
   if (variant < 0 || variant >= temporal_variant_count() || cs < 1 || cs > MAX_CLUSTER || rows_max < 1)
     return nullptr;
   if (temporal_smem(rows_max * W) > kSmemLimit) return nullptr;
-  return kTemporal[variant].fn[field];
+  const TemporalVariant &v = kTemporal[variant];
+  const bool half = v.fn[1][field] && rows_max * ((W + 1) / 2) <= kPairsHalf;
+  *smem = std::min(pair_smem(half ? kPairsHalf : kPairs, rows_max, W), kSmemLimit);
+  return v.fn[half][field];
 }
 
 static cudaLaunchConfig_t temporal_config(int cs, int variant, int nclones, size_t smem, cudaStream_t s,
@@ -900,9 +952,9 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
     if (rows < 1) return cudaErrorInvalidConfiguration;
     rows_max = std::max(rows_max, rows);
   }
-  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field);
+  size_t smem = 0;
+  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field, &smem);
   if (!fn || !temporal_resident(W, rows_max) || a.steps < 1) return cudaErrorInvalidConfiguration;
-  const size_t smem = pair_smem(rows_max, W);
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
   TemporalArgs args = a;
@@ -915,9 +967,9 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
 
 // Whether the cluster shape can be resident at all (occupancy query, no launch).
 int temporal_max_clusters(int cs, int variant, int W, int rows_max, bool field) {
-  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field);
+  size_t smem = 0;
+  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field, &smem);
   if (!fn) return 0;
-  const size_t smem = std::min(pair_smem(rows_max, W), kSmemLimit);
   if (prepare(fn, cs, smem) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = temporal_config(cs, variant, 64, smem, nullptr, attr);

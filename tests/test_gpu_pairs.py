@@ -23,6 +23,7 @@ def variant(cs, tv):
     (3, 50, 0, 1, 20, 24, 1, 0, None, False),          # two pairs per row
     (130, 26, 30, 36, 11, 15, 4, 1, [1, 12, 12, 1], False),  # one-row bands
     (64, 12, 20, 44, 1, 10, 3, 1, None, False),        # square next to both walls, in every band
+    (130, 60, 40, 52, 24, 36, 2, 2, None, True),       # 256 threads with planes of the full size
     (97, 66, 20, 33, 25, 38, 1, 1, None, False),       # accepted, but one node per row too large: streams
 ])
 def test_pairs_equal_streaming(gpu, clbm_lib, W, H, xmin, xmax, ymin, ymax, cs, tv, rows, field):

@@ -61,16 +61,19 @@ def check(W, H, box, rows):
     row0 = [sum(rows[:b]) for b in range(cs + 1)]
     div = ((1 << 32) + Wh - 1) // Wh
     in_box = lambda x, y: xmin <= x <= xmax and ymin <= y <= ymax  # noqa: E731
-    ps = 2 * Wh
+    ps = 2 * 3220  # floats per plane
+    assert max(rows) * Wh <= 3220
     col = lambda x: 2 * x if x < Wh else 2 * (x - Wh) + 1  # noqa: E731
     solid = lambda x, y: xmin < x < xmax and ymin < y < ymax  # noqa: E731
     owner, updated, counts = {}, {}, [0] * 6
 
     def decode(b, row, off):
         """(x, y, k) of float offset `off` in row `row` of band b; x = W: the empty lane"""
-        assert 0 <= row < rows[b] and 0 <= off < 9 * ps
-        k, r = divmod(off, ps)
-        return (r >> 1) + (r & 1) * Wh, row0[b] + row, k
+        assert 0 <= row < rows[b]
+        k, r = divmod(row * 2 * Wh + off, ps)
+        i, h = divmod(r, 2)
+        assert 0 <= k < 9 and i // Wh == row
+        return i % Wh + h * Wh, row0[b] + row, k
 
     def node(x, y, slots):
         """slots[k] = where S(n,k) is read and P(n, opp k) written"""
@@ -160,7 +163,7 @@ def check(W, H, box, rows):
             for i, ly, xh, q in lanes:
                 if q and not on_seam(xh):
                     if c == INNER:
-                        assert xh == i - ly * Wh - 1
+                        assert i - 1 == ly * Wh + xh
                     pair(c, ly, xh)
     assert len(updated) == sum(not solid(x, y) for x in range(W) for y in range(H))
     return counts
