@@ -41,7 +41,7 @@ struct AdjArgs {
 // while the run's field acts (t < field_steps), else beta, as the forward
 template <typename T>
 __device__ __forceinline__ T adj_beta(const RunDev &R, const AdjArgs &a, int clone, int n) {
-  if (!(R.field_mode && a.maps && a.t < R.field_steps)) return (T)R.beta;
+  if (!(R.field_mode && a.maps && a.t < R.field_steps)) return sizeof(T) == 8 ? (T)R.beta : (T)R.f_beta;
   const float m = a.maps[R.map_base + (long long)clone * R.nodes + n];
   if (sizeof(T) == 8) return (T)(R.beta * (1.0 + R.field_eps * (double)m));
   return (T)field_beta_f32(R.f_beta, R.f_field_eps, m);
@@ -103,13 +103,16 @@ __device__ __forceinline__ void drag_grad(const RunDev &R, int x, int y, const T
 template <typename T>
 __device__ __forceinline__ void collide_adjoint(const RunDev &R, const T S[9], const T pi[9], T beta,
                                                 T out[9]) {
-  const T omega = (T)R.omega, om1 = T(1) - omega;
-  const T cf = (T)R.cforce;
+  // (FP32: constants converted on the host -- a conversion from FP64 takes the
+  // FP64 pipe, and three per node made it the bound of the whole kernel)
+  const T omega = sizeof(T) == 8 ? (T)R.omega : (T)R.adj_omega, om1 = T(1) - omega;
+  const T cf = sizeof(T) == 8 ? (T)R.cforce : (T)R.adj_cforce;
   T sum = ((S[0] + (S[1] + S[3])) + (S[2] + S[4])) + ((S[5] + S[7]) + (S[6] + S[8]));
   const T rho = (sizeof(T) == 8 ? sum : T(1) + sum);
   const T jx = (S[1] - S[3]) + ((S[5] - S[7]) + (S[8] - S[6]));
   const T jy = (S[2] - S[4]) + ((S[5] - S[7]) + (S[6] - S[8]));
-  const T ux = (jx + T(0.5) * beta) / rho, uy = jy / rho;
+  const T inv = T(1) / rho;  // one division for all three quotients
+  const T ux = (jx + T(0.5) * beta) * inv, uy = jy * inv;
   const T u2 = T(1.5) * (ux * ux + uy * uy);
   const T wa = T(1) / T(9), wd = T(1) / T(36);
   const T a13 = pi[1] + pi[3], a24 = pi[2] + pi[4];
@@ -125,7 +128,6 @@ __device__ __forceinline__ void collide_adjoint(const RunDev &R, const T S[9], c
   const T Gx = omega * rho * (T(3) * Px + T(9) * (ux * Pxx + uy * Pxy) - T(3) * ux * P0) +
                cf * beta * (T(9) * Pxx - T(3) * P0);
   const T Gy = omega * rho * (T(3) * Py + T(9) * (ux * Pxy + uy * Pyy) - T(3) * uy * P0) + T(9) * cf * beta * Pxy;
-  const T inv = T(1) / rho;
   const T A = G0 - (ux * Gx + uy * Gy) * inv;
   const T Bx = Gx * inv, By = Gy * inv;
 #pragma unroll
@@ -141,9 +143,9 @@ __global__ void __launch_bounds__(STEP_BLOCK) k_adj_step(AdjArgs a) {
   if (n >= R.nodes || clone >= R.nclones) return;
   const long long plane = R.plane;
   const long long cb = R.pop_base + (long long)clone * 9 * plane;
-  const T *sig = (const T *)a.sigma_in + cb;
-  const T *P = (const T *)a.P + cb;
-  T *out = (T *)a.sigma_out + cb;
+  const T *__restrict__ sig = (const T *)a.sigma_in + cb;
+  const T *__restrict__ P = (const T *)a.P + cb;
+  T *__restrict__ out = (T *)a.sigma_out + cb;
   const int W = R.W, y = (int)__umulhi((unsigned)n, R.div_w), x = n - y * W;
   const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
   const int mask = (in_box || y == 0 || y == R.H - 1) ? bounce_mask(R, x, y) : 0;
@@ -154,28 +156,27 @@ __global__ void __launch_bounds__(STEP_BLOCK) k_adj_step(AdjArgs a) {
   }
   const int xl = (x == 0) ? W - 1 : x - 1, xr = (x == W - 1) ? 0 : x + 1;
   const int row = y * W;
-  T S[9], pi[9];
+  // S_t(n,k) = P_{t-1}(n - c_k, k), or P_{t-1}(n, opp k) when bounced;
+  // P(n,k) is read by slot (n, opp k) when that slot bounces, else by (n + c_k, k)
+  int at[9];  // slot (n - c_k, k), the same offset for P and, of direction opp k, for sigma
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const int cx = cx_of(k), cy = cy_of(k);
-    // S_t(n,k) = P_{t-1}(n - c_k, k), or P_{t-1}(n, opp k) when bounced
-    if (a.from_s0) {
-      S[k] = P[k * plane + n];
-    } else {
-      const int sx = cx == 1 ? xl : (cx == -1 ? xr : x);
-      const int srow = cy == 1 ? row - W : (cy == -1 ? row + W : row);
-      S[k] = ((mask >> k) & 1) ? P[opp_of(k) * plane + n] : P[k * plane + srow + sx];
-    }
-    // P(n,k) is read by slot (n, opp k) when that slot bounces, else by (n + c_k, k)
-    const int ok = opp_of(k);
-    if ((mask >> ok) & 1) {
-      pi[k] = sig[ok * plane + n];
-    } else {
-      const int tx = cx == 1 ? xr : (cx == -1 ? xl : x);
-      const int trow = cy == 1 ? row + W : (cy == -1 ? row - W : row);
-      pi[k] = sig[k * plane + trow + tx];
-    }
+    const int sx = cx == 1 ? xl : (cx == -1 ? xr : x);
+    at[k] = (cy == 1 ? row - W : (cy == -1 ? row + W : row)) + sx;
   }
+  T S[9], pi[9];
+  if (a.from_s0) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) S[k] = __ldg(P + k * plane + n);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      S[k] = __ldg(P + (((mask >> k) & 1) ? opp_of(k) * plane + n : k * plane + at[k]));
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++)  // n + c_k = n - c_{opp k}
+    pi[k] = __ldg(sig + (((mask >> opp_of(k)) & 1) ? opp_of(k) * plane + n : k * plane + at[opp_of(k)]));
   T o[9];
   collide_adjoint<T>(R, S, pi, adj_beta<T>(R, a, clone, n), o);
   if (a.with_drag && in_box) {

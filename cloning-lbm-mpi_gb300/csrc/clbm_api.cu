@@ -368,6 +368,8 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
       return fail(CLBM_ERR_INVALID, "tau out of range for the FP32 collision (need 0.5 < tau)");
     }
     R.f_beta = (float)d.beta;
+    R.adj_omega = (float)R.omega;
+    R.adj_cforce = (float)R.cforce;
     R.f_force = f32_force(R.f_beta, R.f_cforce);
     R.f_pairs = f32_pairs(R.f_omega, R.f_om1, R.f_c13, R.f_c2, R.f_force);
     R.f_force2 = f32_force2(R.f_force, R.f_force);

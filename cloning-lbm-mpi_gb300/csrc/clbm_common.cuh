@@ -168,6 +168,7 @@ struct RunDev {
   // grid, c2 ~ omega/12 on a 2^-25 grid), om1 = 1 - omega' and
   // cforce = 1 - omega'/2 exactly; f_force = f32_force(f_beta, f_cforce)
   float f_omega, f_om1, f_c13, f_c2, f_cforce, f_beta;
+  float adj_omega, adj_cforce; // (float)omega, (float)cforce: the FP32 adjoint's
   F32Force f_force;
   F32Pairs f_pairs;            // the same constants packed for the f32x2 collision
   F32Force2 f_force2;          // f_force in both lanes, for the two-node collision
