@@ -121,8 +121,10 @@ __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
     T *terms = (T *)a.terms + (long long)a.step * a.term_slab + R.term_base;
     store_drag_terms<F64>(R, S, x, y, L.clone, terms);
   }
-  // (the density as moments_ref64 sums it: one sum for both uses)
-  if (!(moments_ref64(S).rho > 0.0)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
+  // (the density as moments_ref64 sums it: one sum for both uses; positive or
+  // +inf as an integer test of its bits, off the FP64 pipe)
+  const long long rho = __double_as_longlong(moments_ref64(S).rho);
+  if (!(rho > 0 && rho <= 0x7ff0000000000000ll)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
   if (LAST) {
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = S[k];
