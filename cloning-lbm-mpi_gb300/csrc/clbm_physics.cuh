@@ -458,14 +458,16 @@ __device__ __forceinline__ void store_drag_terms(
     const RunDev &R, const typename std::conditional<F64, double, float>::type S[9], int x, int y,
     int clone, typename std::conditional<F64, double, float>::type *T) {
   const int sy = R.ymax - R.ymin, sx = R.xmax - R.xmin;
-  const int nc = R.nclones;
+  // (32-bit offsets: a step's terms of one run are under 2^32, since W >= 3
+  // and its populations, 18 W H values a clone, fit the device)
+  const unsigned nc = R.nclones;
   if (R.drag_mode == 1) {
     const auto v = me_node_term<F64>(S, bounce_mask(R, x, y));
     const bool corner_x = x == R.xmin || x == R.xmax;
-    if (x == R.xmin) T[(long long)(y - R.ymin) * nc + clone] = v;
-    if (x == R.xmax) T[(long long)(sy + 1 + y - R.ymin) * nc + clone] = v;
-    if (y == R.ymax) T[(long long)(2 * (sy + 1) + x - R.xmin) * nc + clone] = corner_x ? 0 : v;
-    if (y == R.ymin) T[(long long)(2 * (sy + 1) + sx + 1 + x - R.xmin) * nc + clone] = corner_x ? 0 : v;
+    if (x == R.xmin) T[(unsigned)(y - R.ymin) * nc + clone] = v;
+    if (x == R.xmax) T[(unsigned)(sy + 1 + y - R.ymin) * nc + clone] = v;
+    if (y == R.ymax) T[(unsigned)(2 * (sy + 1) + x - R.xmin) * nc + clone] = corner_x ? 0 : v;
+    if (y == R.ymin) T[(unsigned)(2 * (sy + 1) + sx + 1 + x - R.xmin) * nc + clone] = corner_x ? 0 : v;
     return;
   }
   typename std::conditional<F64, double, float>::type west, east, north, south;
@@ -487,10 +489,10 @@ __device__ __forceinline__ void store_drag_terms(
     north = __fmul_rn(-c, pxy);
     south = __fmul_rn(c, pxy);
   }
-  if (x == R.xmin) T[(long long)(y - R.ymin) * nc + clone] = west;
-  if (x == R.xmax) T[(long long)(sy + 1 + y - R.ymin) * nc + clone] = east;
-  if (y == R.ymax) T[(long long)(2 * (sy + 1) + x - R.xmin) * nc + clone] = north;
-  if (y == R.ymin) T[(long long)(2 * (sy + 1) + sx + 1 + x - R.xmin) * nc + clone] = south;
+  if (x == R.xmin) T[(unsigned)(y - R.ymin) * nc + clone] = west;
+  if (x == R.xmax) T[(unsigned)(sy + 1 + y - R.ymin) * nc + clone] = east;
+  if (y == R.ymax) T[(unsigned)(2 * (sy + 1) + x - R.xmin) * nc + clone] = north;
+  if (y == R.ymin) T[(unsigned)(2 * (sy + 1) + sx + 1 + x - R.xmin) * nc + clone] = south;
 }
 
 }  // namespace clbm

@@ -119,6 +119,17 @@ struct RowC {
   __device__ __forceinline__ void st2(int o, f2_t v) const { st_cluster2(a + 4u * o, v); }
 };
 
+// ... by a generic pointer, for rows that are in this CTA for some lanes and in
+// a neighbour for others (a shared::cluster address of this CTA would go over
+// the network between SMs too).
+struct RowG {
+  float *p;
+  __device__ __forceinline__ float ld(int o) const { return p[o]; }
+  __device__ __forceinline__ void st(int o, float v) const { p[o] = v; }
+  __device__ __forceinline__ f2_t ld2(int o) const { return *(const f2_t *)(p + o); }
+  __device__ __forceinline__ void st2(int o, f2_t v) const { *(f2_t *)(p + o) = v; }
+};
+
 // Columns of a pair: float offsets of the pair itself (lane 0; lane 1 is one
 // further) and of its left (m) and right (p) neighbours, per lane.
 struct Cols {
@@ -325,10 +336,10 @@ __device__ __forceinline__ void perimeter_node(const RunDev &R, int ylo, int yhi
 
 // One node of the square's perimeter, not the last step of the interval:
 // bounce-back masks, drag terms.  Gather step: P(n, opp k) goes back to the
-// slot S(n,k) came from, unless that lies inside the square (the push is
-// dropped); with the square at a band edge the rows may lie in adjacent bands
-// (shared::cluster addresses), else the three are in this CTA (plain indexing, which the compiler
-// schedules freely).
+// slot S(n,k) came from (never inside the square: every slot across its
+// surface bounces back); with the square at a band edge the rows may lie in
+// adjacent bands (shared::cluster addresses), else the three are in this CTA
+// (plain indexing, which the compiler schedules freely).
 template <bool GATHER, class Band>
 __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Band &b, int x, int y, bool edge,
                                                  const float *map, float feps, bool &bad, float *terms, float *A) {
@@ -365,19 +376,10 @@ __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Ba
   bad |= !(drho > -1.0f);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const int ok = opp_of(k);
-    bool keep = true;
-    if (GATHER && !((mask >> ok) & 1)) {  // into the square?
-      const int cx = cx_of(k);
-      const int tx = cx == 1 ? (x == b.W - 1 ? 0 : x + 1) : (cx == -1 ? (x == 0 ? b.W - 1 : x - 1) : x);
-      const int ty = y + cy_of(k);
-      keep = !(tx > R.xmin && tx < R.xmax && ty > R.ymin && ty < R.ymax);
-    }
-    if (remote) {
-      if (keep) st_cluster(4u * (unsigned)at[ok], P[k]);
-    } else {
-      if (keep) A[at[ok]] = P[k];
-    }
+    if (remote)
+      st_cluster(4u * (unsigned)at[opp_of(k)], P[k]);
+    else
+      A[at[opp_of(k)]] = P[k];
   }
   store_drag_terms<false>(R, S, x, y, b.clone, terms);
 }
@@ -521,8 +523,8 @@ __device__ __forceinline__ void cluster_wait() {
 
 // One step of the band (all but the interval's last step).  Work comes in
 // warp-sized entries, dealt out in this order:
-//   seam    (gather) the seam pairs of the first and the last row, every slot
-//           at a per-lane shared::cluster address
+//   seam    (gather) the seam pairs of the first and the last row, columns and
+//           neighbour rows per lane
 //   GENERAL segments of a one-row band, or where the square touches a
 //           band-edge row: the same path
 //   EDGE    a band-edge row, the row across the edge at shared::cluster
@@ -625,10 +627,11 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
   const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = pair_of(b, i - ly * b.Wh), y = b.row0 + ly
   auto general = [&](int ly, int xh) {
     const int y = b.row0 + ly;
-    const RowC C{b.own_c + 4u * (unsigned)(ly * rf)};
+    float *C0 = A + ly * rf;
     const bool wb = y == 0, wt = y == b.H - 1;
-    const RowC U{wb ? C.a : (ly == 0 ? b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf) : C.a - 4u * (unsigned)rf)};
-    const RowC D{wt ? C.a : (ly == b.rows - 1 ? b.next_c : C.a + 4u * (unsigned)rf)};
+    const RowL C{C0};
+    const RowG U{wb ? C0 : (ly == 0 ? b.prev + (b.rows_prev - 1) * rf : C0 - rf)};
+    const RowG D{wt ? C0 : (ly == b.rows - 1 ? b.next : C0 + rf)};
     gather_pair<ps, false, 3, true>(R, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh), bad,
                                        in_box(R, xh, y), in_box(R, xh + b.Wh, y), wb, wt);
   };

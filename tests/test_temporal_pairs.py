@@ -103,6 +103,7 @@ def check(W, H, box, rows):
             for k in range(9):
                 row, sx = {1: U, 0: C, -1: D}[CY[k]], {1: cm, 0: co, -1: cp}[CX[k]]
                 slots.append(decode(*C, co + k * ps) if k in m else decode(*row, sx + OPP[k] * ps))
+            assert not any(solid(*s[:2]) for s in slots)  # every slot across the surface bounces back
             node(x, y, slots)
 
         def pair(c, ly, xh):
