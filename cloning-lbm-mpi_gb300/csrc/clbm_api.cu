@@ -774,6 +774,26 @@ static cudaError_t ensure_side(clbm_ctx *c, int n) {
   return cudaSuccess;
 }
 
+// The cluster-resident kernel's arguments for run r of a plan.
+static TemporalArgs temporal_args(const clbm_ctx *c, const LbPlan &p, int r, int steps, const float *src, float *dst) {
+  TemporalArgs ta{};
+  ta.rd = c->runs_h[r];
+  ta.run = r;
+  ta.steps = steps;
+  ta.src = src;
+  ta.dst = dst;
+  ta.terms = (float *)c->d.terms;
+  ta.term_slab = c->d.term_slab;
+  ta.err = c->d.err;
+  ta.maps = c->d_maps;
+  const int cs = p.cs[r];
+  if (r < (int)p.rows.size() && (int)p.rows[r].size() == cs + 1)
+    std::copy(p.rows[r].begin(), p.rows[r].end(), ta.band_row0);
+  else
+    even_band_rows(ta.rd.H, cs, ta.band_row0);
+  return ta;
+}
+
 // Enqueue `steps` LB steps of the plan's runs.  Interval: P_0 in buffer src,
 // S_T left in buffer dst; the streaming runs alternate between the two
 // buffers as the pull scheme does and store S on their last step.  timing
@@ -798,13 +818,12 @@ static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int
     const RunDev &R = c->runs_h[r];
     cudaStream_t ts = c->side[i];
     if ((e = cudaStreamWaitEvent(ts, c->fork_join[0], 0)) != cudaSuccess) return e;
-    TemporalArgs ta{R, r, steps, (const float *)c->pop[src], (float *)c->pop[dst], (float *)c->d.terms,
-                    c->d.term_slab, c->d.err, c->d_maps, {}, fuse ? 1 : 0, fuse ? *fuse : ReseedArgs{}};
     const int cs = p.cs[r];
-    if (r < (int)p.rows.size() && (int)p.rows[r].size() == cs + 1)
-      std::copy(p.rows[r].begin(), p.rows[r].end(), ta.band_row0);
-    else
-      even_band_rows(R.H, cs, ta.band_row0);
+    TemporalArgs ta = temporal_args(c, p, r, steps, (const float *)c->pop[src], (float *)c->pop[dst]);
+    if (fuse) {
+      ta.fused = 1;
+      ta.rs = *fuse;
+    }
     if ((e = launch_temporal(ta, cs, p.tv[r], R.nclones, R.W, ts)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(c->fork_join[1 + i], ts)) != cudaSuccess) return e;
     i++;
@@ -1692,6 +1711,32 @@ static cudaError_t adj_reserve(char *&p, size_t &have, size_t need) {
   return e;
 }
 
+// The adjoint's forward through the cluster-resident kernel: every run
+// resident, uniform force (the kernel's random-field form keeps no
+// checkpoints).  The same bits as the streaming steps; 64 clones of 400x100
+// take 17 us per step against 31.  (The backward's recomputation keeps every
+// step's P, 92 MB each there: writing alone takes 37 us, so it streams.)
+static bool adj_resident(const clbm_ctx *c) {
+  bool all = c->precision == CLBM_FP32 && !c->any_field;
+  for (int r = 0; r < c->nruns; r++) all = all && run_resident(c, r);
+  return all;
+}
+
+// `steps` steps from P_0 in ckpt; P_t kept at ckpt + t / every * (a population
+// buffer) for every t that `every` divides, S_T to dst.
+static cudaError_t adj_forward(clbm_ctx *c, int steps, void *ckpt, int every, void *dst) {
+  const LbPlan p = current_plan(c, false);
+  for (int r = 0; r < c->nruns; r++) {
+    TemporalArgs ta = temporal_args(c, p, r, steps, (const float *)ckpt, (float *)dst);
+    ta.keep = (float *)ckpt;
+    ta.keep_stride = (long long)c->pop_elems;
+    ta.keep_every = every;
+    const cudaError_t e = launch_temporal(ta, p.cs[r], p.tv[r], ta.rd.nclones, ta.rd.W, c->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 extern "C" int clbm_drag_fwd(clbm_ctx *c, int steps, int every, double *J) {
   if (!c) return fail(CLBM_ERR_INVALID, "ctx is NULL");
   if (steps < 1 || steps > c->max_steps || every < 1) return fail(CLBM_ERR_INVALID, "bad steps / checkpoint period");
@@ -1718,7 +1763,9 @@ extern "C" int clbm_drag_fwd(clbm_ctx *c, int steps, int every, double *J) {
   ReseedArgs ra{c->d.runs, c->nruns, c->adj.s0, loc(0), c->d_identity, c->d_zeros, c->d.pert,
                 c->d.prefactors, c->d.snaps, c->d.state, c->d.err, c->d_maps};
   CK(launch_reseed(f64, ra, c->total_blocks, tiles64(c), s));
-  for (int t = 0; t < steps; t++) {
+  const bool resident = adj_resident(c);
+  if (resident) CK(adj_forward(c, steps, c->adj.ckpt, every, c->adj.sig[0]));
+  for (int t = 0; t < steps && !resident; t++) {
     char *dst = (t + 1 < steps) ? loc(t + 1) : c->adj.sig[(t + 1) % 2];
     StepArgs a{c->d.runs, c->nruns, t, loc(t), dst, c->d.terms, c->d.term_slab, c->d.err,
                c->total_clones, c->max_nodes, {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]},

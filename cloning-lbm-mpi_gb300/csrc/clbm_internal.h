@@ -118,6 +118,12 @@ struct TemporalArgs {
   int fused;
   ReseedArgs rs;
   unsigned div_wh;    // ceil(2^32 / pairs per row), set by launch_temporal
+  // checkpoints (uniform force only): P_t of every t that keep_every divides
+  // goes to keep + t / keep_every * keep_stride, laid out as a population
+  // buffer
+  float *keep;
+  long long keep_stride;
+  int keep_every;
 };
 
 

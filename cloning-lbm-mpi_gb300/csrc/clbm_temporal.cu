@@ -204,6 +204,23 @@ __device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, 
   return pair_force<FIELD>(R, FIELD ? pair_map(b, map, y, xh) : 0ull);
 }
 
+// Where a pair's post-collision populations go besides A (checkpoints of the
+// adjoint's forward): node (x, y) of plane 0, nullptr for nowhere; lane 1's
+// node lies half columns further, if there is one.
+struct Keep {
+  float *p;
+  int half;
+};
+template <bool STORE>
+__device__ __forceinline__ void keep_pair(const RunDev &R, const Keep &kp, const f2_t P[9], bool skip0, bool skip1) {
+  if (!STORE || !kp.p) return;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    if (!skip0) kp.p[k * R.plane] = f32x2op::lo(P[k]);
+    if (!skip1 && kp.half) kp.p[k * R.plane + kp.half] = f32x2op::hi(P[k]);
+  }
+}
+
 // One pair of nodes in a gather step.  C, U, D: the pair's row and the rows
 // y - 1 and y + 1.  S(n,k) is read from A[n - c_k][opp k] and P(n, opp k)
 // goes back to that slot (the pull rules make the two the same).  WALL: 1 =
@@ -211,9 +228,9 @@ __device__ __forceinline__ F32Force2 pair_force(const RunDev &R, const Band &b, 
 // wall, slots 4, 7, 8 (the row beyond the wall is not touched); 3 = by the
 // thread's wb / wt.  UNI: both lanes' neighbour columns lie in one pair, every
 // slot pair is one 64-bit access.  PRED: lane h is written only if !skip_h.
-template <int ps, bool UNI, int WALL, bool PRED, class RC, class RU, class RD>
+template <int ps, bool UNI, int WALL, bool PRED, bool STORE, class RC, class RU, class RD>
 __device__ __forceinline__ void gather_pair(const RunDev &R, const RC C, const RU U, const RD D, const Cols &c,
-                                            const F32Force2 &f, bool &bad, bool skip0 = false, bool skip1 = false,
+                                            const F32Force2 &f, const Keep &kp, bool &bad, bool skip0 = false, bool skip1 = false,
                                             bool wb = false, bool wt = false) {
   auto ld = [](const auto &row, int a, int b2, int q) {
     return UNI ? row.ld2(a + q) : f2_bits(row.ld(a + q), row.ld(b2 + q));
@@ -249,6 +266,7 @@ __device__ __forceinline__ void gather_pair(const RunDev &R, const RC C, const R
   }
   f2_t P[9];
   const f2_t drho = collide_f32_nodes(S, P, R.f_pairs, f);
+  keep_pair<STORE>(R, kp, P, PRED && skip0, PRED && skip1);
   bad |= (!(f32x2op::lo(drho) > -1.0f) && !(PRED && skip0)) || (!(f32x2op::hi(drho) > -1.0f) && !(PRED && skip1));
   auto st = [&](const auto &row, int a, int b2, int q, f2_t v) {
     if (UNI && !PRED) {
@@ -290,13 +308,14 @@ __device__ __forceinline__ void gather_pair(const RunDev &R, const RC C, const R
 }
 
 // One pair of nodes in a local step: S(n,k) = A[n][k], P(n,k) -> A[n][opp k].
-template <int ps, bool PRED>
-__device__ __forceinline__ void local_pair(const RunDev &R, float *o, const F32Force2 &f, bool &bad,
+template <int ps, bool PRED, bool STORE>
+__device__ __forceinline__ void local_pair(const RunDev &R, float *o, const F32Force2 &f, const Keep &kp, bool &bad,
                                            bool skip0 = false, bool skip1 = false) {
   f2_t S[9], P[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) S[k] = *(const f2_t *)(o + k * ps);
   const f2_t drho = collide_f32_nodes(S, P, R.f_pairs, f);
+  keep_pair<STORE>(R, kp, P, PRED && skip0, PRED && skip1);
   bad |= (!(f32x2op::lo(drho) > -1.0f) && !(PRED && skip0)) || (!(f32x2op::hi(drho) > -1.0f) && !(PRED && skip1));
 #pragma unroll
   for (int k = 0; k < 9; k++) {
@@ -340,9 +359,9 @@ __device__ __forceinline__ void perimeter_node(const RunDev &R, int ylo, int yhi
 // surface bounces back); with the square at a band edge the rows may lie in
 // adjacent bands (shared::cluster addresses), else the three are in this CTA
 // (plain indexing, which the compiler schedules freely).
-template <bool GATHER, class Band>
+template <bool GATHER, bool STORE, class Band>
 __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Band &b, int x, int y, bool edge,
-                                                 const float *map, float feps, bool &bad, float *terms, float *A) {
+                                                 const float *map, float feps, float *keep, bool &bad, float *terms, float *A) {
   const RunDev &R = a.rd;
   const bool remote = GATHER && edge;  // a local step stays in A
   const int ly = y - b.row0, rf = b.rowf;
@@ -380,6 +399,10 @@ __device__ __forceinline__ void perimeter_update(const TemporalArgs &a, const Ba
       st_cluster(4u * (unsigned)at[opp_of(k)], P[k]);
     else
       A[at[opp_of(k)]] = P[k];
+  }
+  if (STORE && keep) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) keep[k * b.plane + (long long)y * b.W + x] = P[k];
   }
   store_drag_terms<false>(R, S, x, y, b.clone, terms);
 }
@@ -612,7 +635,7 @@ __device__ __forceinline__ WarpPlan warp_plan(const RunDev &R, const Band &b, co
   return p;
 }
 
-template <int NW, bool GATHER, bool FIELD, class Band>
+template <int NW, bool GATHER, bool FIELD, bool STORE, class Band>
 __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, const WarpPlan &w, float *A,
                                           const unsigned short *list, const int *range, int warp, int lane, int t,
                                           const float *map, bool &bad) {
@@ -620,6 +643,13 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
   const float feps = FIELD ? field_eps(a, t) : 0.0f;
   constexpr int ps = Band::ps;
   const int rf = b.rowf;
+  // this step's checkpoint of the clone, if it is one
+  float *keep = STORE && a.keep && (t + 1) % a.keep_every == 0
+                    ? a.keep + (t + 1) / a.keep_every * a.keep_stride + R.pop_base + (long long)b.clone * 9 * b.plane
+                    : nullptr;
+  auto keep_at = [&](int y, int xh) {
+    return Keep{STORE && keep ? keep + (long long)y * b.W + xh : nullptr, STORE && xh + b.Wh < b.W ? b.Wh : 0};
+  };
   // the pair of segment position i: its row and column, inactive past `lim`
 #define CLBM_PAIR(lim)                                                                         \
   const int i = list[k] + lane;                                                                \
@@ -632,13 +662,13 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
     const RowL C{C0};
     const RowG U{wb ? C0 : (ly == 0 ? b.prev + (b.rows_prev - 1) * rf : C0 - rf)};
     const RowG D{wt ? C0 : (ly == b.rows - 1 ? b.next : C0 + rf)};
-    gather_pair<ps, false, 3, true>(R, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh), bad,
+    gather_pair<ps, false, 3, true, STORE>(R, C, U, D, cols_any(b, xh), pair_force<FIELD>(R, b, map, y, xh), keep_at(y, xh), bad,
                                        in_box(R, xh, y), in_box(R, xh + b.Wh, y), wb, wt);
   };
   auto local = [&](int ly, int xh, auto pred) {
     const int y = b.row0 + ly;
     constexpr bool P = decltype(pred)::value;
-    local_pair<ps, P>(R, A + ly * rf + 2 * xh, pair_force<FIELD>(R, b, map, y, xh), bad, P && in_box(R, xh, y),
+    local_pair<ps, P, STORE>(R, A + ly * rf + 2 * xh, pair_force<FIELD>(R, b, map, y, xh), keep_at(y, xh), bad, P && in_box(R, xh, y),
                   P && in_box(R, xh + b.Wh, y));
   };
   const bool lead = w.flags & (PLAN_HEAD << GATHER);
@@ -672,10 +702,10 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         float *C = A + ly * rf;
         const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh);
         if (ly == 0)  // warp-uniform
-          gather_pair<ps, true, 0, false>(R, RowL{C}, RowC{b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf)},
-                                             RowL{C + rf}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 0, false, STORE>(R, RowL{C}, RowC{b.prev_c + 4u * (unsigned)((b.rows_prev - 1) * rf)},
+                                             RowL{C + rf}, cols_inner(xh), f, keep_at(y, xh), bad);
         else
-          gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowC{b.next_c}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 0, false, STORE>(R, RowL{C}, RowL{C - rf}, RowC{b.next_c}, cols_inner(xh), f, keep_at(y, xh), bad);
       }
     } else {
 #pragma unroll 1
@@ -698,7 +728,7 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
       if (j >= h.nper) continue;
       int x, y;
       perimeter_node(R, h.ylo, h.yhi, j, x, y);
-      perimeter_update<GATHER>(a, b, x, y, box_edge, FIELD ? map : nullptr, feps, bad, terms, A);
+      perimeter_update<GATHER, STORE>(a, b, x, y, box_edge, FIELD ? map : nullptr, feps, keep, bad, terms, A);
     }
   }
   if (b.cs > 1 && box_edge) cluster_arrive(true);
@@ -718,8 +748,8 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         if (j >= ninner) continue;
         const int r = ns == 2 ? j >> 1 : j / 3, ly = r + 1, xh = seam_pair(b, j - ns * r), y = b.row0 + ly;
         float *C = A + ly * rf;
-        gather_pair<ps, false, 0, true>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_any(b, xh),
-                                           pair_force<FIELD>(R, b, map, y, xh), bad, in_box(R, xh, y),
+        gather_pair<ps, false, 0, true, STORE>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_any(b, xh),
+                                           pair_force<FIELD>(R, b, map, y, xh), keep_at(y, xh), bad, in_box(R, xh, y),
                                            in_box(R, xh + b.Wh, y));
       }
 #pragma unroll 1
@@ -729,17 +759,17 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
         float *C = A + ly * rf;
         const F32Force2 f = pair_force<FIELD>(R, b, map, y, xh);
         if (y == 0)  // warp-uniform
-          gather_pair<ps, true, 1, false>(R, RowL{C}, RowL{C}, RowL{C + rf}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 1, false, STORE>(R, RowL{C}, RowL{C}, RowL{C + rf}, cols_inner(xh), f, keep_at(y, xh), bad);
         else
-          gather_pair<ps, true, 2, false>(R, RowL{C}, RowL{C - rf}, RowL{C}, cols_inner(xh), f, bad);
+          gather_pair<ps, true, 2, false, STORE>(R, RowL{C}, RowL{C - rf}, RowL{C}, cols_inner(xh), f, keep_at(y, xh), bad);
       }
 #pragma unroll 1
       for (; k < w.nbox; step()) {
         CLBM_PAIR(top);
         if (on_seam(b, xh)) continue;
         float *C = A + ly * rf;
-        gather_pair<ps, true, 0, true>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
-                                          pair_force<FIELD>(R, b, map, y, xh), bad, in_box(R, xh, y),
+        gather_pair<ps, true, 0, true, STORE>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                          pair_force<FIELD>(R, b, map, y, xh), keep_at(y, xh), bad, in_box(R, xh, y),
                                           in_box(R, xh + b.Wh, y));
       }
     } else {
@@ -756,8 +786,8 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
     if (GATHER) {
       if (on_seam(b, xh)) continue;
       float *C = A + ly * rf;
-      gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
-                                         pair_force<FIELD>(R, b, map, y, xh), bad);
+      gather_pair<ps, true, 0, false, STORE>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(xh),
+                                         pair_force<FIELD>(R, b, map, y, xh), keep_at(y, xh), bad);
     } else {
       local(ly, xh, std::integral_constant<bool, false>());
     }
@@ -776,16 +806,22 @@ __device__ __forceinline__ void band_step(const TemporalArgs &a, const Band &b, 
     const f2_t m = ahead;
     ahead = field_at(k + dk);
     const F32Force2 f = pair_force<FIELD>(R, m);
+    Keep kp{nullptr, 0};
+    if (STORE) {
+      const int i = list[k] + lane, ly = (int)__umulhi((unsigned)i, b.div_wh);
+      kp = keep_at(b.row0 + ly, i - ly * b.Wh - 1);
+    }
     if (GATHER)
-      gather_pair<ps, true, 0, false>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(0), f, bad);
+      gather_pair<ps, true, 0, false, STORE>(R, RowL{C}, RowL{C - rf}, RowL{C + rf}, cols_inner(0), f, kp, bad);
     else
-      local_pair<ps, false>(R, C, f, bad);
+      local_pair<ps, false, STORE>(R, C, f, kp, bad);
   }
 #undef CLBM_PAIR
   __syncthreads();
 }
 
-template <int THREADS, int MINB, int NP, bool FIELD>
+// STORE: the adjoint's forward, which keeps checkpoints (TemporalArgs::keep).
+template <int THREADS, int MINB, int NP, bool FIELD, bool STORE>
 __global__ void __launch_bounds__(THREADS, MINB) k_temporal_f32(TemporalArgs a) {
   // A[k][pair]: a warp's accesses to one population are consecutive 64-bit
   // words, in this CTA (no bank conflicts) and across a band edge (whole
@@ -853,14 +889,14 @@ __global__ void __launch_bounds__(THREADS, MINB) k_temporal_f32(TemporalArgs a) 
     const bool field = FIELD && t + 1 < R.field_steps;
     if ((t & 1) == 0) {
       if (field)
-        band_step<NW, true, FIELD>(a, b, plan, A, list, range, warp, lane, t, map, bad);
+        band_step<NW, true, FIELD, STORE>(a, b, plan, A, list, range, warp, lane, t, map, bad);
       else
-        band_step<NW, true, false>(a, b, plan, A, list, range, warp, lane, t, map, bad);
+        band_step<NW, true, false, STORE>(a, b, plan, A, list, range, warp, lane, t, map, bad);
     } else {
       if (field)
-        band_step<NW, false, FIELD>(a, b, plan, A, list, range, warp, lane, t, map, bad);
+        band_step<NW, false, FIELD, STORE>(a, b, plan, A, list, range, warp, lane, t, map, bad);
       else
-        band_step<NW, false, false>(a, b, plan, A, list, range, warp, lane, t, map, bad);
+        band_step<NW, false, false, STORE>(a, b, plan, A, list, range, warp, lane, t, map, bad);
     }
   }
   // the last step stores S_T
@@ -896,28 +932,29 @@ bool temporal_resident(int W, int rows) {
 
 struct TemporalVariant {
   int threads;
-  TemporalFn fn[2][2];  // [plane size: kPairs, kPairsHalf][field]
+  TemporalFn fn[2][3];  // [plane size: kPairs, kPairsHalf][uniform force, random field, checkpoints]
 };
 
-#define GENERIC(T, M, N) {k_temporal_f32<T, M, N, false>, k_temporal_f32<T, M, N, true>}
+#define GENERIC(T, M, N) \
+  {k_temporal_f32<T, M, N, false, false>, k_temporal_f32<T, M, N, true, false>, k_temporal_f32<T, M, N, false, true>}
 // (1024 and 512 threads take an SM's registers alone: no use for the half planes)
-static const TemporalVariant kTemporal[] = {{1024, {GENERIC(1024, 1, kPairs), {nullptr, nullptr}}},
-                                            {512, {GENERIC(512, 1, kPairs), {nullptr, nullptr}}},
+static const TemporalVariant kTemporal[] = {{1024, {GENERIC(1024, 1, kPairs), {nullptr, nullptr, nullptr}}},
+                                            {512, {GENERIC(512, 1, kPairs), {nullptr, nullptr, nullptr}}},
                                             {256, {GENERIC(256, 2, kPairs), GENERIC(256, 2, kPairsHalf)}}};
 #undef GENERIC
 
 int temporal_variant_count() { return (int)(sizeof(kTemporal) / sizeof(kTemporal[0])); }
 
-// the kernel of a variant for this band shape and its shared memory, or
+// the kernel (kind: an index of fn's) of a variant for this band shape and its shared memory, or
 // nullptr when it cannot run it
-static TemporalFn temporal_fn(int variant, int cs, int W, int rows_max, bool field, size_t *smem) {
+static TemporalFn temporal_fn(int variant, int cs, int W, int rows_max, int kind, size_t *smem) {
   if (variant < 0 || variant >= temporal_variant_count() || cs < 1 || cs > MAX_CLUSTER || rows_max < 1)
     return nullptr;
   if (temporal_smem(rows_max * W) > kSmemLimit) return nullptr;
   const TemporalVariant &v = kTemporal[variant];
-  const bool half = v.fn[1][field] && rows_max * ((W + 1) / 2) <= kPairsHalf;
+  const bool half = v.fn[1][kind] && rows_max * ((W + 1) / 2) <= kPairsHalf;
   *smem = std::min(pair_smem(half ? kPairsHalf : kPairs, rows_max, W), kSmemLimit);
-  return v.fn[half][field];
+  return v.fn[half][kind];
 }
 
 static cudaLaunchConfig_t temporal_config(int cs, int variant, int nclones, size_t smem, cudaStream_t s,
@@ -956,7 +993,8 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
     rows_max = std::max(rows_max, rows);
   }
   size_t smem = 0;
-  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field, &smem);
+  if (field && a.keep) return cudaErrorInvalidConfiguration;
+  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, a.keep ? 2 : field, &smem);
   if (!fn || !temporal_resident(W, rows_max) || a.steps < 1) return cudaErrorInvalidConfiguration;
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
