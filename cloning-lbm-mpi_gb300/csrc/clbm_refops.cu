@@ -139,20 +139,33 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
 }
 
 // generatePerturbedState.cpp:4-38 in two passes: fixed-order norm reduction,
-// then the element-wise update.
+// then the element-wise update.  A block takes 1024 values, four per thread
+// (per value the reduction costs the FP64 pipe, which bounds these kernels,
+// 2.5 operations instead of 10, next to the mix's 2 nsnap - 1).  mixed
+// (nullable): where the mix is kept for the update, which forms it again
+// otherwise.
+constexpr int PERTURB_BLOCK = 1024;
 struct Prefactors {
   double v[64];
 };
-__global__ void k_ref_perturb_norms(const double *fin, const double *snaps, int nsnap, int n,
-                                    const Prefactors pref, double *partials) {
+__device__ __forceinline__ double snapshot_mix(const double *snaps, int nsnap, int n, unsigned i,
+                                               const Prefactors &pref) {
+  double mix = DMUL(pref.v[0], snaps[i]);
+  for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
+  return mix;
+}
+__global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, const double *snaps, int nsnap, int n,
+                                                           const Prefactors pref, double *partials, double *mixed) {
   __shared__ double red[2][256 / 32];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double n0 = 0.0, n1 = 0.0;
-  if (i < n) {
-    double mix = DMUL(pref.v[0], snaps[i]);
-    for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
-    n0 = DMUL(fin[i], fin[i]);
-    n1 = DMUL(mix, mix);
+#pragma unroll
+  for (int j = 0; j < PERTURB_BLOCK / 256; j++) {
+    const unsigned i = blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x;
+    if (i >= (unsigned)n) break;
+    const double mix = snapshot_mix(snaps, nsnap, n, i, pref);
+    if (mixed) mixed[i] = mix;
+    n0 = DADD(n0, DMUL(fin[i], fin[i]));
+    n1 = DADD(n1, DMUL(mix, mix));
   }
   for (int o = 16; o > 0; o >>= 1) {
     n0 = DADD(n0, __shfl_down_sync(0xffffffffu, n0, o));
@@ -176,7 +189,7 @@ __global__ void k_ref_perturb_norms(const double *fin, const double *snaps, int 
 
 // The two norms summed over the blocks' partials, once, by one block in a fixed
 // order (thread t the partials t, t + 256, ..., then a tree; a single thread
-// spent 100 us on the 2323 pairs of a 257x257 state): out[0] = |f| / |mix| (the
+// spent 100 us on 2323 pairs): out[0] = |f| / |mix| (the
 // mix weight), out[1] = 1 / (1 + eps * sum(pref) * weight)
 // (generatePerturbedState.cpp:22-36).
 __global__ void __launch_bounds__(256) k_ref_perturb_finalize(const Prefactors pref, int nsnap, const double *partials,
@@ -210,12 +223,11 @@ __global__ void __launch_bounds__(256) k_ref_perturb_finalize(const Prefactors p
 
 // f <- (f + eps * mix * weight) / a with (weight, 1/a) from k_ref_perturb_finalize
 __global__ void k_ref_perturb_apply(double *fin, const double *snaps, int nsnap, int n,
-                                    const Prefactors pref, const double *wa, double eps) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+                                    const Prefactors pref, const double *wa, double eps, const double *mixed) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (unsigned)n) return;
   const double w = wa[0], inv = wa[1];
-  double mix = DMUL(pref.v[0], snaps[i]);
-  for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
+  const double mix = mixed ? mixed[i] : snapshot_mix(snaps, nsnap, n, i, pref);
   fin[i] = DMUL(DADD(fin[i], DMUL(DMUL(eps, mix), w)), inv);
 }
 
@@ -236,15 +248,15 @@ static int check_geom(const clbm_geom *g) {
 }
 
 // The three passes of a perturbation; wa: the weight pair, part: two norm
-// partials per 256 values (device).
+// partials per 1024 values, mixed (nullable): n values (device).
 static cudaError_t run_perturb(double *fin, const double *snaps, double eps, int nsnap, int n, const double *prefactors,
-                               double *wa, double *part, cudaStream_t st) {
+                               double *wa, double *part, double *mixed, cudaStream_t st) {
   Prefactors pref = {};
   for (int q = 0; q < nsnap; q++) pref.v[q] = prefactors[q];
-  const int nb = (n + 255) / 256;
-  k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, part);
+  const int nb = (n + PERTURB_BLOCK - 1) / PERTURB_BLOCK;
+  k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, part, mixed);
   k_ref_perturb_finalize<<<1, 256, 0, st>>>(pref, nsnap, part, nb, eps, wa);
-  k_ref_perturb_apply<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, wa, eps);
+  k_ref_perturb_apply<<<(n + 255) / 256, 256, 0, st>>>(fin, snaps, nsnap, n, pref, wa, eps, mixed);
   return cudaGetLastError();
 }
 
@@ -319,11 +331,11 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
                                         int n, const double *prefactors, void *stream) {
   if (!fin || !snaps || !prefactors || nsnap < 1 || nsnap > 64 || n < 1) return CLBM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  const int nb = (n + 255) / 256;
+  const size_t nb = ((size_t)n + PERTURB_BLOCK - 1) / PERTURB_BLOCK, head = 2 + 2 * nb;
   double *d_buf = nullptr;
-  cudaError_t e = call_alloc((void **)&d_buf, sizeof(double) * (2 + 2 * (size_t)nb), st);
+  cudaError_t e = call_alloc((void **)&d_buf, sizeof(double) * (head + n), st);
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
-  e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, d_buf, d_buf + 2, st);
+  e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, d_buf, d_buf + 2, d_buf + head, st);
   cudaFreeAsync(d_buf, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return clbm_status_from_cuda(e);
@@ -331,7 +343,7 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
 
 // ---------------------------------------------------------------------------
 // clbm_ref_perturbed_state_noalloc: the same kernels as
-// clbm_ref_perturbed_state, with their scratch (two norm partial sums per 256
+// clbm_ref_perturbed_state, with their scratch (two norm partial sums per 1024
 // values, the mix weight) in a fixed device array instead of a per-call
 // allocation.  It serves callers that must not allocate device memory at all:
 // code running under an allocator that already owns the whole device, or
@@ -339,10 +351,10 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
 // is not acceptable.
 namespace {
 constexpr int NOALLOC_MAX_N = 1 << 20;                     // values per state, 9*Dx*Dy
-constexpr int NOALLOC_MAX_BLOCKS = NOALLOC_MAX_N / 256;    // norm partials (pairs)
+constexpr int NOALLOC_MAX_BLOCKS = NOALLOC_MAX_N / PERTURB_BLOCK;  // norm partials (pairs)
 constexpr int NOALLOC_PREF = 64;                           // prefactors (nsnap <= 64)
 // Shared by every call on a device and kept until the process exits
-// (64 KB per device that loads the library): the mix weight and 1/a, then the
+// (16 KB per device that loads the library): the mix weight and 1/a, then the
 // norm partials.  Nothing in it has to start at zero: each call overwrites the
 // weight pair and every partial it reads.
 static __device__ __align__(256) double g_noalloc_scratch[2 + 2 * NOALLOC_MAX_BLOCKS];
@@ -388,7 +400,7 @@ extern "C" int clbm_ref_perturbed_state_noalloc(double *fin, const double *snaps
   double *scratch = nullptr;
   if (int s = noalloc_scratch(&scratch)) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, scratch, scratch + 2, st);
+  cudaError_t e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, scratch, scratch + 2, nullptr, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return clbm_status_from_cuda(e);
 }

@@ -165,7 +165,7 @@ int clbm_ref_perturbed_state(double *fin, const double *snaps, double eps,
  * allocation's implicit synchronisation is not allowed in their loop).  No
  * counterpart in the reference.  It allocates nothing: its scratch (the
  * per-block norm partials and the weight) lives in one fixed device array
- * of 64 KB that every GPU loading the library holds until exit, so n (the
+ * of 16 KB that every GPU loading the library holds until exit, so n (the
  * values of one state, 9*Dx*Dy) is limited to 1048576 and nsnap to 64; larger
  * sizes return CLBM_ERR_INVALID.  The first call on a device looks up the
  * array's device address, so make that first call before any stream capture
