@@ -95,14 +95,143 @@ __device__ __forceinline__ void velocity_ref64(const Moments64 &m, double half_b
   }
 }
 
+// Sums of doubles on the integer pipe.  An FP64 operation occupies an SM's FP64
+// pipe for 16 cycles per warp, while the integer pipes take eight warp
+// instructions in that time and are otherwise nearly idle here, so correctly
+// rounded additions of values of known size are quicker in 64-bit fixed point:
+// a double x, |x| < 1, as x 2^61 rounded to odd (fx: bit 0 also says that
+// lower bits were cut off, which happens below 2^-8), and fx_round rounds a sum
+// to nearest even where a double of its size would be rounded.  Round-to-odd
+// keeps the side and the ties of what was cut off through a sum with an even
+// value (1, a rounded value of 2^-8 or more, a double of 2^-7 or more) that is
+// itself 2^-7 or more, so that two bits or more are rounded away.
+typedef long long fx_t;
+constexpr fx_t FX_ONE = 1ll << 61;
+__device__ __forceinline__ fx_t fx_abs(double x) {  // of |x|
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  const int e = (int)(hi >> 20);
+  const unsigned long long m =
+      (((unsigned long long)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(x)) << 9;
+  const unsigned s = min((unsigned)(1023 - e), 63u);
+  const unsigned long long y = m >> s;
+  return (fx_t)(y | (unsigned long long)((y << s) != m));
+}
+__device__ __forceinline__ fx_t fx(double x) {
+  const fx_t y = fx_abs(x);
+  return __double2hiint(x) < 0 ? -y : y;
+}
+// of a positive x in [2^-9, 1): exact
+__device__ __forceinline__ fx_t fx_exact(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x);
+  const unsigned long long m =
+      (((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x)) << 9;
+  return (fx_t)(m >> (1023 - (int)(hi >> 20)));
+}
+// bits below the last place of a double of this value (0: none to round)
+__device__ __forceinline__ int fx_drop(fx_t v) {
+  int p;
+  asm("bfind.s32 %0, %1;" : "=r"(p) : "r"((int)(v >> 32)));
+  return max(p - 20, 0);
+}
+__device__ __forceinline__ fx_t fx_round(fx_t v) {
+  const int k = fx_drop(v);
+  const unsigned mask = (1u << k) - 1u;
+  v += (fx_t)((mask >> 1) + (((unsigned)v >> k) & mask & 1u));
+  return v & ~(fx_t)mask;
+}
+__device__ __forceinline__ double fx_double(fx_t r) {  // of a positive rounded value of 2^-8 or more
+  const int k = fx_drop(r);
+  return __longlong_as_double((r >> k) + ((fx_t)(1013 + k) << 52));
+}
+__device__ __forceinline__ double fx_signed_double(fx_t r) {  // of any rounded value
+  const double d = __ll2double_rn(r);  // exact
+  return r == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (61 << 20), __double2loint(d));
+}
+
 // 1 + 3 eu + 4.5 eu^2 + u2 for eu = e and eu = -e, u2 = -1.5 |u|^2
 // (streamCollCompute.cpp:32-34): the products of -e are those of e with the
 // sign changed, exactly, so an opposite pair of directions shares them.  t3 = 3 e,
 // h = 4.5 e.
 __device__ __forceinline__ void feq_pair_ref64(double e, double t3, double h, double u2, double &plus, double &minus) {
-  const double ee = DMUL(h, e);  // h = 4.5 e
+  const double ee = DMUL(h, e);
   plus = DADD(DADD(DADD(1.0, t3), ee), u2);
   minus = DADD(DADD(DSUB(1.0, t3), ee), u2);
+}
+// The same; where |e| < 0.3 (slow), in fixed point: every sum then lies in
+// [0.1, 2.4).  u = fx_abs(u2).
+__device__ __forceinline__ void feq_pair_ref64(bool slow, double e, double t3, double h, double u2, fx_t u,
+                                               double &plus, double &minus) {
+  if (slow) {
+    const fx_t t = fx(t3), q = fx_abs(DMUL(h, e));
+    plus = fx_double(fx_round(fx_round(fx_round(FX_ONE + t) + q) - u));
+    minus = fx_double(fx_round(fx_round(fx_round(FX_ONE - t) + q) - u));
+  } else {
+    feq_pair_ref64(e, t3, h, u2, plus, minus);
+  }
+}
+// |ux|, |uy| < 0x3fc30000: 0.1484, so that |ux +- uy| < 0.297 -- for every
+// thread of the warp that is here, as all such choices (a divided warp would
+// go both ways)
+__device__ __forceinline__ bool warp_all(bool v) { return __all_sync(__activemask(), v); }
+__device__ __forceinline__ bool slow_ref64(double ux, double uy) {
+  return warp_all(((unsigned)__double2hiint(ux) & 0x7fffffffu) < 0x3fc30000u &&
+                  ((unsigned)__double2hiint(uy) & 0x7fffffffu) < 0x3fc30000u);
+}
+
+// moments_ref64 in fixed point, for populations in [2^-9, 1), those of the
+// moving directions below 1/4 (every partial sum is then below 3).
+__device__ __forceinline__ bool mid_ref64(const double f[9]) {
+  unsigned lo = (unsigned)__double2hiint(f[0]), hi = 0;
+#pragma unroll
+  for (int k = 1; k < 9; k++) {
+    lo = min(lo, (unsigned)__double2hiint(f[k]));
+    hi = max(hi, (unsigned)__double2hiint(f[k]));
+  }
+  return warp_all(lo >= 0x3f600000u && hi < 0x3fd00000u && (unsigned)__double2hiint(f[0]) < 0x3ff00000u);
+}
+__device__ __forceinline__ Moments64 moments_fx(const double f[9]) {
+  fx_t v[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) v[k] = fx_exact(f[k]);
+  fx_t r = v[0];
+#pragma unroll
+  for (int k = 1; k < 9; k++) r = fx_round(r + v[k]);
+  fx_t x = fx_round(v[1] - v[3]), y = fx_round(v[2] - v[4]);
+  x = fx_round(fx_round(fx_round(fx_round(x + v[5]) - v[6]) - v[7]) + v[8]);
+  y = fx_round(fx_round(fx_round(fx_round(y + v[5]) + v[6]) - v[7]) - v[8]);
+  Moments64 m;
+  m.rho = fx_double(r);
+  m.jx = fx_signed_double(x);
+  m.jy = fx_signed_double(y);
+  return m;
+}
+// rho, jx, jy as moments_ref64 sums them, one for all uses of a node
+__device__ __forceinline__ Moments64 moments64(const double f[9]) {
+  return mid_ref64(f) ? moments_fx(f) : moments_ref64(f);
+}
+
+// out = (a + b) + c, the last two steps of the post-collision populations: in
+// fixed point where b is in [2^-7, 1) and both sums are at least 2^-7
+__device__ __forceinline__ void sum3_ref64(const double a[9], const double b[9], const double c[9], double out[9]) {
+  unsigned lo = 0xffffffffu, hi = 0, top = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    lo = min(lo, (unsigned)__double2hiint(b[k]));
+    hi = max(hi, (unsigned)__double2hiint(b[k]));
+    top = max(top, max((unsigned)__double2hiint(a[k]) & 0x7fffffffu, ((unsigned)__double2hiint(c[k]) & 0x7fffffffu) + 0x100000u));
+  }
+  if (warp_all(lo >= 0x3f800000u && hi < 0x3ff00000u && top < 0x3ff00000u)) {
+    fx_t least = FX_ONE;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const fx_t s = fx_round(fx(a[k]) + fx_exact(b[k])), v = fx_round(s + fx(c[k]));
+      least = min(least, min(s, v));
+      out[k] = fx_double(v);
+    }
+    if (warp_all(least >= (1ll << 54))) return;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++) out[k] = DADD(DADD(a[k], b[k]), c[k]);
 }
 
 // BGK collision with the Guo forcing term, velocity shifted by beta/(2 rho)
@@ -111,26 +240,31 @@ __device__ __forceinline__ void feq_pair_ref64(double e, double t3, double h, do
 // equilibrium and the drive 3 (cx - ux) + 9 cx eu direction by direction;
 // here what differs between directions in sign only is formed once: c_k.u of
 // opposite directions, 3 ux (the drive's of cx = 0), 3 (1 + ux) (minus the
-// drive's of cx = -1), the products w rho.  147 FP64 operations a node
-// (about 205 direction by direction, with three divisions): 2.72 -> 3.42 G
-// updates per second on 256 clones of 256x64.
-__device__ __forceinline__ void collide_ref64(const double f[9], double out[9], double beta,
+// drive's of cx = -1), the products w rho: 147 FP64 operations a node (about
+// 205 direction by direction, with three divisions), about 60 of which, the
+// sums, go to the integer pipe where the values are of ordinary size (moments64,
+// feq_pair_ref64, sum3_ref64).  256 clones of 256x64: 2.72 G updates per second
+// direction by direction, 3.52 by pairs (1192 us a step), 5.46 with the sums
+// in fixed point (768 us).  One node per thread: at one clone of 129x129 (four
+// warps an SM) the chain of dependent operations bounds it, 10.5 -> 10.1 us.
+// m = moments64(f).
+__device__ __forceinline__ void collide_ref64(const double f[9], const Moments64 &m, double out[9], double beta,
                                               const double wcb[9], double omega,
-                                              double om1, double *rho_o = nullptr,
-                                              double *ux_o = nullptr, double *uy_o = nullptr) {
-  const Moments64 m = moments_ref64(f);
+                                              double om1, double *ux_o = nullptr, double *uy_o = nullptr) {
   double ux, uy;
   velocity_ref64(m, DMUL(0.5, beta), ux, uy);
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
   const double es = DADD(ux, uy), ed = DSUB(ux, uy);  // c_5.u = -c_7.u, c_8.u = -c_6.u
   const double t3x = DMUL(3.0, ux);
+  const bool slow = slow_ref64(ux, uy);
+  const fx_t u = fx_abs(u2);
   double q[9];
   q[0] = DADD(1.0, u2);
   const double hx = DMUL(4.5, ux), hs = DMUL(4.5, es), hd = DMUL(4.5, ed);
-  feq_pair_ref64(ux, t3x, hx, u2, q[1], q[3]);
-  feq_pair_ref64(uy, DMUL(3.0, uy), DMUL(4.5, uy), u2, q[2], q[4]);
-  feq_pair_ref64(es, DMUL(3.0, es), hs, u2, q[5], q[7]);
-  feq_pair_ref64(ed, DMUL(3.0, ed), hd, u2, q[8], q[6]);
+  feq_pair_ref64(slow, ux, t3x, hx, u2, u, q[1], q[3]);
+  feq_pair_ref64(slow, uy, DMUL(3.0, uy), DMUL(4.5, uy), u2, u, q[2], q[4]);
+  feq_pair_ref64(slow, es, DMUL(3.0, es), hs, u2, u, q[5], q[7]);
+  feq_pair_ref64(slow, ed, DMUL(3.0, ed), hd, u2, u, q[8], q[6]);
   // 9 eu = 2 (4.5 eu), rounding included, so its sum with the rest of the
   // drive is one fused operation on an exact product
   const double right = DMUL(3.0, DSUB(1.0, ux)), left = DMUL(3.0, DADD(1.0, ux));
@@ -144,23 +278,23 @@ __device__ __forceinline__ void collide_ref64(const double f[9], double out[9], 
   drive[7] = DMUL(wcb[5], __fma_rn(2.0, hs, -left));
   drive[6] = DMUL(wcb[5], __fma_rn(2.0, hd, -left));
   const double r0 = DMUL(w_of(0), m.rho), r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
+  double old[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const double feq = DMUL(k == 0 ? r0 : (k <= 4 ? r1 : r5), q[k]);
-    out[k] = DADD(DADD(DMUL(f[k], om1), DMUL(feq, omega)), drive[k]);
+    old[k] = DMUL(f[k], om1);
+    q[k] = DMUL(DMUL(k == 0 ? r0 : (k <= 4 ? r1 : r5), q[k]), omega);
   }
-  if (rho_o) {
-    *rho_o = m.rho;
-    *ux_o = ux;
-    *uy_o = uy;
-  }
+  sum3_ref64(old, q, drive, out);
+  if (ux_o) *ux_o = ux;
+  if (uy_o) *uy_o = uy;
 }
 
-// Non-equilibrium second moments with the UNshifted velocity
+// Non-equilibrium second moments with the UNshifted velocity, m = moments64(f)
+// (FP64 sums: few lanes of a warp are at the square's side, and the fixed-point
+// chain is the longer one, 10.65 -> 10.2 us a step of one 129x129 clone)
 // (force.cpp:26-46): pi_xx = sum fneq cx cx, pi_xy = sum fneq cx cy.
-__device__ __forceinline__ void pi_ref64(const double f[9], double &rho, double &pxx,
+__device__ __forceinline__ void pi_ref64(const double f[9], const Moments64 &m, double &pxx,
                                          double &pxy) {
-  const Moments64 m = moments_ref64(f);
   const Divisor64 d = divisor64(m.rho);
   const bool fast = d.ok && mid_range64(m.jx) && mid_range64(m.jy);
   const double uy = fast ? div64(m.jy, d) : DDIV(m.jy, m.rho);
@@ -176,7 +310,6 @@ __device__ __forceinline__ void pi_ref64(const double f[9], double &rho, double 
 #pragma unroll
   for (int k = 1; k < 9; k++)
     if (cx_of(k) != 0) fneq[k] = DSUB(f[k], DMUL(k <= 4 ? r1 : r5, q[k]));
-  rho = m.rho;
   pxx = DADD(DADD(DADD(DADD(DADD(fneq[1], fneq[3]), fneq[5]), fneq[6]), fneq[7]), fneq[8]);
   pxy = DSUB(DADD(DSUB(fneq[5], fneq[6]), fneq[7]), fneq[8]);
 }
@@ -456,7 +589,7 @@ __device__ __forceinline__ typename std::conditional<F64, double, float>::type m
 template <bool F64>
 __device__ __forceinline__ void store_drag_terms(
     const RunDev &R, const typename std::conditional<F64, double, float>::type S[9], int x, int y,
-    int clone, typename std::conditional<F64, double, float>::type *T) {
+    int clone, typename std::conditional<F64, double, float>::type *T, const Moments64 *m64 = nullptr) {
   const int sy = R.ymax - R.ymin, sx = R.xmax - R.xmin;
   // (32-bit offsets: a step's terms of one run are under 2^32, since W >= 3
   // and its populations, 18 W H values a clone, fit the device)
@@ -472,8 +605,9 @@ __device__ __forceinline__ void store_drag_terms(
   }
   typename std::conditional<F64, double, float>::type west, east, north, south;
   if constexpr (F64) {
-    double rho, pxx, pxy;
-    pi_ref64(S, rho, pxx, pxy);
+    double pxx, pxy;
+    pi_ref64(S, *m64, pxx, pxy);
+    const double rho = m64->rho;
     const double third = 1. / 3.;
     const double c = R.cforce;
     west = DADD(DMUL(rho, third), DMUL(c, pxx));

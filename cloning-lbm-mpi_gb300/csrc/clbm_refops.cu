@@ -38,8 +38,9 @@ __global__ void k_ref_stream_collide(GeomDev g, double *fin, double *fout, doubl
   double f[9], post[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) f[k] = fin[aos(g, x, y, k)];
-  double r, vx, vy;
-  collide_ref64(f, post, beta, wcb, omega, om1, &r, &vx, &vy);
+  double vx, vy;
+  const Moments64 m = moments64(f);
+  collide_ref64(f, m, post, beta, wcb, omega, om1, &vx, &vy);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     fin[aos(g, x, y, k)] = post[k];
@@ -49,7 +50,7 @@ __global__ void k_ref_stream_collide(GeomDev g, double *fin, double *fout, doubl
   }
   if (ux) ux[t] = vx;
   if (uy) uy[t] = vy;
-  if (rho) rho[t] = r;
+  if (rho) rho[t] = m.rho;
 }
 
 // domain_noSlipWalls.cpp:6-22
@@ -119,8 +120,10 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
     double fn[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) fn[k] = f[aos(g, x, y, k)];
-    double rho, pxx, pxy;
-    pi_ref64(fn, rho, pxx, pxy);
+    const Moments64 m = moments64(fn);
+    const double rho = m.rho;
+    double pxx, pxy;
+    pi_ref64(fn, m, pxx, pxy);
     double v;
     if (side == 0) v = DADD(DMUL(rho, third), DMUL(c, pxx));
     else if (side == 1) v = DSUB(DMUL(-rho, third), DMUL(c, pxx));

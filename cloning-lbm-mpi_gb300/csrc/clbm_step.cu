@@ -73,19 +73,26 @@ __device__ __forceinline__ NodeLoc locate64(const RunDev *runs, int nruns) {
 // Consecutive steps are launched with programmatic stream serialisation: a
 // step's blocks may take their places while the previous step drains, find
 // their nodes, and wait here until it has completed and its writes are
-// visible.  (step_begin is the first thing that touches the populations.)
+// visible.  (The wait comes before anything that touches the populations.)
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void step_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  step_wait();
+  step_release();
 }
 
-// FP64 step, the reference's arithmetic.
+// FP64 step, the reference's arithmetic: bound by the FP64 and integer pipes
+// (collide_ref64).  The next step's blocks are let in after the collision, not
+// before it: let in early they take the room that a grid of about one wave
+// leaves (seven blocks an SM of ten at four clones of 129x129) and keep the rest
+// of this step's blocks waiting on a part of the SMs (26.8 us a step, 19.3 so;
+// 256 clones of 256x64: 767.6 both ways).
 template <bool LAST>
 __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
   using T = double;
   constexpr bool F64 = true;
   const NodeLoc L = locate64(a.runs, a.nruns);
-  step_begin();
+  step_wait();
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const long long plane = R.plane;
@@ -117,23 +124,25 @@ __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
     const T *p = ((mask >> k) & 1) ? src + opp_of(k) * plane + n : src + k * plane + srow + sx;
     S[k] = __ldg(p);
   }
+  const Moments64 m = moments64(S);
   if (in_box) {
     T *terms = (T *)a.terms + (long long)a.step * a.term_slab + R.term_base;
-    store_drag_terms<F64>(R, S, x, y, L.clone, terms);
+    store_drag_terms<F64>(R, S, x, y, L.clone, terms, &m);
   }
-  // (the density as moments_ref64 sums it: one sum for both uses; positive or
-  // +inf as an integer test of its bits, off the FP64 pipe)
-  const long long rho = __double_as_longlong(moments_ref64(S).rho);
-  if (!(rho > 0 && rho <= 0x7ff0000000000000ll)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
   if (LAST) {
+    step_release();
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = S[k];
   } else {
     T P[9];
-    collide_node<F64>(R, S, P, node_map(a.maps, R, L.clone, n, R.field_mode && a.step + 1 < R.field_steps));
+    collide_node<F64>(R, S, P, node_map(a.maps, R, L.clone, n, R.field_mode && a.step + 1 < R.field_steps), &m);
+    step_release();
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = P[k];
   }
+  // (positive or +inf as an integer test of its bits, off the FP64 pipe)
+  const long long bits = __double_as_longlong(m.rho);
+  if (!(bits > 0 && bits <= 0x7ff0000000000000ll)) atomicOr(a.err, (unsigned)ERR_BAD_DENSITY);
 }
 
 // ---------------------------------------------------------------------------
