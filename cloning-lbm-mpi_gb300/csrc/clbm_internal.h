@@ -10,6 +10,7 @@ namespace clbm {
 constexpr int MAX_RANKS = 64;   // virtual MPI ranks per run
 constexpr int MAX_SNAP = 64;    // perturbation snapshots per run
 constexpr int STEP_BLOCK = 256; // nodes per block of the step kernels
+constexpr int TILE64 = 64;      // nodes per block of the FP64 kernels
 
 // Per-run state that lives on the device between kernels (random-stream
 // positions, interval counter), so that captured CUDA graphs replay with the

@@ -26,11 +26,13 @@ namespace clbm {
 
 struct Moments64 {
   double rho, jx, jy;
+  bool mid;  // warp-uniform: every population of ordinary size (mid_ref64)
 };
 
 // rho, jx, jy summed in the reference's k order (streamCollCompute.cpp:21-27)
 __device__ __forceinline__ Moments64 moments_ref64(const double f[9]) {
   Moments64 m;
+  m.mid = false;
   double r = f[0];
 #pragma unroll
   for (int k = 1; k < 9; k++) r = DADD(r, f[k]);
@@ -95,26 +97,29 @@ __device__ __forceinline__ void velocity_ref64(const Moments64 &m, double half_b
   }
 }
 
-// Sums of doubles on the integer pipe.  An FP64 operation occupies an SM's FP64
-// pipe for 16 cycles per warp, while the integer pipes take eight warp
-// instructions in that time and are otherwise nearly idle here, so correctly
-// rounded additions of values of known size are quicker in 64-bit fixed point:
-// a double x, |x| < 1, as x 2^61 rounded to odd (fx: bit 0 also says that
-// lower bits were cut off, which happens below 2^-8), and fx_round rounds a sum
-// to nearest even where a double of its size would be rounded.  Round-to-odd
-// keeps the side and the ties of what was cut off through a sum with an even
-// value (1, a rounded value of 2^-8 or more, a double of 2^-7 or more) that is
-// itself 2^-7 or more, so that two bits or more are rounded away.
+// Doubles on the integer pipes.  An FP64 operation occupies an SM's FP64 pipe
+// for 16 cycles per warp, while the other pipes take a warp instruction in a
+// quarter of a cycle to two and are otherwise nearly idle here, so correctly
+// rounded sums and products of values of known size are quicker in 64-bit
+// fixed point: a double x as x 2^61 (fx_t), with what lies below that rounded
+// to odd (bit 0 also says that lower bits were cut off), and fx_round rounds a
+// sum or product to nearest even where a double of its size would be rounded.
+// Round-to-odd keeps the side and the ties of what was cut off through a sum
+// with an even value, and the rounding is right where it takes two bits or more
+// away: results of 2^-7 or more (2^54 before rounding).
 typedef long long fx_t;
+typedef unsigned long long fxu_t;
 constexpr fx_t FX_ONE = 1ll << 61;
-__device__ __forceinline__ fx_t fx_abs(double x) {  // of |x|
-  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
-  const int e = (int)(hi >> 20);
-  const unsigned long long m =
-      (((unsigned long long)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(x)) << 9;
-  const unsigned s = min((unsigned)(1023 - e), 63u);
-  const unsigned long long y = m >> s;
-  return (fx_t)(y | (unsigned long long)((y << s) != m));
+// significand of |x| with its leading one (none for a subnormal), as an integer
+__device__ __forceinline__ fxu_t fx_significand(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x);
+  return ((fxu_t)((hi & 0xfffffu) | (hi & 0x7ff00000u ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(x);
+}
+__device__ __forceinline__ fx_t fx_abs(double x) {  // of |x| < 1
+  const fxu_t m = fx_significand(x) << 9;
+  const unsigned s = min(1023u - (((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20), 63u);
+  const fxu_t y = m >> s;
+  return (fx_t)(y | (fxu_t)((y << s) != m));
 }
 __device__ __forceinline__ fx_t fx(double x) {
   const fx_t y = fx_abs(x);
@@ -123,62 +128,56 @@ __device__ __forceinline__ fx_t fx(double x) {
 // of a positive x in [2^-9, 1): exact
 __device__ __forceinline__ fx_t fx_exact(double x) {
   const unsigned hi = (unsigned)__double2hiint(x);
-  const unsigned long long m =
-      (((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x)) << 9;
+  const fxu_t m = (((fxu_t)((hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x)) << 9;
   return (fx_t)(m >> (1023 - (int)(hi >> 20)));
 }
-// bits below the last place of a double of this value (0: none to round)
-__device__ __forceinline__ int fx_drop(fx_t v) {
-  int p;
-  asm("bfind.s32 %0, %1;" : "=r"(p) : "r"((int)(v >> 32)));
-  return max(p - 20, 0);
+// Round to the 53 bits of a double (none to round below 2^-8).  A leading bit
+// at 62 - z takes 10 - z bits away: mask has them, half half a unit less one.
+struct FxPlace {
+  unsigned mask, half, shift;
+};
+__device__ __forceinline__ FxPlace fx_place(fx_t v) {
+  FxPlace p;
+  asm("{\n\t.reg .u32 z;\n\t"
+      "bfind.shiftamt.s32 z, %3;\n\t"
+      "shr.u32 %0, 2047, z;\n\t"
+      "shr.u32 %1, 1023, z;\n\t"
+      "sub.u32 %2, 11, z;\n\t}"
+      : "=r"(p.mask), "=r"(p.half), "=r"(p.shift)
+      : "r"((int)(v >> 32)));
+  return p;
 }
 __device__ __forceinline__ fx_t fx_round(fx_t v) {
-  const int k = fx_drop(v);
-  const unsigned mask = (1u << k) - 1u;
-  v += (fx_t)((mask >> 1) + (((unsigned)v >> k) & mask & 1u));
-  return v & ~(fx_t)mask;
+  const FxPlace p = fx_place(v);
+  v += (fx_t)(p.half + (((unsigned)v >> (p.shift & 31)) & p.mask & 1u));
+  return v & ~(fx_t)p.mask;
 }
-__device__ __forceinline__ double fx_double(fx_t r) {  // of a positive rounded value of 2^-8 or more
-  const int k = fx_drop(r);
-  return __longlong_as_double((r >> k) + ((fx_t)(1013 + k) << 52));
+// a b 2^-64, rounded to odd
+__device__ __forceinline__ fx_t fx_mul(fxu_t a, fxu_t b) {
+  const unsigned al = (unsigned)a, ah = (unsigned)(a >> 32), bl = (unsigned)b, bh = (unsigned)(b >> 32);
+  const fxu_t p = (fxu_t)al * bl;
+  const fxu_t q = (fxu_t)ah * bl + (p >> 32);
+  const fxu_t r = (fxu_t)al * bh + (unsigned)q;
+  const fxu_t h = (fxu_t)ah * bh + (q >> 32) + (r >> 32);
+  return (fx_t)(h | (fxu_t)(((unsigned)p | (unsigned)r) != 0u));
+}
+// a positive value of 2^-8 or more, rounded, as a double (a carry out of the
+// significand goes to the exponent)
+__device__ __forceinline__ double fx_double(fx_t v) {
+  const FxPlace p = fx_place(v);
+  v += (fx_t)(p.half + (((unsigned)v >> (p.shift & 31)) & p.mask & 1u));
+  v >>= p.shift & 31;
+  return __hiloint2double((int)(v >> 32) + (int)((1013 + p.shift) << 20), (int)v);
 }
 __device__ __forceinline__ double fx_signed_double(fx_t r) {  // of any rounded value
   const double d = __ll2double_rn(r);  // exact
   return r == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (61 << 20), __double2loint(d));
 }
-
-// 1 + 3 eu + 4.5 eu^2 + u2 for eu = e and eu = -e, u2 = -1.5 |u|^2
-// (streamCollCompute.cpp:32-34): the products of -e are those of e with the
-// sign changed, exactly, so an opposite pair of directions shares them.  t3 = 3 e,
-// h = 4.5 e.
-__device__ __forceinline__ void feq_pair_ref64(double e, double t3, double h, double u2, double &plus, double &minus) {
-  const double ee = DMUL(h, e);
-  plus = DADD(DADD(DADD(1.0, t3), ee), u2);
-  minus = DADD(DADD(DSUB(1.0, t3), ee), u2);
-}
-// The same; where |e| < 0.3 (slow), in fixed point: every sum then lies in
-// [0.1, 2.4).  u = fx_abs(u2).
-__device__ __forceinline__ void feq_pair_ref64(bool slow, double e, double t3, double h, double u2, fx_t u,
-                                               double &plus, double &minus) {
-  if (slow) {
-    const fx_t t = fx(t3), q = fx_abs(DMUL(h, e));
-    plus = fx_double(fx_round(fx_round(fx_round(FX_ONE + t) + q) - u));
-    minus = fx_double(fx_round(fx_round(fx_round(FX_ONE - t) + q) - u));
-  } else {
-    feq_pair_ref64(e, t3, h, u2, plus, minus);
-  }
-}
-// |ux|, |uy| < 0x3fc30000: 0.1484, so that |ux +- uy| < 0.297 -- for every
-// thread of the warp that is here, as all such choices (a divided warp would
-// go both ways)
+// A choice between fixed point and FP64 is made for every thread of the warp
+// that is here: a divided warp would go both ways.
 __device__ __forceinline__ bool warp_all(bool v) { return __all_sync(__activemask(), v); }
-__device__ __forceinline__ bool slow_ref64(double ux, double uy) {
-  return warp_all(((unsigned)__double2hiint(ux) & 0x7fffffffu) < 0x3fc30000u &&
-                  ((unsigned)__double2hiint(uy) & 0x7fffffffu) < 0x3fc30000u);
-}
 
-// moments_ref64 in fixed point, for populations in [2^-9, 1), those of the
+// moments_ref64 in fixed point, for populations in [2^-8, 1), those of the
 // moving directions below 1/4 (every partial sum is then below 3).
 __device__ __forceinline__ bool mid_ref64(const double f[9]) {
   unsigned lo = (unsigned)__double2hiint(f[0]), hi = 0;
@@ -187,12 +186,9 @@ __device__ __forceinline__ bool mid_ref64(const double f[9]) {
     lo = min(lo, (unsigned)__double2hiint(f[k]));
     hi = max(hi, (unsigned)__double2hiint(f[k]));
   }
-  return warp_all(lo >= 0x3f600000u && hi < 0x3fd00000u && (unsigned)__double2hiint(f[0]) < 0x3ff00000u);
+  return warp_all(lo >= 0x3f700000u && hi < 0x3fd00000u && (unsigned)__double2hiint(f[0]) < 0x3ff00000u);
 }
-__device__ __forceinline__ Moments64 moments_fx(const double f[9]) {
-  fx_t v[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) v[k] = fx_exact(f[k]);
+__device__ __forceinline__ Moments64 moments_fx(const fx_t v[9]) {
   fx_t r = v[0];
 #pragma unroll
   for (int k = 1; k < 9; k++) r = fx_round(r + v[k]);
@@ -203,35 +199,87 @@ __device__ __forceinline__ Moments64 moments_fx(const double f[9]) {
   m.rho = fx_double(r);
   m.jx = fx_signed_double(x);
   m.jy = fx_signed_double(y);
+  m.mid = true;
   return m;
 }
+// A thread's node on its way through the collision, in shared memory: in
+// registers it takes 90 and more (ten blocks of 64 threads an SM), and rows
+// allow loops over the directions, whose straight-line code, 50 KB, was
+// waiting for instructions.  f: fixed point where the moments are (mid), else
+// the bits of the double.
+template <int BLOCK>
+struct Node64 {
+  fx_t f[9][BLOCK], q[9][BLOCK];
+  double drive[9][BLOCK];
+};
+__device__ __forceinline__ void column_fence() { asm volatile("" ::: "memory"); }  // no value kept in a register
+template <int BLOCK>
+__device__ __forceinline__ double node_f(const Node64<BLOCK> &s, bool mid, int k) {
+  const fx_t v = s.f[k][threadIdx.x];
+  return mid ? fx_double(v) : __longlong_as_double(v);
+}
 // rho, jx, jy as moments_ref64 sums them, one for all uses of a node
-__device__ __forceinline__ Moments64 moments64(const double f[9]) {
-  return mid_ref64(f) ? moments_fx(f) : moments_ref64(f);
+template <int BLOCK>
+__device__ __forceinline__ Moments64 moments64(Node64<BLOCK> &s, const double f[9]) {
+  Moments64 m;
+  if (mid_ref64(f)) {
+    fx_t v[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) s.f[k][threadIdx.x] = v[k] = fx_exact(f[k]);
+    m = moments_fx(v);
+  } else {
+    m = moments_ref64(f);
+#pragma unroll
+    for (int k = 0; k < 9; k++) s.f[k][threadIdx.x] = __double_as_longlong(f[k]);
+  }
+  column_fence();
+  return m;
 }
 
-// out = (a + b) + c, the last two steps of the post-collision populations: in
-// fixed point where b is in [2^-7, 1) and both sums are at least 2^-7
-__device__ __forceinline__ void sum3_ref64(const double a[9], const double b[9], const double c[9], double out[9]) {
-  unsigned lo = 0xffffffffu, hi = 0, top = 0;
-#pragma unroll
+// 1 + 3 eu + 4.5 eu^2 + u2 for eu = e and eu = -e, u2 = -1.5 |u|^2
+// (streamCollCompute.cpp:32-34): the products of -e are those of e with the
+// sign changed, exactly, so an opposite pair of directions shares them.  t3 = 3 e,
+// ee = 4.5 e e.
+__device__ __forceinline__ void feq_pair_ref64(double t3, double ee, double u2, double &plus, double &minus) {
+  plus = DADD(DADD(DADD(1.0, t3), ee), u2);
+  minus = DADD(DADD(DSUB(1.0, t3), ee), u2);
+}
+// In fixed point where |e| < 0.3 (every sum then lies in [0.1, 2.4)); u = -u2.
+__device__ __forceinline__ void feq_pair_fx(double t3, double ee, fx_t u, fx_t &plus, fx_t &minus) {
+  const fx_t t = fx(t3), q = fx_abs(ee);
+  plus = fx_round(fx_round(fx_round(FX_ONE + t) + q) - u);
+  minus = fx_round(fx_round(fx_round(FX_ONE - t) + q) - u);
+}
+
+// The post-collision populations (f om1 + (w rho) q omega) + drive of a node in
+// fixed point, q = 1 + 3 eu + 4.5 eu^2 + u2 by directions; false where a value
+// is not of the size that needs.  r0 = w[0] rho in [1/4, 1/2): the other
+// products w rho are a quarter and a sixteenth of it, so all have its
+// significand, and all quotients of scale go to the place of omega's.
+template <int BLOCK>
+__device__ __forceinline__ bool relax_fx(Node64<BLOCK> &s64, double r0, double omega, double om1) {
+  const int t = threadIdx.x;
+  const int e1 = (int)(((unsigned)__double2hiint(om1) & 0x7fffffffu) >> 20);  // om1 = 2^(e1 - 1023) M1 2^-63
+  const fxu_t M1 = fx_significand(om1) << 11, R = fx_significand(r0) << 11;
+  const unsigned s1 = om1 == 0.0 ? 2 : 1024 - e1, low1 = (1u << s1) - 1u;
+  const fx_t sign1 = __double2hiint(om1) < 0 ? -1 : 0;
+  const fxu_t Om = fx_significand(omega) << ((__double2hiint(omega) >> 20) - 1016);  // omega 2^59
+  int least = 0x7fffffff;
+#pragma unroll 3
   for (int k = 0; k < 9; k++) {
-    lo = min(lo, (unsigned)__double2hiint(b[k]));
-    hi = max(hi, (unsigned)__double2hiint(b[k]));
-    top = max(top, max((unsigned)__double2hiint(a[k]) & 0x7fffffffu, ((unsigned)__double2hiint(c[k]) & 0x7fffffffu) + 0x100000u));
+    // q r0 2^62, rounded; its product with omega at 2^61
+    const fx_t b = fx_mul((fxu_t)fx_round(fx_mul((fxu_t)s64.q[k][t], R)), k == 0 ? Om << 4 : (k <= 4 ? Om << 2 : Om));
+    // |f om1| at 2^(1085 - e1), rounded, then at 2^61
+    const fx_t a = fx_round(fx_mul((fxu_t)s64.f[k][t] << 2, M1));
+    const fx_t a1 = (fx_t)((fxu_t)a >> s1) | (fx_t)(((unsigned)a & low1) != 0u);
+    const fx_t s = fx_round(b) + (a1 ^ sign1) + (sign1 & 1);
+    const double d = s64.drive[k][t];
+    const fx_t sign = __double2hiint(d) >> 31;
+    const fx_t v = fx_round(s) + (fx_abs(d) ^ sign) + (sign & 1);
+    least = min(least, min((int)(b >> 32), min((int)(s >> 32), (int)(v >> 32))));
+    s64.q[k][t] = __double_as_longlong(fx_double(v));
   }
-  if (warp_all(lo >= 0x3f800000u && hi < 0x3ff00000u && top < 0x3ff00000u)) {
-    fx_t least = FX_ONE;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const fx_t s = fx_round(fx(a[k]) + fx_exact(b[k])), v = fx_round(s + fx(c[k]));
-      least = min(least, min(s, v));
-      out[k] = fx_double(v);
-    }
-    if (warp_all(least >= (1ll << 54))) return;
-  }
-#pragma unroll
-  for (int k = 0; k < 9; k++) out[k] = DADD(DADD(a[k], b[k]), c[k]);
+  return least >= 1 << 22;
 }
 
 // BGK collision with the Guo forcing term, velocity shifted by beta/(2 rho)
@@ -241,14 +289,19 @@ __device__ __forceinline__ void sum3_ref64(const double a[9], const double b[9],
 // here what differs between directions in sign only is formed once: c_k.u of
 // opposite directions, 3 ux (the drive's of cx = 0), 3 (1 + ux) (minus the
 // drive's of cx = -1), the products w rho: 147 FP64 operations a node (about
-// 205 direction by direction, with three divisions), about 60 of which, the
-// sums, go to the integer pipe where the values are of ordinary size (moments64,
-// feq_pair_ref64, sum3_ref64).  256 clones of 256x64: 2.72 G updates per second
-// direction by direction, 3.52 by pairs (1192 us a step), 5.46 with the sums
-// in fixed point (768 us).  One node per thread: at one clone of 129x129 (four
-// warps an SM) the chain of dependent operations bounds it, 10.5 -> 10.1 us.
-// m = moments64(f).
-__device__ __forceinline__ void collide_ref64(const double f[9], const Moments64 &m, double out[9], double beta,
+// 205 direction by direction, with three divisions).  Where the values are of
+// ordinary size the sums and the products of the relaxation, 81 of them, go to
+// the integer pipes (moments64, feq_pair_fx, relax_fx), elsewhere, a warp at a
+// time, they stay FP64.  256 clones of 256x64, us a step: 1540 direction by
+// direction, 1192 by pairs, 768 with the sums in fixed point, 731 with the
+// products too, 545 with the node in shared memory and loops over directions
+// (3 unrolled; 615 unrolled in full, which waits for instructions), 534 with
+// fx_place; the FP64 pipe is then busy 78% of the time and the integer ALU 61%.
+// At one clone of 129x129 (four warps an SM) the chain of dependent operations
+// bounds it, 10.3 us a step whatever the pipe.
+// s and m: the node and moments64 of it.
+template <int BLOCK>
+__device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 &m, double out[9], double beta,
                                               const double wcb[9], double omega,
                                               double om1, double *ux_o = nullptr, double *uy_o = nullptr) {
   double ux, uy;
@@ -256,43 +309,78 @@ __device__ __forceinline__ void collide_ref64(const double f[9], const Moments64
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
   const double es = DADD(ux, uy), ed = DSUB(ux, uy);  // c_5.u = -c_7.u, c_8.u = -c_6.u
   const double t3x = DMUL(3.0, ux);
-  const bool slow = slow_ref64(ux, uy);
-  const fx_t u = fx_abs(u2);
-  double q[9];
-  q[0] = DADD(1.0, u2);
+  const double t3y = DMUL(3.0, uy), t3s = DMUL(3.0, es), t3d = DMUL(3.0, ed);
   const double hx = DMUL(4.5, ux), hs = DMUL(4.5, es), hd = DMUL(4.5, ed);
-  feq_pair_ref64(slow, ux, t3x, hx, u2, u, q[1], q[3]);
-  feq_pair_ref64(slow, uy, DMUL(3.0, uy), DMUL(4.5, uy), u2, u, q[2], q[4]);
-  feq_pair_ref64(slow, es, DMUL(3.0, es), hs, u2, u, q[5], q[7]);
-  feq_pair_ref64(slow, ed, DMUL(3.0, ed), hd, u2, u, q[8], q[6]);
+  const double eex = DMUL(hx, ux), eey = DMUL(DMUL(4.5, uy), uy), ees = DMUL(hs, es), eed = DMUL(hd, ed);
   // 9 eu = 2 (4.5 eu), rounding included, so its sum with the rest of the
   // drive is one fused operation on an exact product
   const double right = DMUL(3.0, DSUB(1.0, ux)), left = DMUL(3.0, DADD(1.0, ux));
-  double drive[9];
-  drive[0] = DMUL(wcb[0], -t3x);
-  drive[2] = drive[4] = DMUL(wcb[1], -t3x);
-  drive[1] = DMUL(wcb[1], __fma_rn(2.0, hx, right));
-  drive[5] = DMUL(wcb[5], __fma_rn(2.0, hs, right));
-  drive[8] = DMUL(wcb[5], __fma_rn(2.0, hd, right));
-  drive[3] = DMUL(wcb[1], __fma_rn(2.0, hx, -left));
-  drive[7] = DMUL(wcb[5], __fma_rn(2.0, hs, -left));
-  drive[6] = DMUL(wcb[5], __fma_rn(2.0, hd, -left));
-  const double r0 = DMUL(w_of(0), m.rho), r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
-  double old[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    old[k] = DMUL(f[k], om1);
-    q[k] = DMUL(DMUL(k == 0 ? r0 : (k <= 4 ? r1 : r5), q[k]), omega);
-  }
-  sum3_ref64(old, q, drive, out);
+  double (*drive)[BLOCK] = s.drive;
+  const int t = threadIdx.x;
+  drive[0][t] = DMUL(wcb[0], -t3x);
+  drive[2][t] = drive[4][t] = DMUL(wcb[1], -t3x);
+  drive[1][t] = DMUL(wcb[1], __fma_rn(2.0, hx, right));
+  drive[5][t] = DMUL(wcb[5], __fma_rn(2.0, hs, right));
+  drive[8][t] = DMUL(wcb[5], __fma_rn(2.0, hd, right));
+  drive[3][t] = DMUL(wcb[1], __fma_rn(2.0, hx, -left));
+  drive[7][t] = DMUL(wcb[5], __fma_rn(2.0, hs, -left));
+  drive[6][t] = DMUL(wcb[5], __fma_rn(2.0, hd, -left));
+  const double r0 = DMUL(w_of(0), m.rho);
   if (ux_o) *ux_o = ux;
   if (uy_o) *uy_o = uy;
+  if (m.mid) {
+    // |u| below 0.1484, r0 in [1/4, 1/2), drives below 1/2, omega in [1/16, 2),
+    // |om1| in [2^-29, 1) or zero
+    unsigned top = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) top = max(top, (unsigned)__double2hiint(drive[k][t]) & 0x7fffffffu);
+    const unsigned o1 = (unsigned)__double2hiint(om1) & 0x7fffffffu;
+    if (warp_all(max((unsigned)__double2hiint(ux) & 0x7fffffffu, (unsigned)__double2hiint(uy) & 0x7fffffffu) < 0x3fc30000u &&
+                 (unsigned)__double2hiint(r0) - 0x3fd00000u < 0x100000u && top < 0x3fe00000u &&
+                 (unsigned)__double2hiint(omega) - 0x3fb00000u < 0x500000u &&
+                 (o1 - 0x3e200000u < 0x1d00000u || om1 == 0.0))) {
+      fx_t (*q)[BLOCK] = s.q;
+      const fx_t u = fx_abs(u2);
+      q[0][t] = fx_round(FX_ONE - u);
+      q[1][t] = __double_as_longlong(t3x), q[3][t] = __double_as_longlong(eex);
+      q[2][t] = __double_as_longlong(t3y), q[4][t] = __double_as_longlong(eey);
+      q[5][t] = __double_as_longlong(t3s), q[7][t] = __double_as_longlong(ees);
+      q[8][t] = __double_as_longlong(t3d), q[6][t] = __double_as_longlong(eed);
+      column_fence();
+#pragma unroll 1
+      for (int j = 0; j < 4; j++) {
+        const int kp = j < 2 ? j + 1 : 3 * j - 1, km = j < 2 ? j + 3 : 9 - j;
+        fx_t plus, minus;
+        feq_pair_fx(__longlong_as_double(q[kp][t]), __longlong_as_double(q[km][t]), u, plus, minus);
+        q[kp][t] = plus;
+        q[km][t] = minus;
+      }
+      if (warp_all(relax_fx(s, r0, omega, om1))) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) out[k] = __longlong_as_double(q[k][t]);
+        return;
+      }
+    }
+  }
+  double q[9];
+  q[0] = DADD(1.0, u2);
+  feq_pair_ref64(t3x, eex, u2, q[1], q[3]);
+  feq_pair_ref64(t3y, eey, u2, q[2], q[4]);
+  feq_pair_ref64(t3s, ees, u2, q[5], q[7]);
+  feq_pair_ref64(t3d, eed, u2, q[8], q[6]);
+  const double r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const double feq = DMUL(k == 0 ? r0 : (k <= 4 ? r1 : r5), q[k]);
+    out[k] = DADD(DADD(DMUL(node_f(s, m.mid, k), om1), DMUL(feq, omega)), drive[k][t]);
+  }
 }
 
-// Non-equilibrium second moments with the UNshifted velocity, m = moments64(f)
-// (FP64 sums: few lanes of a warp are at the square's side, and the fixed-point
-// chain is the longer one, 10.65 -> 10.2 us a step of one 129x129 clone)
-// (force.cpp:26-46): pi_xx = sum fneq cx cx, pi_xy = sum fneq cx cy.
+// Non-equilibrium second moments with the UNshifted velocity
+// (force.cpp:26-46): pi_xx = sum fneq cx cx, pi_xy = sum fneq cx cy, m the
+// moments of f.  (FP64 sums: few lanes of a warp are at the square's side, and the
+// fixed-point chain is the longer one, 10.65 against 10.2 us a step of one
+// 129x129 clone.)
 __device__ __forceinline__ void pi_ref64(const double f[9], const Moments64 &m, double &pxx,
                                          double &pxy) {
   const Divisor64 d = divisor64(m.rho);
@@ -302,9 +390,9 @@ __device__ __forceinline__ void pi_ref64(const double f[9], const Moments64 &m, 
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
   const double es = DADD(ux, uy), ed = DSUB(ux, uy);
   double q[9];
-  feq_pair_ref64(ux, DMUL(3.0, ux), DMUL(4.5, ux), u2, q[1], q[3]);
-  feq_pair_ref64(es, DMUL(3.0, es), DMUL(4.5, es), u2, q[5], q[7]);
-  feq_pair_ref64(ed, DMUL(3.0, ed), DMUL(4.5, ed), u2, q[8], q[6]);
+  feq_pair_ref64(DMUL(3.0, ux), DMUL(DMUL(4.5, ux), ux), u2, q[1], q[3]);
+  feq_pair_ref64(DMUL(3.0, es), DMUL(DMUL(4.5, es), es), u2, q[5], q[7]);
+  feq_pair_ref64(DMUL(3.0, ed), DMUL(DMUL(4.5, ed), ed), u2, q[8], q[6]);
   const double r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
   double fneq[9];
 #pragma unroll

@@ -21,7 +21,7 @@ __device__ __forceinline__ long long aos(const GeomDev &g, int x, int y, int k) 
 
 // streamCollCompute.cpp:7-93: collide in place into fin, push to the periodic
 // neighbour in fout, macroscopic fields of the pre-collision state.
-__global__ void k_ref_stream_collide(GeomDev g, double *fin, double *fout, double *rho,
+__global__ void __launch_bounds__(TILE64) k_ref_stream_collide(GeomDev g, double *fin, double *fout, double *rho,
                                      double *ux, double *uy, double beta0, const double *map,
                                      double tau, double eps) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;  // t = y + ny*x
@@ -39,8 +39,9 @@ __global__ void k_ref_stream_collide(GeomDev g, double *fin, double *fout, doubl
 #pragma unroll
   for (int k = 0; k < 9; k++) f[k] = fin[aos(g, x, y, k)];
   double vx, vy;
-  const Moments64 m = moments64(f);
-  collide_ref64(f, m, post, beta, wcb, omega, om1, &vx, &vy);
+  __shared__ Node64<TILE64> node;
+  const Moments64 m = moments64(node, f);
+  collide_ref64(node, m, post, beta, wcb, omega, om1, &vx, &vy);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     fin[aos(g, x, y, k)] = post[k];
@@ -120,7 +121,7 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
     double fn[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) fn[k] = f[aos(g, x, y, k)];
-    const Moments64 m = moments64(fn);
+    const Moments64 m = moments_ref64(fn);
     const double rho = m.rho;
     double pxx, pxy;
     pi_ref64(fn, m, pxx, pxy);
@@ -273,7 +274,7 @@ extern "C" int clbm_ref_stream_collide(const clbm_geom *g, double *fin, double *
   if (int s = check_geom(g)) return s;
   if (!fin || !fout) return CLBM_ERR_INVALID;
   const int n = g->nx * g->ny;
-  k_ref_stream_collide<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
+  k_ref_stream_collide<<<(n + TILE64 - 1) / TILE64, TILE64, 0, (cudaStream_t)stream>>>(
       to_dev(g), fin, fout, rho, ux, uy, beta, nullptr, tau, 0.0);
   return clbm_status_from_cuda(cudaGetLastError());
 }
@@ -285,7 +286,7 @@ extern "C" int clbm_ref_stream_collide_spatial(const clbm_geom *g, double *fin, 
   if (int s = check_geom(g)) return s;
   if (!fin || !fout || !map) return CLBM_ERR_INVALID;
   const int n = g->nx * g->ny;
-  k_ref_stream_collide<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
+  k_ref_stream_collide<<<(n + TILE64 - 1) / TILE64, TILE64, 0, (cudaStream_t)stream>>>(
       to_dev(g), fin, fout, rho, ux, uy, beta0, map, tau, eps);
   return clbm_status_from_cuda(cudaGetLastError());
 }

@@ -16,20 +16,27 @@ using pop_t = typename std::conditional<F64, double, float>::type;
 
 // map: the node's random-field value when the collision is under the
 // spatial force, beta(x,y) = (1 + eps*map)*beta0 (streamCollCompute.cpp:63)
+template <int BLOCK>
+__device__ __forceinline__ void collide_node64(const RunDev &R, Node64<BLOCK> &node, const Moments64 &m, double P[9],
+                                               const float *map) {
+  if (map) {
+    const double beta = DMUL(DADD(1.0, DMUL(R.field_eps, (double)*map)), R.beta);
+    double wcb[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) wcb[k] = DMUL(DMUL(w_of(k), R.cforce), beta);
+    collide_ref64(node, m, P, beta, wcb, R.omega, R.om1);
+  } else {
+    collide_ref64(node, m, P, R.beta, R.wcb, R.omega, R.om1);
+  }
+}
+
 template <bool F64>
 __device__ __forceinline__ void collide_node(const RunDev &R, const pop_t<F64> S[9], pop_t<F64> P[9],
-                                             const float *map = nullptr, const Moments64 *m64 = nullptr) {
+                                             const float *map = nullptr) {
   if constexpr (F64) {
-    const Moments64 m = m64 ? *m64 : moments64(S);
-    if (map) {
-      const double beta = DMUL(DADD(1.0, DMUL(R.field_eps, (double)*map)), R.beta);
-      double wcb[9];
-#pragma unroll
-      for (int k = 0; k < 9; k++) wcb[k] = DMUL(DMUL(w_of(k), R.cforce), beta);
-      collide_ref64(S, m, P, beta, wcb, R.omega, R.om1);
-    } else {
-      collide_ref64(S, m, P, R.beta, R.wcb, R.omega, R.om1);
-    }
+    __shared__ Node64<TILE64> node;
+    const Moments64 m = moments64(node, S);
+    collide_node64(R, node, m, P, map);
   } else {
     collide_f32_run(R, S, P, map, R.f_field_eps);
   }

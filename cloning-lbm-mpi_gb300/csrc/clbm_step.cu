@@ -52,7 +52,6 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
 // plane / 64 of them.  The FP64 pipe bounds these kernels, and the SM with the
 // most nodes sets the time: tiles of 256 gave 16 clones of 200x50 4.1 of them
 // per SM (5 on some), and one state of 129x129 only 65 busy SMs.
-constexpr int TILE64 = 64;
 __device__ __forceinline__ NodeLoc locate64(const RunDev *runs, int nruns) {
   NodeLoc L;
   const long long first = 9LL * TILE64 * blockIdx.x;  // pop_base the tile would have
@@ -124,10 +123,14 @@ __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
     const T *p = ((mask >> k) & 1) ? src + opp_of(k) * plane + n : src + k * plane + srow + sx;
     S[k] = __ldg(p);
   }
-  const Moments64 m = moments64(S);
+  __shared__ Node64<TILE64> node;
+  const Moments64 m = LAST ? moments_ref64(S) : moments64(node, S);
   if (in_box) {
     T *terms = (T *)a.terms + (long long)a.step * a.term_slab + R.term_base;
-    store_drag_terms<F64>(R, S, x, y, L.clone, terms, &m);
+    T D[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) D[k] = LAST ? S[k] : node_f(node, m.mid, k);
+    store_drag_terms<F64>(R, D, x, y, L.clone, terms, &m);
   }
   if (LAST) {
     step_release();
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
     for (int k = 0; k < 9; k++) dst[k * plane + n] = S[k];
   } else {
     T P[9];
-    collide_node<F64>(R, S, P, node_map(a.maps, R, L.clone, n, R.field_mode && a.step + 1 < R.field_steps), &m);
+    collide_node64(R, node, m, P, node_map(a.maps, R, L.clone, n, R.field_mode && a.step + 1 < R.field_steps));
     step_release();
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = P[k];
