@@ -52,12 +52,14 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
 // plane / 64 of them.  The FP64 pipe bounds these kernels, and the SM with the
 // most nodes sets the time: tiles of 256 gave 16 clones of 200x50 4.1 of them
 // per SM (5 on some), and one state of 129x129 only 65 busy SMs.
-__device__ __forceinline__ NodeLoc locate64(const RunDev *runs, int nruns) {
-  NodeLoc L;
+__device__ __forceinline__ int run64(const RunDev *runs, int nruns) {
   const long long first = 9LL * TILE64 * blockIdx.x;  // pop_base the tile would have
   int r = 0;
   while (r + 1 < nruns && first >= runs[r + 1].pop_base) r++;
-  const RunDev &R = runs[r];
+  return r;
+}
+__device__ __forceinline__ NodeLoc locate64(const RunDev &R, int r) {
+  NodeLoc L;
   const unsigned per = (unsigned)(R.plane / TILE64);
   const unsigned local = blockIdx.x - (unsigned)(R.pop_base / (9 * TILE64));
   L.run = r;
@@ -85,15 +87,29 @@ __device__ __forceinline__ void step_begin() {
 // before it: let in early they take the room that a grid of about one wave
 // leaves (seven blocks an SM of ten at four clones of 129x129) and keep the rest
 // of this step's blocks waiting on a part of the SMs (26.8 us a step, 19.3 so;
-// 256 clones of 256x64: 767.6 both ways).
-template <bool LAST>
-__global__ void __launch_bounds__(TILE64) k_step(StepArgs a) {
+// 256 clones of 256x64: 767.6 both ways).  A context's only run comes with the
+// launch: constants of the table of runs are read from L2 on every SM and step,
+// part of the chain that a small grid waits for (one clone of 129x129 10.3 us a
+// step from the table, 9.6 so; 256 clones of 256x64 534 and 532).
+struct StepArgsOne : StepArgs {
+  RunDev rd;
+};
+template <bool LAST, class Args>
+__global__ void __launch_bounds__(TILE64) k_step(const __grid_constant__ Args a) {
   using T = double;
-  constexpr bool F64 = true;
-  const NodeLoc L = locate64(a.runs, a.nruns);
+  constexpr bool F64 = true, ONE = std::is_same<Args, StepArgsOne>::value;
+  const RunDev *run;
+  int r = 0;
+  if constexpr (ONE) {
+    run = &a.rd;
+  } else {
+    r = run64(a.runs, a.nruns);
+    run = a.runs + r;
+  }
+  const RunDev &R = *run;
+  const NodeLoc L = locate64(R, r);
   step_wait();
   if (!L.valid) return;
-  const RunDev &R = a.runs[L.run];
   const long long plane = R.plane;
   const long long cbase = R.pop_base + (long long)L.clone * 9 * plane;
   const T *__restrict__ src = (const T *)a.src + cbase;
@@ -269,8 +285,14 @@ cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void (*fn)(StepArgs) = f64 ? (last ? k_step<true> : k_step<false>) : (last ? v.last : v.body);
-  return cudaLaunchKernelEx(&cfg, fn, a);
+  if (f64 && a.one) {
+    StepArgsOne o;
+    static_cast<StepArgs &>(o) = a;
+    o.rd = *a.one;
+    return cudaLaunchKernelEx(&cfg, last ? k_step<true, StepArgsOne> : k_step<false, StepArgsOne>, o);
+  }
+  if (f64) return cudaLaunchKernelEx(&cfg, last ? k_step<true, StepArgs> : k_step<false, StepArgs>, a);
+  return cudaLaunchKernelEx(&cfg, last ? v.last : v.body, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -281,7 +303,8 @@ cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, 
 template <bool F64>
 __global__ void __launch_bounds__(F64 ? TILE64 : STEP_BLOCK) k_reseed(ReseedArgs a) {
   using T = pop_t<F64>;
-  const NodeLoc L = F64 ? locate64(a.runs, a.nruns) : locate(a.runs, a.nruns);
+  const int r64 = F64 ? run64(a.runs, a.nruns) : 0;
+  const NodeLoc L = F64 ? locate64(a.runs[r64], r64) : locate(a.runs, a.nruns);
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const int x = L.x, y = L.y, n = L.n;
