@@ -774,6 +774,12 @@ static cudaError_t ensure_side(clbm_ctx *c, int n) {
   return cudaSuccess;
 }
 
+// blocks that store the drag terms in an FP64 step
+static int drag_tiles64(const clbm_ctx *c) {
+  int n = 0;
+  for (const RunDev &R : c->runs_h) n += R.nclones * ((R.nterms + TILE64 - 1) / TILE64);
+  return n;
+}
 static const RunDev *only_run(const clbm_ctx *c) { return c->nruns == 1 ? &c->runs_h[0] : nullptr; }
 
 // The cluster-resident kernel's arguments for run r of a plan.
@@ -834,7 +840,7 @@ static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int
     int cur = src;
     for (int t = 0; t < steps; t++) {
       StepArgs a{p.table, p.nstream, t, c->pop[cur], c->pop[1 - cur], c->d.terms, c->d.term_slab,
-                 c->d.err, c->total_clones, c->max_nodes, {p.tiles[0], p.tiles[1], p.tiles[2]}, c->d_maps, tiles64(c), only_run(c)};
+                 c->d.err, c->total_clones, c->max_nodes, {p.tiles[0], p.tiles[1], p.tiles[2]}, c->d_maps, tiles64(c), drag_tiles64(c), only_run(c)};
       if ((e = launch_step(f64, !timing && t == steps - 1, a, s, p.variant)) != cudaSuccess)
         return e;
       if (!timing) cur = 1 - cur;
@@ -1771,7 +1777,7 @@ extern "C" int clbm_drag_fwd(clbm_ctx *c, int steps, int every, double *J) {
     char *dst = (t + 1 < steps) ? loc(t + 1) : c->adj.sig[(t + 1) % 2];
     StepArgs a{c->d.runs, c->nruns, t, loc(t), dst, c->d.terms, c->d.term_slab, c->d.err,
                c->total_clones, c->max_nodes, {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]},
-               c->d_maps, tiles64(c), only_run(c)};
+               c->d_maps, tiles64(c), drag_tiles64(c), only_run(c)};
     CK(launch_step(f64, false, a, s, c->step_variant));
   }
   CK(launch_drag_reduce(f64, c->d, c->nruns, c->total_clones, steps, c->any_stress, c->any_momentum, s));
@@ -1801,7 +1807,7 @@ extern "C" int clbm_drag_bwd(clbm_ctx *c) {
     for (int p = lo; p < hi; p++) {  // recompute P_lo .. P_hi from the checkpoint (step p of the forward)
       StepArgs a{c->d.runs, c->nruns, p, segP(lo, p), segP(lo, p + 1), c->d.terms, c->d.term_slab,
                  c->d.err, c->total_clones, c->max_nodes,
-                 {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]}, c->d_maps, tiles64(c), only_run(c)};
+                 {c->total_tiles[0], c->total_tiles[1], c->total_tiles[2]}, c->d_maps, tiles64(c), drag_tiles64(c), only_run(c)};
       CK(launch_step(f64, false, a, s, c->step_variant));
     }
     for (int p = hi; p >= lo; p--) {

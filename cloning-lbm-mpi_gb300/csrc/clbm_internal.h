@@ -80,6 +80,7 @@ struct StepArgs {
   int total_tiles[3]; // FP32 step grid for tiles of 128 / 256 / 512 nodes
   const float *maps;  // random body-force fields (nullable)
   int tiles64;        // FP64 step grid: 64-node tiles of every clone (pop elements / 576)
+  int drag_tiles;     // blocks of the FP64 step that store drag terms: 64 of a clone each
   const RunDev *one;  // the only run (nruns = 1), in host memory, for the FP64 step; nullptr: read runs
 };
 

@@ -298,7 +298,8 @@ __device__ __forceinline__ bool relax_fx(Node64<BLOCK> &s64, double r0, double o
 // (3 unrolled; 615 unrolled in full, which waits for instructions), 534 with
 // fx_place; the FP64 pipe is then busy 78% of the time and the integer ALU 61%.
 // At one clone of 129x129 (four warps an SM) the chain of dependent operations
-// bounds it, 10.3 us a step whatever the pipe.
+// bounds a step whatever the pipe: 10.05 us with the sums in fixed point, 10.3 in
+// this form.
 // s and m: the node and moments64 of it.
 template <int BLOCK>
 __device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 &m, double out[9], double beta,
@@ -378,9 +379,8 @@ __device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 
 
 // Non-equilibrium second moments with the UNshifted velocity
 // (force.cpp:26-46): pi_xx = sum fneq cx cx, pi_xy = sum fneq cx cy, m the
-// moments of f.  (FP64 sums: few lanes of a warp are at the square's side, and the
-// fixed-point chain is the longer one, 10.65 against 10.2 us a step of one
-// 129x129 clone.)
+// moments of f.  (FP64 sums: the perimeter's few warps leave the FP64 pipe
+// free, and the fixed-point chain is the longer one.)
 __device__ __forceinline__ void pi_ref64(const double f[9], const Moments64 &m, double &pxx,
                                          double &pxy) {
   const Divisor64 d = divisor64(m.rho);

@@ -52,16 +52,16 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
 // plane / 64 of them.  The FP64 pipe bounds these kernels, and the SM with the
 // most nodes sets the time: tiles of 256 gave 16 clones of 200x50 4.1 of them
 // per SM (5 on some), and one state of 129x129 only 65 busy SMs.
-__device__ __forceinline__ int run64(const RunDev *runs, int nruns) {
-  const long long first = 9LL * TILE64 * blockIdx.x;  // pop_base the tile would have
+__device__ __forceinline__ int run64(const RunDev *runs, int nruns, int block) {
+  const long long first = 9LL * TILE64 * block;  // pop_base the tile would have
   int r = 0;
   while (r + 1 < nruns && first >= runs[r + 1].pop_base) r++;
   return r;
 }
-__device__ __forceinline__ NodeLoc locate64(const RunDev &R, int r) {
+__device__ __forceinline__ NodeLoc locate64(const RunDev &R, int r, int block) {
   NodeLoc L;
   const unsigned per = (unsigned)(R.plane / TILE64);
-  const unsigned local = blockIdx.x - (unsigned)(R.pop_base / (9 * TILE64));
+  const unsigned local = (unsigned)block - (unsigned)(R.pop_base / (9 * TILE64));
   L.run = r;
   L.clone = (int)(local / per);
   L.n = (int)(local - (unsigned)L.clone * per) * TILE64 + threadIdx.x;
@@ -94,66 +94,104 @@ __device__ __forceinline__ void step_begin() {
 struct StepArgsOne : StepArgs {
   RunDev rd;
 };
-template <bool LAST, class Args>
-__global__ void __launch_bounds__(TILE64) k_step(const __grid_constant__ Args a) {
-  using T = double;
-  constexpr bool F64 = true, ONE = std::is_same<Args, StepArgsOne>::value;
-  const RunDev *run;
-  int r = 0;
-  if constexpr (ONE) {
-    run = &a.rd;
-  } else {
-    r = run64(a.runs, a.nruns);
-    run = a.runs + r;
-  }
-  const RunDev &R = *run;
-  const NodeLoc L = locate64(R, r);
-  step_wait();
-  if (!L.valid) return;
-  const long long plane = R.plane;
-  const long long cbase = R.pop_base + (long long)L.clone * 9 * plane;
-  const T *__restrict__ src = (const T *)a.src + cbase;
-  T *__restrict__ dst = (T *)a.dst + cbase;
-  const int x = L.x, y = L.y, n = L.n, W = R.W;
-
-  const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
-  const int mask = (in_box || y == 0 || y == R.H - 1) ? bounce_mask(R, x, y) : 0;
-  if (mask & 512) {
-    // inside the square: reset to w[k] (stored shifted as 0 in FP32); its
-    // post-collision values are never pulled by a fluid node
-    if (LAST) {
-#pragma unroll
-      for (int k = 0; k < 9; k++) dst[k * plane + n] = F64 ? (T)w_of(k) : (T)0;
-    }
-    return;
-  }
+// S of node (x,y): the populations pulled from P
+__device__ __forceinline__ void pull64(const double *__restrict__ src, long long plane, int W, int x, int y, int mask,
+                                       double S[9]) {
+  const int n = y * W + x;
   const int xl = (x == 0) ? W - 1 : x - 1;
   const int xr = (x == W - 1) ? 0 : x + 1;
   const int row = y * W;
-  T S[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const int cx = cx_of(k), cy = cy_of(k);
     const int sx = cx == 1 ? xl : (cx == -1 ? xr : x);
     const int srow = cy == 1 ? row - W : (cy == -1 ? row + W : row);
-    const T *p = ((mask >> k) & 1) ? src + opp_of(k) * plane + n : src + k * plane + srow + sx;
+    const double *p = ((mask >> k) & 1) ? src + opp_of(k) * plane + n : src + k * plane + srow + sx;
     S[k] = __ldg(p);
   }
+}
+// The blocks before the tiles of nodes: the drag terms of a clone's perimeter,
+// a slot per thread (a corner's two threads store the same values).  The stress
+// of a perimeter node costs most of a collision's FP64 operations; in the nodes'
+// own blocks the two columns of the square had it run by one lane of every row's
+// warps, a tenth of the FP64 pipe's work at a square of 32 in 129x129, with the
+// collision after it in the longest chain of the step.  us a step: one clone of
+// 129x129 9.6 -> 7.3, 16 of 200x50 31.1 -> 26.3, 32 of 101x101 58.5 -> 46.5, 256
+// of 256x64 532 -> 498.
+__device__ __forceinline__ void drag_block64(const StepArgs &a, const RunDev &R, int block) {
+  const int per = (R.nterms + TILE64 - 1) / TILE64;
+  const int clone = block / per, i = (block - clone * per) * TILE64 + (int)threadIdx.x;
+  step_wait();
+  step_release();
+  if (i >= R.nterms) return;
+  const int ny = R.ymax - R.ymin + 1, nx = R.xmax - R.xmin + 1;
+  const bool side = i < 2 * ny;
+  const int j = side ? (i < ny ? i : i - ny) : (i - 2 * ny < nx ? i - 2 * ny : i - 2 * ny - nx);
+  const int x = side ? (i < ny ? R.xmin : R.xmax) : R.xmin + j;
+  const int y = side ? R.ymin + j : (i - 2 * ny < nx ? R.ymax : R.ymin);
+  double S[9];
+  pull64((const double *)a.src + R.pop_base + (long long)clone * 9 * R.plane, R.plane, R.W, x, y,
+         bounce_mask(R, x, y), S);
+  const Moments64 m = moments_ref64(S);
+  store_drag_terms<true>(R, S, x, y, clone, (double *)a.terms + (long long)a.step * a.term_slab + R.term_base, &m);
+}
+template <bool LAST, class Args>
+__global__ void __launch_bounds__(TILE64) k_step(const __grid_constant__ Args a) {
+  constexpr bool ONE = std::is_same<Args, StepArgsOne>::value;
+  int block = blockIdx.x;
+  if (block < a.drag_tiles) {
+    if constexpr (ONE) {
+      drag_block64(a, a.rd, block);
+    } else {
+      int r = 0, n;
+      while (block >= (n = a.runs[r].nclones * ((a.runs[r].nterms + TILE64 - 1) / TILE64))) {
+        block -= n;
+        r++;
+      }
+      drag_block64(a, a.runs[r], block);
+    }
+    return;
+  }
+  block -= a.drag_tiles;
+  const RunDev *run;
+  int r = 0;
+  if constexpr (ONE) {
+    run = &a.rd;
+  } else {
+    r = run64(a.runs, a.nruns, block);
+    run = a.runs + r;
+  }
+  const RunDev &R = *run;
+  const NodeLoc L = locate64(R, r, block);
+  step_wait();
+  if (!L.valid) return;
+  const long long plane = R.plane;
+  const long long cbase = R.pop_base + (long long)L.clone * 9 * plane;
+  const double *src = (const double *)a.src + cbase;
+  double *__restrict__ dst = (double *)a.dst + cbase;
+  const int x = L.x, y = L.y, n = L.n;
+
+  const bool in_box = x >= R.xmin && x <= R.xmax && y >= R.ymin && y <= R.ymax;
+  const int mask = (in_box || y == 0 || y == R.H - 1) ? bounce_mask(R, x, y) : 0;
+  if (mask & 512) {
+    // inside the square: reset to w[k]; its post-collision values are never
+    // pulled by a fluid node
+    if (LAST) {
+#pragma unroll
+      for (int k = 0; k < 9; k++) dst[k * plane + n] = w_of(k);
+    }
+    return;
+  }
+  double S[9];
+  pull64(src, plane, R.W, x, y, mask, S);
   __shared__ Node64<TILE64> node;
   const Moments64 m = LAST ? moments_ref64(S) : moments64(node, S);
-  if (in_box) {
-    T *terms = (T *)a.terms + (long long)a.step * a.term_slab + R.term_base;
-    T D[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) D[k] = LAST ? S[k] : node_f(node, m.mid, k);
-    store_drag_terms<F64>(R, D, x, y, L.clone, terms, &m);
-  }
   if (LAST) {
     step_release();
 #pragma unroll
     for (int k = 0; k < 9; k++) dst[k * plane + n] = S[k];
   } else {
-    T P[9];
+    double P[9];
     collide_node64(R, node, m, P, node_map(a.maps, R, L.clone, n, R.field_mode && a.step + 1 < R.field_steps));
     step_release();
 #pragma unroll
@@ -277,7 +315,7 @@ cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, 
   const F32Variant &v = kF32Variants[variant];
   const int ts = v.block == 128 ? 0 : (v.block == 256 ? 1 : 2);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(f64 ? a.tiles64 : a.total_tiles[ts]);
+  cfg.gridDim = dim3(f64 ? a.drag_tiles + a.tiles64 : a.total_tiles[ts]);
   cfg.blockDim = dim3(f64 ? TILE64 : v.block);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -303,8 +341,8 @@ cudaError_t launch_step(bool f64, bool last, const StepArgs &a, cudaStream_t s, 
 template <bool F64>
 __global__ void __launch_bounds__(F64 ? TILE64 : STEP_BLOCK) k_reseed(ReseedArgs a) {
   using T = pop_t<F64>;
-  const int r64 = F64 ? run64(a.runs, a.nruns) : 0;
-  const NodeLoc L = F64 ? locate64(a.runs[r64], r64) : locate(a.runs, a.nruns);
+  const int r64 = F64 ? run64(a.runs, a.nruns, (int)blockIdx.x) : 0;
+  const NodeLoc L = F64 ? locate64(a.runs[r64], r64, (int)blockIdx.x) : locate(a.runs, a.nruns);
   if (!L.valid) return;
   const RunDev &R = a.runs[L.run];
   const int x = L.x, y = L.y, n = L.n;
