@@ -357,6 +357,7 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
     R.om1 = 1.0 - R.omega;
     R.cforce = 1.0 - 0.5 * R.omega;
     R.beta = d.beta;
+    R.half_beta = 0.5 * d.beta;
     for (int k = 0; k < 9; k++) R.wcb[k] = w_of(k) * R.cforce * d.beta;
     R.alpha = d.alpha;
     R.force_scale = d.force_scale;

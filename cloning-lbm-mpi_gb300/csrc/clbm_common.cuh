@@ -161,7 +161,7 @@ struct RunDev {
   long long term_base;         // offset of this run in a step's term slab
   long long snap_base;         // element offset of this run's snapshots
   // physics, FP64 (reference order) and FP32 copies
-  double tau, omega, om1, cforce, beta;
+  double tau, omega, om1, cforce, beta, half_beta;
   double wcb[9];               // (w[k]*cforce)*beta, the reference's order
   double alpha, force_scale, force_shift, dt, eps;
   // FP32 collision: omega' = 2 c13 + 4 c2 exactly (c13 ~ omega/3 on a 2^-24

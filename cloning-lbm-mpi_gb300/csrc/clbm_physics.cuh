@@ -121,10 +121,6 @@ __device__ __forceinline__ fx_t fx_abs(double x) {  // of |x| < 1
   const fxu_t y = m >> s;
   return (fx_t)(y | (fxu_t)((y << s) != m));
 }
-__device__ __forceinline__ fx_t fx(double x) {
-  const fx_t y = fx_abs(x);
-  return __double2hiint(x) < 0 ? -y : y;
-}
 // of a positive x in [2^-9, 1): exact
 __device__ __forceinline__ fx_t fx_exact(double x) {
   const unsigned hi = (unsigned)__double2hiint(x);
@@ -169,9 +165,23 @@ __device__ __forceinline__ double fx_double(fx_t v) {
   v >>= p.shift & 31;
   return __hiloint2double((int)(v >> 32) + (int)((1013 + p.shift) << 20), (int)v);
 }
-__device__ __forceinline__ double fx_signed_double(fx_t r) {  // of any rounded value
-  const double d = __ll2double_rn(r);  // exact
-  return r == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (61 << 20), __double2loint(d));
+// any rounded value as a double (a conversion would take the FP64 pipe)
+__device__ __forceinline__ double fx_signed_double(fx_t r) {
+  const fxu_t m = (fxu_t)(r < 0 ? -r : r);
+  const int z = __clzll((fx_t)m);  // 64 for zero
+  const fxu_t v = m << (z & 63) >> 11;  // leading one at 52
+  const int hi = (int)(v >> 32) + ((1023 + 1 - z) << 20);
+  return m == 0 ? 0.0 : __hiloint2double(hi | ((int)(r >> 32) & (int)0x80000000u), (int)v);
+}
+// 3 |x|, rounded as a double, for |x| < 0.32
+__device__ __forceinline__ fx_t fx_abs3(double x) {
+  fxu_t m = 3u * (fx_significand(x) << 9);  // leading one at 62 or 63
+  const unsigned k = 10u + (unsigned)(m >> 63), mask = (1u << k) - 1u;
+  m += (fxu_t)((mask >> 1) + (((unsigned)m >> k) & 1u));
+  m &= ~(fxu_t)mask;
+  const unsigned s = min(1023u - (((unsigned)__double2hiint(x) & 0x7fffffffu) >> 20), 63u);
+  const fxu_t y = m >> s;
+  return (fx_t)(y | (fxu_t)((y << s) != m));
 }
 // A choice between fixed point and FP64 is made for every thread of the warp
 // that is here: a divided warp would go both ways.
@@ -245,8 +255,8 @@ __device__ __forceinline__ void feq_pair_ref64(double t3, double ee, double u2, 
   minus = DADD(DADD(DSUB(1.0, t3), ee), u2);
 }
 // In fixed point where |e| < 0.3 (every sum then lies in [0.1, 2.4)); u = -u2.
-__device__ __forceinline__ void feq_pair_fx(double t3, double ee, fx_t u, fx_t &plus, fx_t &minus) {
-  const fx_t t = fx(t3), q = fx_abs(ee);
+__device__ __forceinline__ void feq_pair_fx(double e, double ee, fx_t u, fx_t &plus, fx_t &minus) {
+  const fx_t t3 = fx_abs3(e), q = fx_abs(ee), t = __double2hiint(e) < 0 ? -t3 : t3;
   plus = fx_round(fx_round(fx_round(FX_ONE + t) + q) - u);
   minus = fx_round(fx_round(fx_round(FX_ONE - t) + q) - u);
 }
@@ -296,21 +306,23 @@ __device__ __forceinline__ bool relax_fx(Node64<BLOCK> &s64, double r0, double o
 // direction, 1192 by pairs, 768 with the sums in fixed point, 731 with the
 // products too, 545 with the node in shared memory and loops over directions
 // (3 unrolled; 615 unrolled in full, which waits for instructions), 534 with
-// fx_place; the FP64 pipe is then busy 78% of the time and the integer ALU 61%.
+// fx_place; 498 with the drag's terms in other blocks, 479 with 3 e, 4 wcb[1] and
+// the signed sums' conversion off the FP64 pipe too: 55 operations are left to
+// it, it is busy 75% of the time (back-to-back products reach 86%) and the integer
+// ALU 71%, so that what is moved from one to the other gains no more.
 // At one clone of 129x129 (four warps an SM) the chain of dependent operations
 // bounds a step whatever the pipe: 10.05 us with the sums in fixed point, 10.3 in
 // this form.
 // s and m: the node and moments64 of it.
 template <int BLOCK>
-__device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 &m, double out[9], double beta,
+__device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 &m, double out[9], double half_beta,
                                               const double wcb[9], double omega,
                                               double om1, double *ux_o = nullptr, double *uy_o = nullptr) {
   double ux, uy;
-  velocity_ref64(m, DMUL(0.5, beta), ux, uy);
+  velocity_ref64(m, half_beta, ux, uy);
   const double u2 = DMUL(-1.5, DADD(DMUL(ux, ux), DMUL(uy, uy)));
   const double es = DADD(ux, uy), ed = DSUB(ux, uy);  // c_5.u = -c_7.u, c_8.u = -c_6.u
   const double t3x = DMUL(3.0, ux);
-  const double t3y = DMUL(3.0, uy), t3s = DMUL(3.0, es), t3d = DMUL(3.0, ed);
   const double hx = DMUL(4.5, ux), hs = DMUL(4.5, es), hd = DMUL(4.5, ed);
   const double eex = DMUL(hx, ux), eey = DMUL(DMUL(4.5, uy), uy), ees = DMUL(hs, es), eed = DMUL(hd, ed);
   // 9 eu = 2 (4.5 eu), rounding included, so its sum with the rest of the
@@ -318,8 +330,13 @@ __device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 
   const double right = DMUL(3.0, DSUB(1.0, ux)), left = DMUL(3.0, DADD(1.0, ux));
   double (*drive)[BLOCK] = s.drive;
   const int t = threadIdx.x;
-  drive[0][t] = DMUL(wcb[0], -t3x);
-  drive[2][t] = drive[4][t] = DMUL(wcb[1], -t3x);
+  const double up = DMUL(wcb[1], -t3x);
+  drive[2][t] = drive[4][t] = up;
+  // wcb[0] is four times wcb[1], and so are the products where neither they nor
+  // wcb are at the ends of the exponent range
+  drive[0][t] = mid_range64(up) && up != 0.0 && mid_range64(wcb[1])
+                    ? __hiloint2double(__double2hiint(up) + 0x200000, __double2loint(up))
+                    : DMUL(wcb[0], -t3x);
   drive[1][t] = DMUL(wcb[1], __fma_rn(2.0, hx, right));
   drive[5][t] = DMUL(wcb[5], __fma_rn(2.0, hs, right));
   drive[8][t] = DMUL(wcb[5], __fma_rn(2.0, hd, right));
@@ -343,10 +360,10 @@ __device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 
       fx_t (*q)[BLOCK] = s.q;
       const fx_t u = fx_abs(u2);
       q[0][t] = fx_round(FX_ONE - u);
-      q[1][t] = __double_as_longlong(t3x), q[3][t] = __double_as_longlong(eex);
-      q[2][t] = __double_as_longlong(t3y), q[4][t] = __double_as_longlong(eey);
-      q[5][t] = __double_as_longlong(t3s), q[7][t] = __double_as_longlong(ees);
-      q[8][t] = __double_as_longlong(t3d), q[6][t] = __double_as_longlong(eed);
+      q[1][t] = __double_as_longlong(ux), q[3][t] = __double_as_longlong(eex);
+      q[2][t] = __double_as_longlong(uy), q[4][t] = __double_as_longlong(eey);
+      q[5][t] = __double_as_longlong(es), q[7][t] = __double_as_longlong(ees);
+      q[8][t] = __double_as_longlong(ed), q[6][t] = __double_as_longlong(eed);
       column_fence();
 #pragma unroll 1
       for (int j = 0; j < 4; j++) {
@@ -366,9 +383,9 @@ __device__ __forceinline__ void collide_ref64(Node64<BLOCK> &s, const Moments64 
   double q[9];
   q[0] = DADD(1.0, u2);
   feq_pair_ref64(t3x, eex, u2, q[1], q[3]);
-  feq_pair_ref64(t3y, eey, u2, q[2], q[4]);
-  feq_pair_ref64(t3s, ees, u2, q[5], q[7]);
-  feq_pair_ref64(t3d, eed, u2, q[8], q[6]);
+  feq_pair_ref64(DMUL(3.0, uy), eey, u2, q[2], q[4]);
+  feq_pair_ref64(DMUL(3.0, es), ees, u2, q[5], q[7]);
+  feq_pair_ref64(DMUL(3.0, ed), eed, u2, q[8], q[6]);
   const double r1 = DMUL(w_of(1), m.rho), r5 = DMUL(w_of(5), m.rho);
 #pragma unroll
   for (int k = 0; k < 9; k++) {

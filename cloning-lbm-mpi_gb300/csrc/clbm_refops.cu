@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(TILE64) k_ref_stream_collide(GeomDev g, double
   double vx, vy;
   __shared__ Node64<TILE64> node;
   const Moments64 m = moments64(node, f);
-  collide_ref64(node, m, post, beta, wcb, omega, om1, &vx, &vy);
+  collide_ref64(node, m, post, DMUL(0.5, beta), wcb, omega, om1, &vx, &vy);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     fin[aos(g, x, y, k)] = post[k];

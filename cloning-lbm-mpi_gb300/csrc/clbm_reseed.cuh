@@ -24,9 +24,9 @@ __device__ __forceinline__ void collide_node64(const RunDev &R, Node64<BLOCK> &n
     double wcb[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) wcb[k] = DMUL(DMUL(w_of(k), R.cforce), beta);
-    collide_ref64(node, m, P, beta, wcb, R.omega, R.om1);
+    collide_ref64(node, m, P, DMUL(0.5, beta), wcb, R.omega, R.om1);
   } else {
-    collide_ref64(node, m, P, R.beta, R.wcb, R.omega, R.om1);
+    collide_ref64(node, m, P, R.half_beta, R.wcb, R.omega, R.om1);
   }
 }
 
