@@ -19,11 +19,36 @@ __device__ __forceinline__ long long aos(const GeomDev &g, int x, int y, int k) 
   return k + 9LL * (y + (long long)g.ny * x);
 }
 
+// A time step is five small kernels in a row, a perturbation three: each is
+// launched with programmatic stream serialisation, so that its blocks take
+// their places while the kernel before it drains, and waits here, before it
+// touches memory, until that has completed and its writes are visible (a step of
+// a 129x129 state 63 -> 51 us, a perturbation of a 257x257 state 65 -> 58.5).
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+static cudaError_t launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // streamCollCompute.cpp:7-93: collide in place into fin, push to the periodic
 // neighbour in fout, macroscopic fields of the pre-collision state.
 __global__ void __launch_bounds__(TILE64) k_ref_stream_collide(GeomDev g, double *fin, double *fout, double *rho,
                                      double *ux, double *uy, double beta0, const double *map,
                                      double tau, double eps) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;  // t = y + ny*x
   if (t >= g.nx * g.ny) return;
   const int x = t / g.ny, y = t - x * g.ny;
@@ -56,6 +81,7 @@ __global__ void __launch_bounds__(TILE64) k_ref_stream_collide(GeomDev g, double
 
 // domain_noSlipWalls.cpp:6-22
 __global__ void k_ref_walls(GeomDev g, double *fout, const double *fin) {
+  after_previous();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= g.nx) return;
   const int top = g.ny - 1;
@@ -69,6 +95,7 @@ __global__ void k_ref_walls(GeomDev g, double *fout, const double *fin) {
 
 // square.cpp:24-50 (the live _TEST variant); one thread per perimeter node
 __global__ void k_ref_square(GeomDev g, double *fout, const double *fin) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int sx = g.xmax - g.xmin, sy = g.ymax - g.ymin;
   const int bottom[3] = {7, 4, 8}, top[3] = {5, 2, 6}, left[3] = {6, 3, 7}, right[3] = {8, 1, 5};
@@ -96,6 +123,7 @@ __global__ void k_ref_square(GeomDev g, double *fout, const double *fin) {
 
 // pops driver :430-439
 __global__ void k_ref_interior(GeomDev g, double *fout) {
+  after_previous();
   const int sx = g.xmax - g.xmin - 1, sy = g.ymax - g.ymin - 1;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (sx <= 0 || sy <= 0 || i >= sx * sy) return;
@@ -107,6 +135,7 @@ __global__ void k_ref_interior(GeomDev g, double *fout) {
 // force.cpp:8-144: per-node terms in parallel, then each side summed in node
 // order by a thread of its own.
 __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *out) {
+  after_previous();
   extern __shared__ double terms[];
   const int sx = g.xmax - g.xmin + 1, sy = g.ymax - g.ymin + 1;
   const int nterm = 2 * sy + 2 * sx;
@@ -145,7 +174,8 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
 // generatePerturbedState.cpp:4-38 in two passes: fixed-order norm reduction,
 // then the element-wise update.  A block takes 1024 values, four per thread
 // (per value the reduction costs the FP64 pipe, which bounds these kernels,
-// 2.5 operations instead of 10, next to the mix's 2 nsnap - 1).  mixed
+// 0.5 operations instead of 8, next to the 2 of the squares and the mix's
+// 2 nsnap - 1).  mixed
 // (nullable): where the mix is kept for the update, which forms it again
 // otherwise.
 constexpr int PERTURB_BLOCK = 1024;
@@ -160,6 +190,7 @@ __device__ __forceinline__ double snapshot_mix(const double *snaps, int nsnap, i
 }
 __global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, const double *snaps, int nsnap, int n,
                                                            const Prefactors pref, double *partials, double *mixed) {
+  after_previous();
   __shared__ double red[2][256 / 32];
   double n0 = 0.0, n1 = 0.0;
 #pragma unroll
@@ -168,8 +199,8 @@ __global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, co
     if (i >= (unsigned)n) break;
     const double mix = snapshot_mix(snaps, nsnap, n, i, pref);
     if (mixed) mixed[i] = mix;
-    n0 = DADD(n0, DMUL(fin[i], fin[i]));
-    n1 = DADD(n1, DMUL(mix, mix));
+    n0 = __fma_rn(fin[i], fin[i], n0);
+    n1 = __fma_rn(mix, mix, n1);
   }
   for (int o = 16; o > 0; o >>= 1) {
     n0 = DADD(n0, __shfl_down_sync(0xffffffffu, n0, o));
@@ -198,6 +229,7 @@ __global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, co
 // (generatePerturbedState.cpp:22-36).
 __global__ void __launch_bounds__(256) k_ref_perturb_finalize(const Prefactors pref, int nsnap, const double *partials,
                                                               int nblocks, double eps, double *out) {
+  after_previous();
   __shared__ double red[2][256 / 32];
   double a0 = 0.0, a1 = 0.0;
   for (int b = threadIdx.x; b < nblocks; b += 256) {
@@ -228,6 +260,7 @@ __global__ void __launch_bounds__(256) k_ref_perturb_finalize(const Prefactors p
 // f <- (f + eps * mix * weight) / a with (weight, 1/a) from k_ref_perturb_finalize
 __global__ void k_ref_perturb_apply(double *fin, const double *snaps, int nsnap, int n,
                                     const Prefactors pref, const double *wa, double eps, const double *mixed) {
+  after_previous();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (unsigned)n) return;
   const double w = wa[0], inv = wa[1];
@@ -258,10 +291,10 @@ static cudaError_t run_perturb(double *fin, const double *snaps, double eps, int
   Prefactors pref = {};
   for (int q = 0; q < nsnap; q++) pref.v[q] = prefactors[q];
   const int nb = (n + PERTURB_BLOCK - 1) / PERTURB_BLOCK;
-  k_ref_perturb_norms<<<nb, 256, 0, st>>>(fin, snaps, nsnap, n, pref, part, mixed);
-  k_ref_perturb_finalize<<<1, 256, 0, st>>>(pref, nsnap, part, nb, eps, wa);
-  k_ref_perturb_apply<<<(n + 255) / 256, 256, 0, st>>>(fin, snaps, nsnap, n, pref, wa, eps, mixed);
-  return cudaGetLastError();
+  cudaError_t e = launch_after(k_ref_perturb_norms, nb, 256, 0, st, fin, snaps, nsnap, n, pref, part, mixed);
+  if (e == cudaSuccess) e = launch_after(k_ref_perturb_finalize, 1, 256, 0, st, pref, nsnap, part, nb, eps, wa);
+  if (e == cudaSuccess) e = launch_after(k_ref_perturb_apply, (n + 255) / 256, 256, 0, st, fin, snaps, nsnap, n, pref, wa, eps, mixed);
+  return e;
 }
 
 static GeomDev to_dev(const clbm_geom *g) {
@@ -274,9 +307,8 @@ extern "C" int clbm_ref_stream_collide(const clbm_geom *g, double *fin, double *
   if (int s = check_geom(g)) return s;
   if (!fin || !fout) return CLBM_ERR_INVALID;
   const int n = g->nx * g->ny;
-  k_ref_stream_collide<<<(n + TILE64 - 1) / TILE64, TILE64, 0, (cudaStream_t)stream>>>(
-      to_dev(g), fin, fout, rho, ux, uy, beta, nullptr, tau, 0.0);
-  return clbm_status_from_cuda(cudaGetLastError());
+  return clbm_status_from_cuda(launch_after(k_ref_stream_collide, (n + TILE64 - 1) / TILE64, TILE64, 0,
+                                            (cudaStream_t)stream, to_dev(g), fin, fout, rho, ux, uy, beta, (const double *)nullptr, tau, 0.0));
 }
 
 extern "C" int clbm_ref_stream_collide_spatial(const clbm_geom *g, double *fin, double *fout,
@@ -286,32 +318,28 @@ extern "C" int clbm_ref_stream_collide_spatial(const clbm_geom *g, double *fin, 
   if (int s = check_geom(g)) return s;
   if (!fin || !fout || !map) return CLBM_ERR_INVALID;
   const int n = g->nx * g->ny;
-  k_ref_stream_collide<<<(n + TILE64 - 1) / TILE64, TILE64, 0, (cudaStream_t)stream>>>(
-      to_dev(g), fin, fout, rho, ux, uy, beta0, map, tau, eps);
-  return clbm_status_from_cuda(cudaGetLastError());
+  return clbm_status_from_cuda(launch_after(k_ref_stream_collide, (n + TILE64 - 1) / TILE64, TILE64, 0,
+                                            (cudaStream_t)stream, to_dev(g), fin, fout, rho, ux, uy, beta0, map, tau, eps));
 }
 
 extern "C" int clbm_ref_walls_bb(const clbm_geom *g, double *fout, const double *fin,
                                  void *stream) {
   if (int s = check_geom(g)) return s;
-  k_ref_walls<<<(g->nx + 127) / 128, 128, 0, (cudaStream_t)stream>>>(to_dev(g), fout, fin);
-  return clbm_status_from_cuda(cudaGetLastError());
+  return clbm_status_from_cuda(launch_after(k_ref_walls, (g->nx + 127) / 128, 128, 0, (cudaStream_t)stream, to_dev(g), fout, fin));
 }
 
 extern "C" int clbm_ref_square_bb(const clbm_geom *g, double *fout, const double *fin,
                                   void *stream) {
   if (int s = check_geom(g)) return s;
   const int nthreads = (g->xmax - g->xmin - 1) + (g->ymax - g->ymin - 1) + 1;
-  k_ref_square<<<(nthreads + 127) / 128, 128, 0, (cudaStream_t)stream>>>(to_dev(g), fout, fin);
-  return clbm_status_from_cuda(cudaGetLastError());
+  return clbm_status_from_cuda(launch_after(k_ref_square, (nthreads + 127) / 128, 128, 0, (cudaStream_t)stream, to_dev(g), fout, fin));
 }
 
 extern "C" int clbm_ref_interior_reset(const clbm_geom *g, double *fout, void *stream) {
   if (int s = check_geom(g)) return s;
   const int sx = g->xmax - g->xmin - 1, sy = g->ymax - g->ymin - 1;
   if (sx <= 0 || sy <= 0) return CLBM_OK;
-  k_ref_interior<<<(sx * sy + 127) / 128, 128, 0, (cudaStream_t)stream>>>(to_dev(g), fout);
-  return clbm_status_from_cuda(cudaGetLastError());
+  return clbm_status_from_cuda(launch_after(k_ref_interior, (sx * sy + 127) / 128, 128, 0, (cudaStream_t)stream, to_dev(g), fout));
 }
 
 extern "C" int clbm_ref_force_on_square(const clbm_geom *g, const double *f, double omega,
@@ -323,8 +351,7 @@ extern "C" int clbm_ref_force_on_square(const clbm_geom *g, const double *f, dou
   cudaError_t e = call_alloc((void **)&d_out, sizeof(double), st);
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
   const int nterm = 2 * (g->xmax - g->xmin + 1) + 2 * (g->ymax - g->ymin + 1);
-  k_ref_force<<<1, 256, nterm * sizeof(double), st>>>(to_dev(g), f, omega, d_out);
-  e = cudaGetLastError();
+  e = launch_after(k_ref_force, 1, 256, nterm * sizeof(double), st, to_dev(g), f, omega, d_out);
   if (e == cudaSuccess) e = cudaMemcpyAsync(result, d_out, sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(d_out, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
