@@ -32,14 +32,16 @@
 // FMA pipe of a scheduler (154), and 36 cycles of the SM's shared memory for
 // four schedulers' 18 accesses each (144).  On the 256x64 channel (bands
 // 23/18/23, 512 threads) a segment takes about 210 (local step) to 260 cycles;
-// 4096 clones run at 0.297 ms per step, where one node per thread with the
+// 4096 clones run at 0.289 ms per step, where one node per thread with the
 // four direction pairs packed took 0.367; 1024 clones of 400x100 (9 bands) at
-// 0.204 against 0.353.  What made the difference besides the packing (ms per
+// 0.196 against 0.353.  What made the difference besides the packing (ms per
 // step of the 256x64 case): each warp's share of the deal kept in registers
 // instead of worked out in every step (0.344 -> 0.317), whole planes per
 // population instead of node records, so that what crosses a band edge goes as
 // whole sectors (0.317 -> 0.306; 400x100: 0.265 -> 0.225), planes a constant
 // distance apart, so that a pair's slots are constant offsets (0.306 -> 0.297),
+// row ends inside the band through plain shared memory and a perimeter update
+// of its own (0.298 -> 0.289),
 // and the split cluster barrier with the edge rows first (400x100: 0.33 ->
 // 0.28).  Random-field steps read two values per pair from L2: loaded one
 // segment ahead, 0.343 -> 0.329 ms per step over an interval with 20 of 100
