@@ -191,34 +191,52 @@ __device__ __forceinline__ double snapshot_mix(const double *snaps, int nsnap, i
   for (int q = 1; q < nsnap; q++) mix = DADD(mix, DMUL(pref.v[q], snaps[(long long)q * n + i]));
   return mix;
 }
-// The same mix with its sums in fixed point (the FP64 pipe bounds the pass, and
-// the sums are half of its operations; clbm_physics.cuh has the method): at
-// 2^(59 - place) over the power of two of the first snapshot's value, room for
-// sums of four times that value by the prefactors.  false where a product is
-// negative, a sum too large or one of the partial sums less than 2^-8 of the
+// The mixes of four values at once (their loads in flight together), the sums
+// in fixed point: the FP64 pipe bounds the pass, and the sums are half of its
+// operations (clbm_physics.cuh has the method).  At 2^(59 - place) over the
+// power of two of the first snapshot's value, room for sums of four times that
+// value by the prefactors.  A bit of the result for each value that has a
+// negative product, too large a sum or a partial sum of less than 2^-8 of the
 // room.  The first product is exact there (mix_place).  Ten snapshots of a
-// 257x257 state: the perturbation 58.5 -> 47 us.
-__device__ __forceinline__ bool snapshot_mix_fx(const double *snaps, int nsnap, int n, unsigned i,
-                                                const Prefactors &pref, double &mix) {
-  const double first = snaps[i];
-  const int e0 = __double2hiint(first) >> 20;
-  int bad = e0 - 900 | 1100 - e0, least = 0x7fffffff, most = 0;
-  fx_t acc = 0;
+// 257x257 state, from a cold L2: the pass 37 us in FP64, 30 one value at a time,
+// 22 four at a time; the whole perturbation 61, 57, 48 us.
+__device__ __forceinline__ unsigned snapshot_mix_fx(const double *snaps, int nsnap, int n, const unsigned i[4],
+                                                    const Prefactors &pref, double mix[4]) {
+  fx_t acc[4];
+  int e0[4], bad[4], least[4], most[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) acc[j] = 0, least[j] = 0x7fffffff, most[j] = 0;
   for (int q = 0; q < nsnap; q++) {
-    const double p = DMUL(pref.v[q], q == 0 ? first : snaps[(long long)q * n + i]);
-    const int hi = __double2hiint(p), s = pref.place + e0 + 2 - (hi >> 20);
-    bad |= hi | s;
-    const fxu_t m = (((fxu_t)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(p)) << 9;
-    const unsigned c = min((unsigned)s, 63u);
-    const fxu_t y = m >> c;
-    const fx_t v = acc + (fx_t)(y | (fxu_t)((y << c) != m));
-    if (q > 0) least = min(least, (int)(v >> 32));
-    most = max(most, (int)(v >> 32));
-    acc = q > 0 ? fx_round(v) : v;
+    const double *snap = snaps + (long long)q * n;
+    double p[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) p[j] = snap[i[j]];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (q == 0) {
+        e0[j] = __double2hiint(p[j]) >> 20;
+        bad[j] = e0[j] - 900 | 1100 - e0[j];
+      }
+      p[j] = DMUL(pref.v[q], p[j]);
+      const int hi = __double2hiint(p[j]), s = pref.place + e0[j] + 2 - (hi >> 20);
+      bad[j] |= hi | s;
+      const fxu_t m = (((fxu_t)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(p[j])) << 9;
+      const unsigned c = min((unsigned)s, 63u);
+      const fxu_t y = m >> c;
+      const fx_t v = acc[j] + (fx_t)(y | (fxu_t)((y << c) != m));
+      if (q > 0) least[j] = min(least[j], (int)(v >> 32));
+      most[j] = max(most[j], (int)(v >> 32));
+      acc[j] = q > 0 ? fx_round(v) : v;
+    }
   }
-  const double d = fx_double(acc);
-  mix = __hiloint2double(__double2hiint(d) + ((pref.place + e0 + 2 - 1023) << 20), __double2loint(d));
-  return bad >= 0 && least >= 1 << 22 && most < 1 << 30;
+  unsigned off = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const double d = fx_double(acc[j]);
+    mix[j] = __hiloint2double(__double2hiint(d) + ((pref.place + e0[j] + 2 - 1023) << 20), __double2loint(d));
+    off |= (unsigned)!(bad[j] >= 0 && least[j] >= 1 << 22 && most[j] < 1 << 30) << j;
+  }
+  return off;
 }
 // The place for the prefactors: none below zero, the first at least 2^-7 and the
 // first two together 2^-5 of the sum's power of two, so that few values are
@@ -240,16 +258,19 @@ __global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, co
   after_previous();
   __shared__ double red[2][256 / 32];
   double n0 = 0.0, n1 = 0.0;
+  static_assert(PERTURB_BLOCK == 4 * 256, "four values per thread");
+  unsigned i[4], off = 15;
+  double mix[4];
 #pragma unroll
-  for (int j = 0; j < PERTURB_BLOCK / 256; j++) {
-    const unsigned i = blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x;
-    if (i >= (unsigned)n) break;
-    double mix;
-    if (pref.place == NO_PLACE || !snapshot_mix_fx(snaps, nsnap, n, i, pref, mix))
-      mix = snapshot_mix(snaps, nsnap, n, i, pref);
-    if (mixed) mixed[i] = mix;
-    n0 = __fma_rn(fin[i], fin[i], n0);
-    n1 = __fma_rn(mix, mix, n1);
+  for (int j = 0; j < 4; j++) i[j] = min(blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x, (unsigned)n - 1);
+  if (pref.place != NO_PLACE) off = snapshot_mix_fx(snaps, nsnap, n, i, pref, mix);
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x >= (unsigned)n) break;
+    if (off >> j & 1) mix[j] = snapshot_mix(snaps, nsnap, n, i[j], pref);
+    if (mixed) mixed[i[j]] = mix[j];
+    n0 = __fma_rn(fin[i[j]], fin[i[j]], n0);
+    n1 = __fma_rn(mix[j], mix[j], n1);
   }
   for (int o = 16; o > 0; o >>= 1) {
     n0 = DADD(n0, __shfl_down_sync(0xffffffffu, n0, o));
