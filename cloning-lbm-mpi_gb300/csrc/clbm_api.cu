@@ -718,10 +718,11 @@ static int run_rows_max(const clbm_ctx *c, int r) {
   return m;
 }
 
-// whether run r runs cluster-resident: its plan says so and its bands are
-// held on chip (temporal_resident); every other run streams
+// whether run r runs cluster-resident: its plan says so, its bands are held on
+// chip (temporal_resident) and the kernel takes its square (temporal_square);
+// every other run streams
 static bool run_resident(const clbm_ctx *c, int r) {
-  return c->run_cs[r] > 0 && temporal_resident(c->runs_h[r].W, run_rows_max(c, r));
+  return c->run_cs[r] > 0 && temporal_square(c->runs_h[r]) && temporal_resident(c->runs_h[r].W, run_rows_max(c, r));
 }
 
 static LbPlan current_plan(const clbm_ctx *c, bool f64) {
@@ -1281,9 +1282,9 @@ static bool shape_fits(const RunDev &R, int cs, int tv) {
          temporal_max_clusters(cs, tv, R.W, (R.H + cs - 1) / cs, R.field_mode != 0) >= 1;
 }
 
-// ... and is held on chip at it (the autotuner's candidates)
+// ... and does run so at it (the autotuner's candidates)
 static bool shape_resident(const RunDev &R, int cs, int tv) {
-  return temporal_resident(R.W, (R.H + cs - 1) / cs) && shape_fits(R, cs, tv);
+  return temporal_square(R) && temporal_resident(R.W, (R.H + cs - 1) / cs) && shape_fits(R, cs, tv);
 }
 
 // largest band of a split row0[0..cs]
@@ -1364,8 +1365,8 @@ static cudaError_t full_plan(clbm_ctx *c, const std::vector<int> &cs, const std:
 // (the best streaming shape against every cluster-resident shape that fits
 // it), and that per-run plan -- cluster-resident runs concurrent with the
 // streaming ones -- is timed as a whole and kept if it beats the uniform
-// winner.  Results are cached per (lattice sizes, clone counts) for the
-// process.
+// winner.  Results are cached per (lattice sizes, clone counts, whether the
+// cluster-resident kernel takes the square) for the process.
 struct TuneResult {
   int best;
   std::vector<int> cs, tv;
@@ -1389,6 +1390,7 @@ extern "C" int clbm_autotune(clbm_ctx *c, int launches, int *best, double *ms_pe
     key.push_back(R.W);
     key.push_back(R.H);
     key.push_back(R.nclones);
+    key.push_back(temporal_square(R));
   }
   if (!ms_per_variant) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);

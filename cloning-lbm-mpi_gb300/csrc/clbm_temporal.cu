@@ -339,14 +339,14 @@ __device__ __forceinline__ bool in_box(const RunDev &R, int x, int y) {
 // such nodes is perimeter_count.
 __device__ __forceinline__ int perimeter_count(const RunDev &R, int ylo, int yhi) {
   if (yhi < ylo) return 0;
-  const int ncol = R.xmax > R.xmin ? 2 : 1, nin = R.xmax > R.xmin ? R.xmax - R.xmin - 1 : 0;
-  return ncol * (yhi - ylo + 1) + (ylo == R.ymin ? nin : 0) + (yhi == R.ymax && R.ymax > R.ymin ? nin : 0);
+  const int nin = R.xmax - R.xmin - 1;
+  return 2 * (yhi - ylo + 1) + (ylo == R.ymin ? nin : 0) + (yhi == R.ymax ? nin : 0);
 }
 __device__ __forceinline__ void perimeter_node(const RunDev &R, int ylo, int yhi, int j, int &x, int &y) {
-  const int ncol = R.xmax > R.xmin ? 2 : 1, side = ncol * (yhi - ylo + 1), nin = R.xmax - R.xmin - 1;
+  const int side = 2 * (yhi - ylo + 1), nin = R.xmax - R.xmin - 1;
   if (j < side) {
-    y = ylo + (ncol == 2 ? j >> 1 : j);
-    x = ncol == 2 && (j & 1) ? R.xmax : R.xmin;
+    y = ylo + (j >> 1);
+    x = (j & 1) ? R.xmax : R.xmin;
   } else {
     const int q = j - side;
     const bool bottom = ylo == R.ymin && q < nin;
@@ -997,7 +997,8 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
   size_t smem = 0;
   if (field && a.keep) return cudaErrorInvalidConfiguration;
   TemporalFn fn = temporal_fn(variant, cs, W, rows_max, a.keep ? 2 : field, &smem);
-  if (!fn || !temporal_resident(W, rows_max) || a.steps < 1) return cudaErrorInvalidConfiguration;
+  if (!fn || !temporal_resident(W, rows_max) || !temporal_square(a.rd) || a.steps < 1)
+    return cudaErrorInvalidConfiguration;
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
   TemporalArgs args = a;
