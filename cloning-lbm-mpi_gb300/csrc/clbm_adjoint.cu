@@ -9,7 +9,8 @@
 //   sigma_t = J_C(S_t)^T Pull^T sigma_{t+1} + kappa grad D(S_t),  1 <= t < T
 //   sigma_0 = J_C(S_0)^T Pull^T sigma_1
 // Pull^T is a gather too: P(m,k) is read by exactly one slot, the node's own
-// (m, opp k) when that slot is bounced back, else (m + c_k, k); square-interior
+// (m, opp k) when that slot is bounced back, else (m + c_k, k) -- around a square
+// one node thick by both of them, or by none (adj_gather_thin); square-interior
 // nodes carry no sensitivity (they are reset every step).  The collision
 // Jacobian is a rank-3 update of (1-omega) I through rho, jx, jy, so its
 // transpose costs three reductions per node.  D is the stress-integration drag
@@ -144,7 +145,27 @@ __device__ __forceinline__ void collide_adjoint(const RunDev &R, const T S[9], c
   for (int k = 0; k < 9; k++) out[k] = om1 * pi[k] + A + (T)cx_of(k) * Bx + (T)cy_of(k) * By;
 }
 
-template <bool F64>
+// Pull^T of node (x, y) of a run whose square is one node thick: its nodes bounce
+// back on both sides, so P(n,k) is read by the node's own slot (n, opp k) if that
+// bounces and also by (n + c_k, k) if that does not.  at: offset of (n - c_k).
+template <typename T>
+__device__ __forceinline__ void adj_gather_thin(const RunDev &R, const T *sig, int x, int y, int mask,
+                                                const int at[9], T pi[9]) {
+  const long long n = (long long)y * R.W + x;
+  const int xl = (x == 0) ? R.W - 1 : x - 1, xr = (x == R.W - 1) ? 0 : x + 1;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const int cx = cx_of(k), cy = cy_of(k), tx = cx == 1 ? xr : (cx == -1 ? xl : x), ty = y + cy;
+    T v = T(0);
+    if ((mask >> opp_of(k)) & 1) v = sig[opp_of(k) * R.plane + n];
+    if (ty >= 0 && ty < R.H && !((bounce_mask(R, tx, ty) >> k) & 1)) v += sig[k * R.plane + at[opp_of(k)]];
+    pi[k] = v;
+  }
+}
+
+// THIN: some run's square is one node thick (the others pay for no more than the
+// choice; a context without one takes the kernel without it)
+template <bool F64, bool THIN>
 __global__ void __launch_bounds__(STEP_BLOCK) k_adj_step(AdjArgs a) {
   using T = real_t<F64>;
   int clone, n;
@@ -184,9 +205,13 @@ __global__ void __launch_bounds__(STEP_BLOCK) k_adj_step(AdjArgs a) {
     for (int k = 0; k < 9; k++)
       S[k] = __ldg(P + (((mask >> k) & 1) ? opp_of(k) * plane + n : k * plane + at[k]));
   }
+  if (THIN && !square_thick(R)) {
+    adj_gather_thin<T>(R, sig, x, y, mask, at, pi);
+  } else {
 #pragma unroll
-  for (int k = 0; k < 9; k++)  // n + c_k = n - c_{opp k}
-    pi[k] = __ldg(sig + (((mask >> opp_of(k)) & 1) ? opp_of(k) * plane + n : k * plane + at[opp_of(k)]));
+    for (int k = 0; k < 9; k++)  // n + c_k = n - c_{opp k}
+      pi[k] = __ldg(sig + (((mask >> opp_of(k)) & 1) ? opp_of(k) * plane + n : k * plane + at[opp_of(k)]));
+  }
   T o[9];
   collide_adjoint<T>(R, S, pi, adj_beta<T>(R, a, clone, n), o);
   if (a.with_drag && in_box) {
@@ -247,12 +272,11 @@ cudaError_t launch_adj_init(bool f64, const RunDev *runs, int nruns, const void 
 
 cudaError_t launch_adj_step(bool f64, const RunDev *runs, int nruns, const void *sigma_in,
                             void *sigma_out, const void *P, bool with_drag, bool from_s0, int t,
-                            const float *maps, int blocks, cudaStream_t s) {
+                            const float *maps, bool thin, int blocks, cudaStream_t s) {
   AdjArgs a{runs, nruns, sigma_in, sigma_out, P, with_drag ? 1 : 0, from_s0 ? 1 : 0, t, maps};
-  if (f64)
-    k_adj_step<true><<<blocks, STEP_BLOCK, 0, s>>>(a);
-  else
-    k_adj_step<false><<<blocks, STEP_BLOCK, 0, s>>>(a);
+  const auto kernel = f64 ? (thin ? k_adj_step<true, true> : k_adj_step<true, false>)
+                          : (thin ? k_adj_step<false, true> : k_adj_step<false, false>);
+  kernel<<<blocks, STEP_BLOCK, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -719,10 +719,10 @@ static int run_rows_max(const clbm_ctx *c, int r) {
 }
 
 // whether run r runs cluster-resident: its plan says so, its bands are held on
-// chip (temporal_resident) and the kernel takes its square (temporal_square);
+// chip (temporal_resident) and the kernel takes its square (square_thick);
 // every other run streams
 static bool run_resident(const clbm_ctx *c, int r) {
-  return c->run_cs[r] > 0 && temporal_square(c->runs_h[r]) && temporal_resident(c->runs_h[r].W, run_rows_max(c, r));
+  return c->run_cs[r] > 0 && square_thick(c->runs_h[r]) && temporal_resident(c->runs_h[r].W, run_rows_max(c, r));
 }
 
 static LbPlan current_plan(const clbm_ctx *c, bool f64) {
@@ -1284,7 +1284,7 @@ static bool shape_fits(const RunDev &R, int cs, int tv) {
 
 // ... and does run so at it (the autotuner's candidates)
 static bool shape_resident(const RunDev &R, int cs, int tv) {
-  return temporal_square(R) && temporal_resident(R.W, (R.H + cs - 1) / cs) && shape_fits(R, cs, tv);
+  return square_thick(R) && temporal_resident(R.W, (R.H + cs - 1) / cs) && shape_fits(R, cs, tv);
 }
 
 // largest band of a split row0[0..cs]
@@ -1390,7 +1390,7 @@ extern "C" int clbm_autotune(clbm_ctx *c, int launches, int *best, double *ms_pe
     key.push_back(R.W);
     key.push_back(R.H);
     key.push_back(R.nclones);
-    key.push_back(temporal_square(R));
+    key.push_back(square_thick(R));
   }
   if (!ms_per_variant) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -1802,6 +1802,8 @@ extern "C" int clbm_drag_bwd(clbm_ctx *c) {
   cudaStream_t s = c->stream;
   const int nseg = (T + C - 1) / C;
   int cur = 0;  // sig[cur] holds sigma_{t+1}
+  bool thin = false;
+  for (const RunDev &R : c->runs_h) thin = thin || !square_thick(R);
   auto segP = [&](int lo, int p) -> char * {
     return p == lo ? c->adj.ckpt + (size_t)(lo / C) * pop : c->adj.seg + (size_t)(p - lo) * pop;
   };
@@ -1818,13 +1820,13 @@ extern "C" int clbm_drag_bwd(clbm_ctx *c) {
         CK(launch_adj_init(f64, c->d.runs, c->nruns, segP(lo, p), c->adj.sig[cur], c->total_blocks, s));
       } else {
         CK(launch_adj_step(f64, c->d.runs, c->nruns, c->adj.sig[cur], c->adj.sig[1 - cur], segP(lo, p),
-                           true, false, p + 1, c->d_maps, c->total_blocks, s));
+                           true, false, p + 1, c->d_maps, thin, c->total_blocks, s));
         cur = 1 - cur;
       }
     }
   }
   CK(launch_adj_step(f64, c->d.runs, c->nruns, c->adj.sig[cur], c->adj.sig[1 - cur], c->adj.s0, false,
-                     true, 0, c->d_maps, c->total_blocks, s));
+                     true, 0, c->d_maps, thin, c->total_blocks, s));
   c->adj.result = 1 - cur;
   CK(cudaStreamSynchronize(s));
   return check_error_word(c);

@@ -215,6 +215,13 @@ __host__ __device__ inline int bounce_mask(const RunDev &r, int x, int y) {
   return m;
 }
 
+// Whether every post-collision population is read by one slot: a square one node
+// thick bounces back on both sides of its nodes, and the populations between
+// them and their fluid neighbours are read by two slots or by none.  The
+// cluster-resident kernel's in-place update needs one (such a run streams), the
+// adjoint takes another gather for the rest.
+__host__ __device__ inline bool square_thick(const RunDev &r) { return r.xmax > r.xmin && r.ymax > r.ymin; }
+
 // ---- Philox4x32-10 (Salmon et al., SC'11) -------------------------------
 __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32_t k1) {
 #pragma unroll

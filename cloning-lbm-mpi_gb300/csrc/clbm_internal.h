@@ -150,7 +150,7 @@ cudaError_t launch_adj_init(bool f64, const RunDev *runs, int nruns, const void 
                             int blocks, cudaStream_t s);
 cudaError_t launch_adj_step(bool f64, const RunDev *runs, int nruns, const void *sigma_in,
                             void *sigma_out, const void *P, bool with_drag, bool from_s0, int t,
-                            const float *maps, int blocks, cudaStream_t s);
+                            const float *maps, bool thin, int blocks, cudaStream_t s);
 cudaError_t launch_hist_drag(const DevArrays &d, int total_clones, int steps, double *hist, int max_hist,
                              cudaStream_t s);
 cudaError_t launch_hist_labels(const DevArrays &d, int total_clones, int *hist, int max_hist,
@@ -180,11 +180,6 @@ int temporal_rows_limit(int W);
 // the room of one node more, so a band at the very limit may not be (its run
 // then steps through the streaming kernel, the same results)
 bool temporal_resident(int W, int rows);
-// whether the cluster-resident kernel can take a run's square at all: its
-// in-place update needs every slot to belong to one node, and where the square
-// is one node thick its nodes bounce back on both sides, so that the slots
-// between them and their fluid neighbours belong to two (such a run streams)
-inline bool temporal_square(const RunDev &R) { return R.xmax > R.xmin && R.ymax > R.ymin; }
 int temporal_variant_count();
 // band splits (clbm_bands.cu): row0[0..cs] of H rows in cs bands, the first
 // H % cs one row more; or balanced for an estimated per-step cost in which a

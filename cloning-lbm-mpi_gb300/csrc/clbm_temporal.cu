@@ -997,7 +997,7 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
   size_t smem = 0;
   if (field && a.keep) return cudaErrorInvalidConfiguration;
   TemporalFn fn = temporal_fn(variant, cs, W, rows_max, a.keep ? 2 : field, &smem);
-  if (!fn || !temporal_resident(W, rows_max) || !temporal_square(a.rd) || a.steps < 1)
+  if (!fn || !temporal_resident(W, rows_max) || !square_thick(a.rd) || a.steps < 1)
     return cudaErrorInvalidConfiguration;
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
