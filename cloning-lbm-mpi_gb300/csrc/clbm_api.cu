@@ -339,12 +339,13 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
       const int tb = 128 << q;
       R.tiles[q] = (R.nodes + tb - 1) / tb;
       // clone = umulhi(local tile, ceil(2^32/tiles)) is exact while
-      // local * (tiles - 1) < 2^32
+      // local * (tiles - 1) < 2^32; a lattice of one tile has no such factor
+      // in 32 bits: 0 stands for it (k_step_f32)
       if ((unsigned long long)d.nclones * R.tiles[q] * (unsigned long long)(R.tiles[q] - 1) >= (1ULL << 32)) {
         delete c;
         return fail(CLBM_ERR_INVALID, "too many clones for the lattice size in one run (clones * tiles^2 >= 2^32)");
       }
-      R.tiles_div[q] = (unsigned)(((1ULL << 32) + R.tiles[q] - 1) / R.tiles[q]);
+      R.tiles_div[q] = R.tiles[q] > 1 ? (unsigned)(((1ULL << 32) + R.tiles[q] - 1) / R.tiles[q]) : 0u;
       R.tile_base[q] = c->total_tiles[q];
       c->total_tiles[q] += d.nclones * R.tiles[q];
     }

@@ -152,7 +152,7 @@ struct RunDev {
   unsigned div_w;              // ceil(2^32 / W): y = umulhi(n, div_w)
   int drag_mode;               // 0 stress integration, 1 momentum exchange
   // tile tables of the FP32 step for tiles of 128 / 256 / 512 nodes: first
-  // block of this run, tiles per clone and ceil(2^32 / tiles)
+  // block of this run, tiles per clone and ceil(2^32 / tiles) (0 for one tile)
   int tile_base[3];
   int tiles[3];
   unsigned tiles_div[3];

@@ -221,7 +221,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_f32(StepArgs a) {
   while (r + 1 < a.nruns && b >= a.runs[r + 1].tile_base[TS]) r++;
   const RunDev &R = a.runs[r];
   const unsigned local = (unsigned)(b - R.tile_base[TS]);
-  const int clone = (int)__umulhi(local, R.tiles_div[TS]);
+  const unsigned div = R.tiles_div[TS];  // 0: a clone is one tile
+  const int clone = (int)(div ? __umulhi(local, div) : local);
   const int tile = (int)local - clone * R.tiles[TS];
   const int n = tile * BLOCK + threadIdx.x;
   const int W = R.W, H = R.H;
