@@ -94,8 +94,9 @@ __device__ __forceinline__ void step_begin() {
 struct StepArgsOne : StepArgs {
   RunDev rd;
 };
-// S of node (x,y): the populations pulled from P
-__device__ __forceinline__ void pull64(const double *__restrict__ src, long long plane, int W, int x, int y, int mask,
+// S of node (x,y): the populations pulled from P.  (Plain loads: while a step's
+// blocks wait the step before still writes P, which read-only loads rule out.)
+__device__ __forceinline__ void pull64(const double *src, long long plane, int W, int x, int y, int mask,
                                        double S[9]) {
   const int n = y * W + x;
   const int xl = (x == 0) ? W - 1 : x - 1;
@@ -107,7 +108,7 @@ __device__ __forceinline__ void pull64(const double *__restrict__ src, long long
     const int sx = cx == 1 ? xl : (cx == -1 ? xr : x);
     const int srow = cy == 1 ? row - W : (cy == -1 ? row + W : row);
     const double *p = ((mask >> k) & 1) ? src + opp_of(k) * plane + n : src + k * plane + srow + sx;
-    S[k] = __ldg(p);
+    S[k] = *p;
   }
 }
 // The blocks before the tiles of nodes: the drag terms of a clone's perimeter,
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_f32(StepArgs a) {
   if (!valid) return;
   const int plane = (int)R.plane;
   const long long cb = R.pop_base + (long long)clone * 9 * R.plane;
-  const float *__restrict__ src = (const float *)a.src + cb;
+  const float *src = (const float *)a.src + cb;
   float *__restrict__ dst = (float *)a.dst + cb;
   const int xl = (x == 0) ? W - 1 : x - 1;
   const int xr = (x == W - 1) ? 0 : x + 1;
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_f32(StepArgs a) {
   }
   float S[9];
 #pragma unroll
-  for (int k = 0; k < 9; k++) S[k] = __ldg(src + off[k]);
+  for (int k = 0; k < 9; k++) S[k] = src[off[k]];  // (plain loads, as pull64)
   if (in_box) {
     float *terms = (float *)a.terms + (long long)a.step * a.term_slab + R.term_base;
     store_drag_terms<false>(R, S, x, y, clone, terms);
