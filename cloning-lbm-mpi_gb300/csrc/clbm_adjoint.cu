@@ -112,17 +112,7 @@ __device__ __forceinline__ void collide_adjoint(const RunDev &R, const T S[9], c
   const T rho = (sizeof(T) == 8 ? sum : T(1) + sum);
   const T jx = (S[1] - S[3]) + ((S[5] - S[7]) + (S[8] - S[6]));
   const T jy = (S[2] - S[4]) + ((S[5] - S[7]) + (S[6] - S[8]));
-  // FP64: one division for all three quotients (its pipe is the bound); FP32
-  // waits for memory and divides each
-  T ux, uy, inv;
-  if constexpr (sizeof(T) == 8) {
-    inv = T(1) / rho;
-    ux = (jx + T(0.5) * beta) * inv;
-    uy = jy * inv;
-  } else {
-    ux = (jx + T(0.5) * beta) / rho;
-    uy = jy / rho;
-  }
+  const T ux = (jx + T(0.5) * beta) / rho, uy = jy / rho;
   const T u2 = T(1.5) * (ux * ux + uy * uy);
   const T wa = T(1) / T(9), wd = T(1) / T(36);
   const T a13 = pi[1] + pi[3], a24 = pi[2] + pi[4];
@@ -138,7 +128,7 @@ __device__ __forceinline__ void collide_adjoint(const RunDev &R, const T S[9], c
   const T Gx = omega * rho * (T(3) * Px + T(9) * (ux * Pxx + uy * Pxy) - T(3) * ux * P0) +
                cf * beta * (T(9) * Pxx - T(3) * P0);
   const T Gy = omega * rho * (T(3) * Py + T(9) * (ux * Pxy + uy * Pyy) - T(3) * uy * P0) + T(9) * cf * beta * Pxy;
-  if constexpr (sizeof(T) == 4) inv = T(1) / rho;
+  const T inv = T(1) / rho;
   const T A = G0 - (ux * Gx + uy * Gy) * inv;
   const T Bx = Gx * inv, By = Gy * inv;
 #pragma unroll
