@@ -805,40 +805,62 @@ static TemporalArgs temporal_args(const clbm_ctx *c, const LbPlan &p, int r, int
   return ta;
 }
 
+// Launch the plan's cluster-resident runs, P_0 in src, S_T left in dst, each on
+// a side stream of its own behind what the context's stream holds; join_resident
+// makes the context's stream wait for them.  fuse: the kernels form P_0
+// themselves from the reseed's inputs (fuse->src, a buffer other than dst)
+// instead of reading src.  keep: checkpoints, P_t of every t that `every` divides
+// at keep + t / every * (a population buffer).
+static cudaError_t fork_resident(clbm_ctx *c, const LbPlan &p, int steps, const void *src, void *dst,
+                                 const ReseedArgs *fuse, void *keep, int every, int &nside) {
+  cudaError_t e;
+  nside = 0;
+  for (int r = 0; r < c->nruns; r++) nside += p.cs[r] > 0 && plan_active(p, r);
+  if (nside) {
+    if ((e = ensure_side(c, nside)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(c->fork_join[0], c->stream)) != cudaSuccess) return e;
+  }
+  int i = 0;
+  for (int r = 0; r < c->nruns; r++) {
+    if (!(p.cs[r] > 0 && plan_active(p, r))) continue;
+    cudaStream_t ts = c->side[i];
+    if ((e = cudaStreamWaitEvent(ts, c->fork_join[0], 0)) != cudaSuccess) return e;
+    TemporalArgs ta = temporal_args(c, p, r, steps, (const float *)src, (float *)dst);
+    if (fuse) {
+      ta.fused = 1;
+      ta.rs = *fuse;
+    }
+    if (keep) {
+      ta.keep = (float *)keep;
+      ta.keep_stride = (long long)c->pop_elems;
+      ta.keep_every = every;
+    }
+    if ((e = launch_temporal(ta, p.cs[r], p.tv[r], ta.rd.nclones, ta.rd.W, ts)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(c->fork_join[1 + i], ts)) != cudaSuccess) return e;
+    i++;
+  }
+  return cudaSuccess;
+}
+static cudaError_t join_resident(clbm_ctx *c, int nside) {
+  cudaError_t e;
+  for (int k = 0; k < nside; k++)
+    if ((e = cudaStreamWaitEvent(c->stream, c->fork_join[1 + k], 0)) != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
 // Enqueue `steps` LB steps of the plan's runs.  Interval: P_0 in buffer src,
 // S_T left in buffer dst; the streaming runs alternate between the two
 // buffers as the pull scheme does and store S on their last step.  timing
 // (autotuner): every streaming launch reads src and writes the other buffer
 // and none is a last step, so the state in src is left untouched.  fuse
-// (cluster-resident runs only): the kernels form P_0 themselves from the
-// reseed's inputs (fuse->src, a buffer other than dst) instead of reading src.
+// (cluster-resident runs only): as fork_resident.
 static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int src, int dst, bool timing,
                                     const ReseedArgs *fuse = nullptr) {
   const bool f64 = c->precision == CLBM_FP64;
   cudaStream_t s = c->stream;
   cudaError_t e;
   int nside = 0;
-  for (int r = 0; r < c->nruns; r++) nside += p.cs[r] > 0 && plan_active(p, r);
-  if (nside) {
-    if ((e = ensure_side(c, nside)) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(c->fork_join[0], s)) != cudaSuccess) return e;
-  }
-  int i = 0;
-  for (int r = 0; r < c->nruns; r++) {
-    if (!(p.cs[r] > 0 && plan_active(p, r))) continue;
-    const RunDev &R = c->runs_h[r];
-    cudaStream_t ts = c->side[i];
-    if ((e = cudaStreamWaitEvent(ts, c->fork_join[0], 0)) != cudaSuccess) return e;
-    const int cs = p.cs[r];
-    TemporalArgs ta = temporal_args(c, p, r, steps, (const float *)c->pop[src], (float *)c->pop[dst]);
-    if (fuse) {
-      ta.fused = 1;
-      ta.rs = *fuse;
-    }
-    if ((e = launch_temporal(ta, cs, p.tv[r], R.nclones, R.W, ts)) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(c->fork_join[1 + i], ts)) != cudaSuccess) return e;
-    i++;
-  }
+  if ((e = fork_resident(c, p, steps, c->pop[src], c->pop[dst], fuse, nullptr, 0, nside)) != cudaSuccess) return e;
   if (p.nstream > 0) {
     int cur = src;
     for (int t = 0; t < steps; t++) {
@@ -849,9 +871,7 @@ static cudaError_t enqueue_lb_steps(clbm_ctx *c, const LbPlan &p, int steps, int
       if (!timing) cur = 1 - cur;
     }
   }
-  for (int k = 0; k < nside; k++)
-    if ((e = cudaStreamWaitEvent(s, c->fork_join[1 + k], 0)) != cudaSuccess) return e;
-  return cudaSuccess;
+  return join_resident(c, nside);
 }
 
 // The streaming runs' table after a change of the plan or of a band split;
@@ -1734,19 +1754,15 @@ static bool adj_resident(const clbm_ctx *c) {
   return all;
 }
 
-// `steps` steps from P_0 in ckpt; P_t kept at ckpt + t / every * (a population
-// buffer) for every t that `every` divides, S_T to dst.
+// `steps` steps from P_0 in ckpt, where the checkpoints go too; S_T to dst.  The
+// runs side by side, as in an interval: one after the other each is a chain of
+// its own steps that leaves most of the chip idle (100 steps, 16 runs of four
+// clones of 129x129 6.4 ms, 32 of one of 97x33 9.0; 0.91 and 0.46 ms so, streaming 2.2
+// and 1.1).
 static cudaError_t adj_forward(clbm_ctx *c, int steps, void *ckpt, int every, void *dst) {
-  const LbPlan p = current_plan(c, false);
-  for (int r = 0; r < c->nruns; r++) {
-    TemporalArgs ta = temporal_args(c, p, r, steps, (const float *)ckpt, (float *)dst);
-    ta.keep = (float *)ckpt;
-    ta.keep_stride = (long long)c->pop_elems;
-    ta.keep_every = every;
-    const cudaError_t e = launch_temporal(ta, p.cs[r], p.tv[r], ta.rd.nclones, ta.rd.W, c->stream);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  int nside = 0;
+  cudaError_t e = fork_resident(c, current_plan(c, false), steps, ckpt, dst, nullptr, ckpt, every, nside);
+  return e == cudaSuccess ? join_resident(c, nside) : e;
 }
 
 extern "C" int clbm_drag_fwd(clbm_ctx *c, int steps, int every, double *J) {
