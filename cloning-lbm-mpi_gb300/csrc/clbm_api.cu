@@ -30,6 +30,9 @@ extern "C" void clbm_set_error(const char *msg) { g_last_error = msg ? msg : "";
 
 extern "C" int clbm_status_from_cuda(cudaError_t e) {
   if (e == cudaSuccess) return CLBM_OK;
+  // reported here: left in the runtime's last error (where cudaLaunchKernelEx and
+  // the allocations put it) it would fail the next call that launches a kernel
+  cudaGetLastError();
   g_last_error = std::string("CUDA: ") + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? CLBM_ERR_NOMEM : CLBM_ERR_CUDA;
 }
