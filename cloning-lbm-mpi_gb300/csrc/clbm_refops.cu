@@ -361,10 +361,10 @@ static cudaError_t run_perturb(double *fin, const double *snaps, double eps, int
   Prefactors pref = {};
   for (int q = 0; q < nsnap; q++) pref.v[q] = prefactors[q];
   pref.place = mix_place(prefactors, nsnap);
-  const int nb = (n + PERTURB_BLOCK - 1) / PERTURB_BLOCK;
+  const int nb = (n - 1) / PERTURB_BLOCK + 1;
   cudaError_t e = launch_after(k_ref_perturb_norms, nb, 256, 0, st, fin, snaps, nsnap, n, pref, part, mixed);
   if (e == cudaSuccess) e = launch_after(k_ref_perturb_finalize, 1, 256, 0, st, pref, nsnap, part, nb, eps, wa);
-  if (e == cudaSuccess) e = launch_after(k_ref_perturb_apply, (n + 255) / 256, 256, 0, st, fin, snaps, nsnap, n, pref, wa, eps, mixed);
+  if (e == cudaSuccess) e = launch_after(k_ref_perturb_apply, (n - 1) / 256 + 1, 256, 0, st, fin, snaps, nsnap, n, pref, wa, eps, mixed);
   return e;
 }
 
@@ -433,7 +433,7 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
                                         int n, const double *prefactors, void *stream) {
   if (!fin || !snaps || !prefactors || nsnap < 1 || nsnap > 64 || n < 1) return CLBM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t nb = ((size_t)n + PERTURB_BLOCK - 1) / PERTURB_BLOCK, head = 2 + 2 * nb;
+  const size_t nb = (size_t)(n - 1) / PERTURB_BLOCK + 1, head = 2 + 2 * nb;
   double *d_buf = nullptr;
   cudaError_t e = call_alloc((void **)&d_buf, sizeof(double) * (head + n), st);
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
