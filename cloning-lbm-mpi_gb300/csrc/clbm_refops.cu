@@ -435,9 +435,16 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nb = (size_t)(n - 1) / PERTURB_BLOCK + 1, head = 2 + 2 * nb;
   double *d_buf = nullptr;
+  // (without room for a further state the mix is formed twice, the same values)
+  bool keep = true;
   cudaError_t e = call_alloc((void **)&d_buf, sizeof(double) * (head + n), st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    keep = false;
+    e = call_alloc((void **)&d_buf, sizeof(double) * head, st);
+  }
   if (e != cudaSuccess) return clbm_status_from_cuda(e);
-  e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, d_buf, d_buf + 2, d_buf + head, st);
+  e = run_perturb(fin, snaps, eps, nsnap, n, prefactors, d_buf, d_buf + 2, keep ? d_buf + head : nullptr, st);
   cudaFreeAsync(d_buf, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return clbm_status_from_cuda(e);
