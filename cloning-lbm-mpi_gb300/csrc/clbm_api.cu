@@ -12,7 +12,6 @@
 #include <cstring>
 #include <string>
 #include <algorithm>
-#include <atomic>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -51,14 +50,16 @@ static int fail(int status, const char *msg) {
 // The pool of call_alloc.  The device's default pool gives its memory back to
 // the system at every synchronisation, which made each small temporary cost
 // about 200 us of mapping; this one keeps up to 64 MB (a dump's or a snapshot's
-// stage) and gives it back with the last context.  Stream-ordered, so any
-// stream and thread may use it.  One per CUDA context, told apart by the
-// context's id: a pool does not outlive a cudaDeviceReset.
+// stage) and gives it back with the device's last clbm_ctx, or by
+// clbm_destroy(NULL): a program of the reference's functions alone has no
+// clbm_ctx.  Stream-ordered, so any stream and thread may use it.  One per CUDA
+// context, told apart by the context's id: a pool does not outlive a
+// cudaDeviceReset.
 namespace {
 constexpr unsigned long long kPoolKeep = 64ull << 20;
 std::mutex g_pool_mutex;
 std::map<unsigned long long, cudaMemPool_t> g_pools;
-std::atomic<int> g_contexts{0};
+std::map<int, int> g_contexts;  // clbm_ctx alive, by device
 
 // the current context's pool, or nullptr (create: make it if there is none)
 cudaMemPool_t current_pool(bool create) {
@@ -97,6 +98,29 @@ cudaMemPool_t current_pool(bool create) {
   g_pools[id] = pool;
   return pool;
 }
+
+void give_back() {
+  if (cudaMemPool_t pool = current_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
+
+int count_context() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  g_contexts[dev]++;
+  return dev;
+}
+void drop_context(int dev) {
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (--g_contexts[dev] > 0) return;
+  }
+  int cur = 0;
+  const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != dev;
+  if (other && cudaSetDevice(dev) != cudaSuccess) return;
+  give_back();
+  if (other) cudaSetDevice(cur);
+}
 }  // namespace
 
 cudaError_t clbm::call_alloc(void **p, size_t bytes, cudaStream_t s) {
@@ -110,11 +134,8 @@ struct GraphEntry {
 };
 
 struct clbm_ctx {
-  clbm_ctx() { g_contexts++; }
-  ~clbm_ctx() {
-    if (--g_contexts == 0)
-      if (cudaMemPool_t pool = current_pool(false)) cudaMemPoolTrimTo(pool, 0);
-  }
+  const int device = count_context();
+  ~clbm_ctx() { drop_context(device); }
   int nruns = 0, precision = 0, max_steps = 0, flags = 0;
   std::vector<clbm_run_desc> desc;
   std::vector<RunDev> runs_h;
@@ -242,7 +263,10 @@ static void destroy_graphs(clbm_ctx *c) {
 }
 
 extern "C" int clbm_destroy(clbm_ctx *c) {
-  if (!c) return CLBM_OK;
+  if (!c) {
+    give_back();
+    return CLBM_OK;
+  }
   destroy_graphs(c);
   for (cudaStream_t t : c->side) cudaStreamDestroy(t);
   for (cudaEvent_t e : c->fork_join) cudaEventDestroy(e);

@@ -197,6 +197,10 @@ int clbm_ref_random_field(int dx, int dy, double sigma, unsigned long long seed,
 /* max_steps bounds the steps of one interval (drag-term storage). */
 int clbm_create(const clbm_run_desc *runs, int nruns, int precision,
                 int max_steps, int flags, clbm_ctx **out);
+/* Destroys a context; NULL is no context.  The library keeps up to 64 MB of
+ * device memory per device for the temporaries of its calls (the function
+ * level's too) and gives it back with the device's last context, or by
+ * clbm_destroy(NULL) on the current device. */
 int clbm_destroy(clbm_ctx *ctx);
 
 /* HOST FP64 arrays in the reference AoS layout, N = 9*Dx*Dy values per clone.
