@@ -1705,7 +1705,7 @@ extern "C" int clbm_set_band_rows(clbm_ctx *c, int run, const int *rows, int nba
 extern "C" int clbm_get_band_rows(clbm_ctx *c, int run, int *rows, int *nbands) {
   if (!c || !rows || !nbands) return fail(CLBM_ERR_INVALID, "NULL argument");
   if (run < 0 || run >= c->nruns) return fail(CLBM_ERR_INVALID, "run out of range");
-  const int cs = c->run_cs[run];
+  const int cs = run_resident(c, run) ? c->run_cs[run] : 0;
   *nbands = cs;
   if (!cs) return CLBM_OK;
   std::vector<int> row0 = c->run_rows[run];
@@ -1720,7 +1720,7 @@ extern "C" int clbm_get_band_rows(clbm_ctx *c, int run, int *rows, int *nbands) 
 extern "C" int clbm_get_run_variants(clbm_ctx *c, int *variants) {
   if (!c || !variants) return fail(CLBM_ERR_INVALID, "NULL argument");
   for (int r = 0; r < c->nruns; r++)
-    variants[r] = c->run_cs[r] ? variant_index(c->run_cs[r], c->run_tv[r]) : c->step_variant;
+    variants[r] = run_resident(c, r) ? variant_index(c->run_cs[r], c->run_tv[r]) : c->step_variant;
   return CLBM_OK;
 }
 

@@ -324,7 +324,11 @@ int clbm_set_step_variant(clbm_ctx *ctx, int variant);
  * it concurrently, each on its own stream; the runs given a streaming variant
  * share one step launch per step and must name the same streaming variant */
 int clbm_set_run_variants(clbm_ctx *ctx, const int *variants);
-/* the variant each run uses now (nruns entries) */
+/* the variant each run uses now (nruns entries): for a run that was given a
+ * cluster-resident one but steps through the streaming kernel, that one's.  So
+ * runs one whose square is one node thick, and one whose largest band has too
+ * many rows of an odd width (a row is stored as (W + 1) / 2 pairs of nodes, and
+ * a band holds 3220 pairs; the shape is accepted by the nodes' number) */
 int clbm_get_run_variants(clbm_ctx *ctx, int *variants);
 /* Band split of a cluster-resident run: cluster rank b holds rows[b]
  * consecutive lattice rows (from the bottom wall up) of every clone.  An even
