@@ -477,8 +477,11 @@ __device__ __forceinline__ Band make_band(const TemporalArgs &a, float *A, cg::c
 // P_0 into the "after a local step" layout A[n][opp k].  FUSED: formed here
 // from the previous interval's S (parent copy, perturbation, first collision;
 // the same per-node function as the reseed kernel, so bit-identical).
-// Square-interior nodes and the empty lane of an odd width's last pair get
-// zeros (the fluid at rest).
+// Square-interior nodes get zeros (the fluid at rest).  The empty lane of an odd
+// width's last pair gets a fluid of density 2^40 at rest: the force moves it by
+// 2^-40 of what it does the others, so that it takes part in the density test at
+// no cost (an open column of density one, driven where the square blocks the rest,
+// reaches speeds at which FP32 loses its density).
 template <int THREADS, bool FUSED, class Band>
 __device__ __forceinline__ void load_band(const TemporalArgs &a, const Band &b, float *A) {
   const RunDev &R = a.rd;
@@ -487,7 +490,10 @@ __device__ __forceinline__ void load_band(const TemporalArgs &a, const Band &b, 
     const int h = j >= b.np, i = h ? j - b.np : j;
     const int ly = (int)__umulhi((unsigned)i, b.div_wh), xh = i - ly * b.Wh, x = xh + h * b.Wh, y = b.row0 + ly;
     float P[9];
-    if (x >= b.W || (FUSED && x > R.xmin && x < R.xmax && y > R.ymin && y < R.ymax)) {
+    if (x >= b.W) {
+#pragma unroll
+      for (int k = 0; k < 9; k++) P[k] = 0x1p40f * (float)w_of(k);
+    } else if (FUSED && x > R.xmin && x < R.xmax && y > R.ymin && y < R.ymax) {
 #pragma unroll
       for (int k = 0; k < 9; k++) P[k] = 0.0f;
     } else if (FUSED) {
