@@ -517,12 +517,12 @@ __device__ __forceinline__ float field_eps(const TemporalArgs &a, int t) {
 // byte per segment and the ends of the list's ranges.  temporal_smem (a
 // function of the nodes alone) is what a shape is accepted by; a plane of
 // kPairs takes the largest band of an even width that it accepts (3219
-// pairs), one of kPairsHalf lets two CTAs share an SM.
+// pairs), one of kPairsHalf lets two CTAs share an SM, one of kPairsQuarter four.
 __host__ __device__ inline size_t temporal_smem(int nb) {
   const int nseg = (nb + 31) / 32;
   return sizeof(float) * 9 * (size_t)nb + 2 * (size_t)((nseg + 7) & ~7) + (size_t)((nseg + 15) & ~15) + 32;
 }
-constexpr int kPairs = 3220, kPairsHalf = 1600;
+constexpr int kPairs = 3220, kPairsHalf = 1600, kPairsQuarter = 784;
 // segments of 32 pairs: the first and the last row by themselves, then the
 // rows between them
 __host__ __device__ inline int segment_count(int rows, int Wh) {
@@ -938,38 +938,51 @@ bool temporal_resident(int W, int rows) {
   return (long long)rows * ((W + 1) / 2) <= kPairs && pair_smem(kPairs, rows, W) <= kSmemLimit;
 }
 
-struct TemporalVariant {
-  int threads;
-  TemporalFn fn[2][3];  // [plane size: kPairs, kPairsHalf][uniform force, random field, checkpoints]
+struct TemporalKernel {
+  int pairs, threads;  // of a plane, of a block
+  TemporalFn fn[3];    // uniform force, random field, checkpoints
 };
 
-#define GENERIC(T, M, N) \
-  {k_temporal_f32<T, M, N, false, false>, k_temporal_f32<T, M, N, true, false>, k_temporal_f32<T, M, N, false, true>}
-// (1024 and 512 threads take an SM's registers alone: no use for the half planes)
-static const TemporalVariant kTemporal[] = {{1024, {GENERIC(1024, 1, kPairs), {nullptr, nullptr, nullptr}}},
-                                            {512, {GENERIC(512, 1, kPairs), {nullptr, nullptr, nullptr}}},
-                                            {256, {GENERIC(256, 2, kPairs), GENERIC(256, 2, kPairsHalf)}}};
-#undef GENERIC
+#define KERNEL(T, M, N) \
+  {N, T, {k_temporal_f32<T, M, N, false, false>, k_temporal_f32<T, M, N, true, false>, k_temporal_f32<T, M, N, false, true>}}
+// By variant, for bands of up to `pairs`.  (1024 and 512 threads take an SM's
+// registers alone: no use for smaller planes.)
+static const TemporalKernel kTemporal[][3] = {
+    {KERNEL(1024, 1, kPairs)},
+    {KERNEL(512, 1, kPairs)},
+    {KERNEL(256, 2, kPairs), KERNEL(256, 2, kPairsHalf), KERNEL(128, 4, kPairsQuarter)}};
+#undef KERNEL
 
 int temporal_variant_count() { return (int)(sizeof(kTemporal) / sizeof(kTemporal[0])); }
 
-// the kernel (kind: an index of fn's) of a variant for this band shape and its shared memory, or
-// nullptr when it cannot run it
-static TemporalFn temporal_fn(int variant, int cs, int W, int rows_max, int kind, size_t *smem) {
+// The kernel of a variant for `blocks` bands of this shape and its shared memory,
+// or nullptr when it cannot run it: the smallest planes that hold the band, for as
+// many CTAs an SM as they allow, the quarter's only for more blocks than the half
+// planes hold at once (its 128 threads take longer over one band).  us a step,
+// half and quarter planes: 8192 clones of 24x16 34.8 and 26.4, of 32x24 48.3 and
+// 41.5, 4096 of 64x24 32.4 and 30.0 (a kernel of one node a thread, four CTAs an SM
+// too, took 35.2, 42.5 and 31.4); 320 clones of 48x32 3.93 and 3.48, 304 (two an
+// SM) 2.50 and 2.84, one 1.77 and 2.32.
+static const TemporalKernel *temporal_kernel(int variant, int cs, int W, int rows_max, int blocks, size_t *smem) {
   if (variant < 0 || variant >= temporal_variant_count() || cs < 1 || cs > MAX_CLUSTER || rows_max < 1)
     return nullptr;
   if (temporal_smem(rows_max * W) > kSmemLimit) return nullptr;
-  const TemporalVariant &v = kTemporal[variant];
-  const bool half = v.fn[1][kind] && rows_max * ((W + 1) / 2) <= kPairsHalf;
-  *smem = std::min(pair_smem(half ? kPairsHalf : kPairs, rows_max, W), kSmemLimit);
-  return v.fn[half][kind];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return nullptr;
+  const TemporalKernel *k = kTemporal[variant];
+  for (int i = 1; i < (blocks > 2 * sms ? 3 : 2); i++)
+    if (kTemporal[variant][i].pairs >= rows_max * ((W + 1) / 2)) k = &kTemporal[variant][i];
+  *smem = std::min(pair_smem(k->pairs, rows_max, W), kSmemLimit);
+  return k;
 }
 
-static cudaLaunchConfig_t temporal_config(int cs, int variant, int nclones, size_t smem, cudaStream_t s,
+static cudaLaunchConfig_t temporal_config(int cs, int threads, int nclones, size_t smem, cudaStream_t s,
                                           cudaLaunchAttribute *attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs * nclones);
-  cfg.blockDim = dim3(kTemporal[variant].threads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1002,27 +1015,29 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
   }
   size_t smem = 0;
   if (field && a.keep) return cudaErrorInvalidConfiguration;
-  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, a.keep ? 2 : field, &smem);
-  if (!fn || !temporal_resident(W, rows_max) || !square_thick(a.rd) || a.steps < 1)
+  const TemporalKernel *k = temporal_kernel(variant, cs, W, rows_max, cs * nclones, &smem);
+  if (!k || !temporal_resident(W, rows_max) || !square_thick(a.rd) || a.steps < 1)
     return cudaErrorInvalidConfiguration;
+  const TemporalFn fn = k->fn[a.keep ? 2 : field];
   cudaError_t e = prepare(fn, cs, smem);
   if (e != cudaSuccess) return e;
   TemporalArgs args = a;
   const unsigned long long wh = (W + 1) / 2;
   args.div_wh = (unsigned)(((1ULL << 32) + wh - 1) / wh);
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = temporal_config(cs, variant, nclones, smem, s, attr);
+  cudaLaunchConfig_t cfg = temporal_config(cs, k->threads, nclones, smem, s, attr);
   return cudaLaunchKernelEx(&cfg, fn, args);
 }
 
 // Whether the cluster shape can be resident at all (occupancy query, no launch).
 int temporal_max_clusters(int cs, int variant, int W, int rows_max, bool field) {
   size_t smem = 0;
-  TemporalFn fn = temporal_fn(variant, cs, W, rows_max, field, &smem);
-  if (!fn) return 0;
+  const TemporalKernel *k = temporal_kernel(variant, cs, W, rows_max, 0, &smem);
+  if (!k) return 0;
+  const TemporalFn fn = k->fn[field];
   if (prepare(fn, cs, smem) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = temporal_config(cs, variant, 64, smem, nullptr, attr);
+  cudaLaunchConfig_t cfg = temporal_config(cs, k->threads, 64, smem, nullptr, attr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, (void *)fn, &cfg) != cudaSuccess) {
     cudaGetLastError();
