@@ -297,6 +297,9 @@ static cudaError_t dalloc(T *&p, size_t n) {
   return cudaMalloc((void **)&p, n * sizeof(T));
 }
 
+// blocks that store a run's drag terms in an FP64 step
+static int run_drag_tiles64(const RunDev &R) { return R.nclones * ((R.nterms + TILE64 - 1) / TILE64); }
+
 extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, int max_steps,
                            int flags, clbm_ctx **out) {
   if (!out) return fail(CLBM_ERR_INVALID, "out is NULL");
@@ -360,6 +363,7 @@ extern "C" int clbm_create(const clbm_run_desc *runs, int nruns, int precision, 
     R.nodes = d.width * d.height;
     R.blocks_per_clone = (R.nodes + STEP_BLOCK - 1) / STEP_BLOCK;
     R.nterms = 2 * (d.ymax - d.ymin + 1) + 2 * (d.xmax - d.xmin + 1);
+    if (r > 0) R.drag_base = c->runs_h[r - 1].drag_base + run_drag_tiles64(c->runs_h[r - 1]);
     R.div_w = (unsigned)(((1ULL << 32) + (unsigned long long)d.width - 1) / (unsigned long long)d.width);
     R.plane = ((long long)R.nodes + 63) / 64 * 64;
     for (int q = 0; q < 3; q++) {
@@ -805,11 +809,7 @@ static cudaError_t ensure_side(clbm_ctx *c, int n) {
 }
 
 // blocks that store the drag terms in an FP64 step
-static int drag_tiles64(const clbm_ctx *c) {
-  int n = 0;
-  for (const RunDev &R : c->runs_h) n += R.nclones * ((R.nterms + TILE64 - 1) / TILE64);
-  return n;
-}
+static int drag_tiles64(const clbm_ctx *c) { return c->runs_h.back().drag_base + run_drag_tiles64(c->runs_h.back()); }
 static const RunDev *only_run(const clbm_ctx *c) { return c->nruns == 1 ? &c->runs_h[0] : nullptr; }
 
 // The cluster-resident kernel's arguments for run r of a plan.

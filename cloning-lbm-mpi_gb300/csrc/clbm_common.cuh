@@ -156,6 +156,7 @@ struct RunDev {
   int tile_base[3];
   int tiles[3];
   unsigned tiles_div[3];
+  int drag_base;               // first of this run's drag blocks in an FP64 step
   long long pop_base;          // element offset of this run's clone 0
   long long plane;             // elements per population plane (padded)
   long long term_base;         // offset of this run in a step's term slab

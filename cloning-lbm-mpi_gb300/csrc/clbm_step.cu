@@ -47,6 +47,25 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
   return L;
 }
 
+// The last run for which reached(r) holds, as it does up to some run (0 among
+// them).  By halves down to 32 runs and from there one by one: each look at the
+// table of runs is a load that the next waits for.  us a step, 1024 runs of a clone
+// of 40x24: 884 one by one, 145 so (halves only: 137); 32 runs of a clone of 97x33,
+// where one by one is as fast as it gets: 19.7 (halves only: 20.4).
+template <class F>
+__device__ __forceinline__ int last_run(int nruns, F reached) {
+  int lo = 0, hi = nruns;
+  while (hi - lo > 32) {
+    const int mid = (lo + hi) / 2;
+    if (reached(mid))
+      lo = mid;
+    else
+      hi = mid;
+  }
+  while (lo + 1 < hi && reached(lo + 1)) lo++;
+  return lo;
+}
+
 // The FP64 step and reseed take tiles of 64 nodes: the planes are multiples of
 // 64 elements, so a run's tiles start at pop_base / 576 and a clone has
 // plane / 64 of them.  The FP64 pipe bounds these kernels, and the SM with the
@@ -54,9 +73,7 @@ __device__ __forceinline__ NodeLoc locate(const RunDev *runs, int nruns) {
 // per SM (5 on some), and one state of 129x129 only 65 busy SMs.
 __device__ __forceinline__ int run64(const RunDev *runs, int nruns, int block) {
   const long long first = 9LL * TILE64 * block;  // pop_base the tile would have
-  int r = 0;
-  while (r + 1 < nruns && first >= runs[r + 1].pop_base) r++;
-  return r;
+  return last_run(nruns, [&](int r) { return runs[r].pop_base <= first; });
 }
 __device__ __forceinline__ NodeLoc locate64(const RunDev &R, int r, int block) {
   NodeLoc L;
@@ -144,12 +161,8 @@ __global__ void __launch_bounds__(TILE64) k_step(const __grid_constant__ Args a)
     if constexpr (ONE) {
       drag_block64(a, a.rd, block);
     } else {
-      int r = 0, n;
-      while (block >= (n = a.runs[r].nclones * ((a.runs[r].nterms + TILE64 - 1) / TILE64))) {
-        block -= n;
-        r++;
-      }
-      drag_block64(a, a.runs[r], block);
+      const int r = last_run(a.nruns, [&](int q) { return a.runs[q].drag_base <= block; });
+      drag_block64(a, a.runs[r], block - a.runs[r].drag_base);
     }
     return;
   }
