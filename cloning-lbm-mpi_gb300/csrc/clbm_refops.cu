@@ -180,6 +180,7 @@ __global__ void k_ref_force(GeomDev g, const double *f, double omega, double *ou
 // (nullable): where the mix is kept for the update, which forms it again
 // otherwise.
 constexpr int PERTURB_BLOCK = 1024;
+constexpr int PERTURB_SMALL = 256;  // of small states, one per thread (perturb_block)
 struct Prefactors {
   double v[64];
   int place;  // exponent of their sum where snapshot_mix_fx takes them, else NO_PLACE
@@ -253,20 +254,22 @@ static int mix_place(const double *prefactors, int nsnap) {
   const bool ok = prefactors[0] >= std::ldexp(1.0, e - 7) && prefactors[0] + 0.5 * prefactors[1] >= std::ldexp(1.0, e - 5);
   return ok ? e : NO_PLACE;
 }
+template <int PER>
 __global__ void __launch_bounds__(256) k_ref_perturb_norms(const double *fin, const double *snaps, int nsnap, int n,
                                                            const Prefactors pref, double *partials, double *mixed) {
   after_previous();
   __shared__ double red[2][256 / 32];
   double n0 = 0.0, n1 = 0.0;
-  static_assert(PERTURB_BLOCK == 4 * 256, "four values per thread");
-  unsigned i[4], off = 15;
-  double mix[4];
+  const unsigned first = blockIdx.x * (256 * PER) + threadIdx.x;
+  unsigned i[PER], off = (1u << PER) - 1;
+  double mix[PER];
 #pragma unroll
-  for (int j = 0; j < 4; j++) i[j] = min(blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x, (unsigned)n - 1);
-  if (pref.place != NO_PLACE) off = snapshot_mix_fx(snaps, nsnap, n, i, pref, mix);
+  for (int j = 0; j < PER; j++) i[j] = min(first + j * 256, (unsigned)n - 1);
+  if constexpr (PER == 4)
+    if (pref.place != NO_PLACE) off = snapshot_mix_fx(snaps, nsnap, n, i, pref, mix);
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (blockIdx.x * PERTURB_BLOCK + j * 256 + threadIdx.x >= (unsigned)n) break;
+  for (int j = 0; j < PER; j++) {
+    if (first + j * 256 >= (unsigned)n) break;
     if (off >> j & 1) mix[j] = snapshot_mix(snaps, nsnap, n, i[j], pref);
     if (mixed) mixed[i[j]] = mix[j];
     n0 = __fma_rn(fin[i[j]], fin[i[j]], n0);
@@ -354,15 +357,23 @@ static int check_geom(const clbm_geom *g) {
   return CLBM_OK;
 }
 
+// Values a block of the norms takes.  Four per thread where there are blocks for
+// all SMs; one per thread up to two such blocks an SM, whose 1024 values kept a
+// few SMs' FP64 pipes busy while the others had none.  us a call that allocates
+// nothing, one per thread and four: 12x9 with 40 snapshots 34.8 and 48.2, 80x60 with
+// 10 28.0 and 29.9, 97x97 33.2 and 32.2, 129x129 37.4 and 34.9.
+static int perturb_block(int n) { return n <= 2 * 152 * 256 ? PERTURB_SMALL : PERTURB_BLOCK; }
+
 // The three passes of a perturbation; wa: the weight pair, part: two norm
-// partials per 1024 values, mixed (nullable): n values (device).
+// partials per block (perturb_block), mixed (nullable): n values (device).
 static cudaError_t run_perturb(double *fin, const double *snaps, double eps, int nsnap, int n, const double *prefactors,
                                double *wa, double *part, double *mixed, cudaStream_t st) {
   Prefactors pref = {};
   for (int q = 0; q < nsnap; q++) pref.v[q] = prefactors[q];
   pref.place = mix_place(prefactors, nsnap);
-  const int nb = (n - 1) / PERTURB_BLOCK + 1;
-  cudaError_t e = launch_after(k_ref_perturb_norms, nb, 256, 0, st, fin, snaps, nsnap, n, pref, part, mixed);
+  const int values = perturb_block(n), nb = (n - 1) / values + 1;
+  cudaError_t e = launch_after(values == PERTURB_SMALL ? k_ref_perturb_norms<1> : k_ref_perturb_norms<4>, nb, 256, 0, st,
+                               fin, snaps, nsnap, n, pref, part, mixed);
   if (e == cudaSuccess) e = launch_after(k_ref_perturb_finalize, 1, 256, 0, st, pref, nsnap, part, nb, eps, wa);
   if (e == cudaSuccess) e = launch_after(k_ref_perturb_apply, (n - 1) / 256 + 1, 256, 0, st, fin, snaps, nsnap, n, pref, wa, eps, mixed);
   return e;
@@ -433,7 +444,7 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
                                         int n, const double *prefactors, void *stream) {
   if (!fin || !snaps || !prefactors || nsnap < 1 || nsnap > 64 || n < 1) return CLBM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t nb = (size_t)(n - 1) / PERTURB_BLOCK + 1, head = 2 + 2 * nb;
+  const size_t nb = (size_t)(n - 1) / perturb_block(n) + 1, head = 2 + 2 * nb;
   double *d_buf = nullptr;
   // (without room for a further state the mix is formed twice, the same values)
   bool keep = true;
@@ -452,15 +463,15 @@ extern "C" int clbm_ref_perturbed_state(double *fin, const double *snaps, double
 
 // ---------------------------------------------------------------------------
 // clbm_ref_perturbed_state_noalloc: the same kernels as
-// clbm_ref_perturbed_state, with their scratch (two norm partial sums per 1024
-// values, the mix weight) in a fixed device array instead of a per-call
+// clbm_ref_perturbed_state, with their scratch (two norm partial sums per
+// block, the mix weight) in a fixed device array instead of a per-call
 // allocation.  It serves callers that must not allocate device memory at all:
 // code running under an allocator that already owns the whole device, or
 // inside a time-critical loop where an allocation's implicit synchronisation
 // is not acceptable.
 namespace {
 constexpr int NOALLOC_MAX_N = 1 << 20;                     // values per state, 9*Dx*Dy
-constexpr int NOALLOC_MAX_BLOCKS = NOALLOC_MAX_N / PERTURB_BLOCK;  // norm partials (pairs)
+constexpr int NOALLOC_MAX_BLOCKS = NOALLOC_MAX_N / PERTURB_BLOCK;  // norm partials (pairs; perturb_block: 304 of the small)
 constexpr int NOALLOC_PREF = 64;                           // prefactors (nsnap <= 64)
 // Shared by every call on a device and kept until the process exits
 // (16 KB per device that loads the library): the mix weight and 1/a, then the
