@@ -128,7 +128,7 @@ __device__ __forceinline__ fx_t fx_exact(double x) {
   return (fx_t)(m >> (1023 - (int)(hi >> 20)));
 }
 // Round to the 53 bits of a double (none to round below 2^-8).  A leading bit
-// at 62 - z takes 10 - z bits away: mask has them, half half a unit less one.
+// at 63 - z takes 11 - z bits away: mask has them, half half a unit less one.
 struct FxPlace {
   unsigned mask, half, shift;
 };
