@@ -994,8 +994,10 @@ static cudaLaunchConfig_t temporal_config(int cs, int threads, int nclones, size
   return cfg;
 }
 
-static cudaError_t prepare(TemporalFn fn, int cs, size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// (the limit and not a shape's own need: the attribute is the kernel's, and contexts
+// in other threads set it for their shapes between this and the launch)
+static cudaError_t prepare(TemporalFn fn, int cs) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
   if (e == cudaSuccess && cs > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
 }
@@ -1019,7 +1021,7 @@ cudaError_t launch_temporal(const TemporalArgs &a, int cs, int variant, int nclo
   if (!k || !temporal_resident(W, rows_max) || !square_thick(a.rd) || a.steps < 1)
     return cudaErrorInvalidConfiguration;
   const TemporalFn fn = k->fn[a.keep ? 2 : field];
-  cudaError_t e = prepare(fn, cs, smem);
+  cudaError_t e = prepare(fn, cs);
   if (e != cudaSuccess) return e;
   TemporalArgs args = a;
   const unsigned long long wh = (W + 1) / 2;
@@ -1035,7 +1037,7 @@ int temporal_max_clusters(int cs, int variant, int W, int rows_max, bool field) 
   const TemporalKernel *k = temporal_kernel(variant, cs, W, rows_max, 0, &smem);
   if (!k) return 0;
   const TemporalFn fn = k->fn[field];
-  if (prepare(fn, cs, smem) != cudaSuccess) return 0;
+  if (prepare(fn, cs) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = temporal_config(cs, k->threads, 64, smem, nullptr, attr);
   int n = 0;
